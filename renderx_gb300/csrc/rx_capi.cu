@@ -58,7 +58,7 @@ void rx_destroy(rx_context* c) {
     cudaDeviceSynchronize();
     for (DevBuf* b : {&c->d_bvh, &c->d_bvh4, &c->d_bvh8, &c->d_tris, &c->d_tri_nrm, &c->d_ref, &c->d_ref_leaf_node, &c->d_ref_leaf_range, &c->d_ref_tris,
                       &c->d_anc_range, &c->d_anc_nodes, &c->d_anc_box, &c->d_slot_n, &c->d_tri_v, &c->d_tri_n, &c->d_tri_obj,
-                      &c->d_objects, &c->d_light_cdf, &c->d_light_tri,
+                      &c->d_objects, &c->d_light_cdf, &c->d_light_tri, &c->d_media,
                       &c->d_counters, &c->d_queue})
       b->release();
     for (int k = 0; k < rx_context::kRing; k++) {
@@ -335,6 +335,33 @@ rx_status rx_context::build_scene() {
     cdf.push_back((float)acc);
     ltri.push_back(t);
   }
+  // the medium objects in find_inside's order (last first), each with its bounds padded by
+  // a thousandth of its size and a ten-thousandth of its coordinates: far above the
+  // rounding of a hit's distance, so that no line through a point outside the padded
+  // bounds meets the object on both sides of the point
+  std::vector<float> bounds(6 * (size_t)nobj);  // of the medium objects: lo xyz, hi xyz
+  for (size_t k = 0; k < bounds.size(); k++) bounds[k] = k % 6 < 3 ? INFINITY : -INFINITY;
+  for (uint32_t t = 0; t < nt; t++) {
+    if (objs[c->tri_obj[t]].material != rx::kVPM) continue;
+    float* b = &bounds[6 * (size_t)c->tri_obj[t]];
+    for (int k = 0; k < 3; k++) {
+      const float4 v = tv[3 * (size_t)t + k];
+      const float x[3] = {v.x, v.y, v.z};
+      for (int a = 0; a < 3; a++) b[a] = std::min(b[a], x[a]), b[3 + a] = std::max(b[3 + a], x[a]);
+    }
+  }
+  std::vector<float4> media;
+  for (uint32_t o = nobj; o-- > 0;) {
+    if (objs[o].material != rx::kVPM) continue;
+    const float* b = &bounds[6 * (size_t)o];  // an object without triangles keeps its empty bounds
+    float pad = 0.0f, id;
+    for (int a = 0; a < 3; a++)
+      if (b[a] <= b[3 + a])
+        pad = std::max(pad, 1e-3f * (b[3 + a] - b[a]) + 1e-4f * std::max(std::fabs(b[a]), std::fabs(b[3 + a])) + 1e-5f);
+    std::memcpy(&id, &o, 4);
+    media.push_back(make_float4(b[0] - pad, b[1] - pad, b[2] - pad, id));
+    media.push_back(make_float4(b[3] + pad, b[4] + pad, b[5] + pad, 0.0f));
+  }
   DeviceGuard g(c->device);
   rx_status st;
   if ((st = upload(c, c->d_tri_v, tv.data(), tv.size() * sizeof(float4), "upload triangle vertices")) != RX_OK) return st;
@@ -347,6 +374,9 @@ rx_status rx_context::build_scene() {
     if ((st = upload(c, c->d_light_cdf, cdf.data(), cdf.size() * 4, "upload light cdf")) != RX_OK) return st;
     if ((st = upload(c, c->d_light_tri, ltri.data(), ltri.size() * 4, "upload light triangles")) != RX_OK) return st;
   }
+  if (!media.empty() &&
+      (st = upload(c, c->d_media, media.data(), media.size() * sizeof(float4), "upload media")) != RX_OK)
+    return st;
   rx::DevScene& S = c->scene;
   S.accel = c->accel;
   S.slot_n = c->d_slot_n.as<float4>();
@@ -359,6 +389,8 @@ rx_status rx_context::build_scene() {
   S.light_tri = c->d_light_tri.as<uint32_t>();
   S.num_lights = (uint32_t)cdf.size();
   S.light_area = (float)acc;
+  S.media = c->d_media.as<float4>();
+  S.num_media = (uint32_t)(media.size() / 2);
   c->scene_ready = true;
   return RX_OK;
 }

@@ -167,7 +167,7 @@ struct rx_context {
   rx::DevBuf d_bvh, d_tris, d_tri_nrm, d_ref, d_ref_leaf_node, d_ref_leaf_range, d_ref_tris, d_anc_range, d_anc_nodes, d_anc_box;
   rx::DevScene scene{};
   bool scene_ready = false;
-  rx::DevBuf d_slot_n, d_tri_v, d_tri_n, d_tri_obj, d_objects, d_light_cdf, d_light_tri;
+  rx::DevBuf d_slot_n, d_tri_v, d_tri_n, d_tri_obj, d_objects, d_light_cdf, d_light_tri, d_media;
   rx::DevBuf d_counters;     // 4 x u64 diagnostics + per-slot queue lengths
   rx::DevBuf d_queue;        // closest-hit scratch (winner leaves + eager queue)
   // staging ring for host-buffer calls

@@ -44,6 +44,9 @@ struct DevScene {
   const uint32_t* light_tri;
   uint32_t num_lights;
   float light_area;         // total emitter area (Scene::SurfaceSampler totals)
+  const float4* media;      // the medium objects, last first: 2 float4 each, the padded bounds
+                            // (lo.xyz, object id bits), (hi.xyz, 0); see find_inside
+  uint32_t num_media;
 };
 
 }  // namespace rx
