@@ -569,10 +569,14 @@ struct Grid {
   const int* ref;         // photon light vertices (path * maxv + index) in bucket order
   const float4* join;     // per photon in bucket order, kJoin float4: the light side of a merge
 };
-// The light side of a merge with a photon at light vertex ci + 1, gathered once per
-// photon into bucket order: vertex ci (L, 4 float4), vertex ci - 1 (Lm, 4 float4, zero
-// when ci = 0) and L's record (2 float4; MisL::pad carries ci).
-constexpr int kJoin = 10;
+// The light side of a merge with a photon at light vertex ci + 1, gathered once per photon
+// into bucket order: what the pair needs of L (vertex ci), its predecessor Lm and L's
+// record, with everything that does not depend on the eye vertex already formed:
+//   0: L's origin, dprob x oprob            3: direction to Lm (rev_to), tla
+//   1: L's contact normal, flags            4: Lm's direction, prob
+//   2: thr x colour of L, sla               5: contact, inside, Lm's inside
+constexpr int kJoin = 6;
+constexpr uint32_t kJoinRandom = 1u, kJoinPred = 2u;  // L sampled at random; L has a predecessor
 __device__ __forceinline__ unsigned cell_hash(int x, int y, int z, unsigned mask) {
   return ((unsigned)(x * 73856093) ^ (unsigned)(y * 19349663) ^ (unsigned)(z * 83492791)) & mask;
 }
@@ -586,31 +590,38 @@ __global__ void k_grid_count(const float4* pos, const unsigned* n_photons, unsig
     atomicAdd(&count[k], 1u);
   }
 }
-__global__ void k_grid_scatter(const unsigned* key, const float4* pos, const int* ref, const unsigned* n_photons,
-                               unsigned cap, unsigned* cursor, float4* pos_out, int* ref_out, const float4* lv,
-                               const MisL* lmis, uint32_t maxv, float4* join) {
+__global__ void __launch_bounds__(256) k_grid_scatter(DevScene S, VcmParams P, const unsigned* key, const float4* pos,
+                                                      const int* ref, const unsigned* n_photons, unsigned cap,
+                                                      unsigned* cursor, float4* pos_out, int* ref_out,
+                                                      const float4* lv, const MisL* lmis, float4* join) {
   unsigned n = min(*n_photons, cap);
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     unsigned slot = atomicAdd(&cursor[key[i]], 1u);
     const int r = ref[i];
     pos_out[slot] = pos[i];
     ref_out[slot] = r;
-    const uint32_t lp = (uint32_t)r / maxv, ci = (uint32_t)r % maxv - 1;
-    const float4* L = lv + 4 * ((size_t)lp * maxv + ci);
-    float4* out = join + (size_t)kJoin * slot;
-#pragma unroll
-    for (int k = 0; k < 4; k++) out[k] = L[k];
+    const uint32_t lp = (uint32_t)r / P.maxv, ci = (uint32_t)r % P.maxv - 1;
+    const float4* lb = lv + 4 * ((size_t)lp * P.maxv + ci);
+    const PV L = load_pv(lb);
+    const MisL m = lmis[(size_t)lp * P.maxv + ci];
+    const F3 n0 = contact_normal(S, P.cam, L), c = m.thr * L.c;
+    uint32_t flags = rnd(L) ? kJoinRandom : 0u;
+    F3 rd{0, 0, 0}, pd{0, 0, 0};
+    int pin = kNone;
     if (ci > 0) {
-      const float4* Lm = L - 4;
-#pragma unroll
-      for (int k = 0; k < 4; k++) out[4 + k] = Lm[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) out[4 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const PV Lm = load_pv(lb - 4);
+      flags |= kJoinPred;
+      rd = rev_to(L, Lm).d;
+      pd = Lm.d;
+      pin = Lm.inside;
     }
-    MisL m = lmis[(size_t)lp * maxv + ci];
-    out[8] = make_float4(m.sla, m.tla, m.prob, __int_as_float((int)ci));
-    out[9] = make_float4(m.thr.x, m.thr.y, m.thr.z, 0.0f);
+    float4* out = join + (size_t)kJoin * slot;
+    out[0] = make_float4(L.o.x, L.o.y, L.o.z, L.dprob * L.oprob);
+    out[1] = make_float4(n0.x, n0.y, n0.z, __uint_as_float(flags));
+    out[2] = make_float4(c.x, c.y, c.z, m.sla);
+    out[3] = make_float4(rd.x, rd.y, rd.z, m.tla);
+    out[4] = make_float4(pd.x, pd.y, pd.z, m.prob);
+    out[5] = make_float4(__int_as_float(L.contact), __int_as_float(L.inside), __int_as_float(pin), 0.0f);
   }
 }
 
@@ -1154,31 +1165,6 @@ __global__ void k_merge_fill(DevScene S, VcmParams P, const float4* ev, const in
   }
 }
 
-// The contribution of merging eye vertex E (pe before it, records me) with the photon
-// whose light side is `jd` (kJoin float4): the photon's predecessor L = w[ci] is joined
-// with E as connectRays does for a merge, then colour, probability and MIS weight from
-// the records (zero where the reference drops the path).
-__device__ __forceinline__ F3 merge_pair(const DevScene& S, const VcmParams& P, const float4* jd, const PV& E,
-                                         const PV& pe, const MisE& me) {
-  const PV L = load_pv(jd);
-  const float4 m0 = jd[8], m1 = jd[9];
-  const int ci = __float_as_int(m0.w);
-  MisL ml;
-  ml.sla = m0.x;
-  ml.tla = m0.y;
-  ml.prob = m0.z;
-  ml.thr = f3(m1);
-  PV Lm, Lp, Ep;
-  if (ci > 0) Lm = load_pv(jd + 4);
-  join(S, P.cam, L, ci > 0 ? &Lm : nullptr, E, &pe, true, Lp, Ep);
-  F3 col;
-  float prob, wt;
-  if (!join_eval(S, P.cam, L, ci > 0 ? &Lm : nullptr, Lp, Ep, &pe, ml, me, true, false, P.radius, P.norm, col, prob,
-                 wt))
-    return F3{0, 0, 0};
-  return col * (wt / prob) * (1.0f / P.norm);
-}
-
 // The iteration's merge queries in spatial order. A query is an eye vertex that merges
 // (colorByMergingPaths, VCMTracer.cpp:566-636: vertex ei >= 1 of the pixel's eye path,
 // sampled at random, before the first emitter); its key is the Morton code of its
@@ -1237,115 +1223,246 @@ __global__ void __launch_bounds__(128) k_merge_queries(DevScene S, VcmParams P, 
   }
 }
 
-// Merge pairs (colorByMergingPaths, VCMTracer.cpp:566-636), one warp per query of the
-// spatially sorted list, positions [j0, j1): the 32 lanes hash the cells the sphere
-// touches, and the warp walks each distinct bucket 128 sorted photons per step
-// (coalesced positions, the strict |p - x| < r test), appending the photons inside as
-// (query, photon slot in bucket order) pairs with one atomic per step. Pairs past `cap`
-// are counted, not written (the host then grows the list or splits the range). Queries
-// taken in spatial order make the pairs that follow one another gather the same photons.
-__global__ void __launch_bounds__(256) k_merge_walk(VcmParams P, const float4* ev, Grid G, const uint32_t* qlist,
-                                                    const uint32_t* order, uint32_t j0, uint32_t j1,
-                                                    unsigned long long cap, uint32_t* pair_q, int* pair_ref,
-                                                    unsigned long long* npairs) {
-  const int lane = threadIdx.x & 31;
+// The eye side of a merge query, formed once per query in spatial order (k_merge_eye):
+// what a pair needs of the eye vertex E, its predecessor pe and E's record.
+struct alignas(16) EyeSide {
+  F3 o;         // E's origin
+  float oprob;
+  F3 n;         // E's contact normal
+  int contact;
+  F3 rd;        // direction to pe (rev_to)
+  int inside;
+  F3 pd;        // pe's direction
+  int pin;      // pe's inside object
+  F3 thr;
+  float prob;
+  float pbr, sea;
+  uint32_t prand;  // pe sampled at random
+  uint32_t pixel;
+};
+__global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, const float4* ev, const MisE* emis,
+                                                   const uint32_t* qlist, const uint32_t* order, const unsigned* count,
+                                                   EyeSide* out) {
+  const uint32_t n = *count;
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const uint32_t q = __ldg(&qlist[__ldg(&order[j])]);  // vertex q % maxv >= 1 of pixel q / maxv
+    const PV E = load_pv(ev + 4 * (size_t)q), pe = load_pv(ev + 4 * ((size_t)q - 1));
+    const MisE me = emis[q];
+    EyeSide e;
+    e.o = E.o;
+    e.oprob = E.oprob;
+    e.n = contact_normal(S, P.cam, E);
+    e.contact = E.contact;
+    e.rd = rev_to(E, pe).d;
+    e.inside = E.inside;
+    e.pd = pe.d;
+    e.pin = pe.inside;
+    e.thr = me.thr;
+    e.prob = me.prob;
+    e.pbr = me.pbr;
+    e.sea = me.sea;
+    e.prand = rnd(pe) ? 1u : 0u;
+    e.pixel = q / P.maxv;
+    out[j] = e;
+  }
+}
+
+// bsdf_of and dir_pdf at a merge's vertices, whose contact normal `n` is at hand: `obj` is
+// the vertex's contact object, or its inside object when it has no contact (`volume`).
+__device__ __forceinline__ F3 merge_bsdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
+  if (obj < 0) return F3{0, 0, 0};
+  const DevObject& ob = S.objects[obj];
+  if (volume) return ob.material == kVPM ? f3v(ob.sigma_s) * hg(ob.g, dot(in, out)) : F3{0, 0, 0};
+  if (ob.material == kEmissive) return dot(n, out) < 0.0f ? F3{0, 0, 0} : f3v(ob.color);
+  F3 f = {0, 0, 0};
+  if (!(dot(n, in) <= 0.0f && dot(n, out) >= 0.0f)) return f;
+  if (ob.material == kDiffuse || ob.material == kPhong)
+    f = f + (ob.material == kPhong ? f3v(ob.diffuse_color) : f3v(ob.color)) * (1.0f / RX_PI);
+  if (ob.material == kGlossy || ob.material == kPhong) {
+    const F3 c = f3v(ob.color), r = n * (-dot(n, in) * 2.0f) + in;
+    const float rw = dot(r, out);
+    if (rw > 0.0f) f = f + c * (maxc(c) * powf(rw, ob.coeff));
+  }
+  return f;
+}
+__device__ __forceinline__ float merge_pdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
+  if (obj < 0) return 0.0f;
+  const DevObject& ob = S.objects[obj];
+  if (volume) {
+    if (ob.material != kVPM) return ob.material == kRefractive || ob.material == kReflective ? 1.0f : 0.0f;
+    const float albedo = lum(f3v(ob.sigma_s)) / lum(sigma_t(ob));
+    return albedo * hg(ob.g, dot(normalize(in), out));
+  }
+  switch (ob.material) {
+    case kDiffuse: return maxc(f3v(ob.color)) * cos_lobe_pdf(n, out, 1.0f);
+    case kRefractive:
+    case kReflective: return 1.0f;
+    case kGlossy: return cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff);
+    case kPhong:
+      return (maxc(f3v(ob.diffuse_color)) * cos_lobe_pdf(n, out, 1.0f) +
+              cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff)) / 2.0f;
+    default: return 0.0f;  // emitters, medium boundaries
+  }
+}
+
+// The contribution of merging the eye vertex of `e` with the photon whose light side is
+// `jd` (kJoin float4): the photon's predecessor L = w[ci] is joined with E as connectRays
+// does for a merge, then colour, probability and MIS weight from the records (join and
+// join_eval with merged set, on the parts formed per photon and per query; zero where the
+// reference drops the path). r: the merge radius.
+__device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, const EyeSide& e, float r, float norm) {
+  const float4 j0 = __ldg(jd), j1 = __ldg(jd + 1), j2 = __ldg(jd + 2), j5 = __ldg(jd + 5);
+  const int lcontact = __float_as_int(j5.x), linside = __float_as_int(j5.y);
+  const uint32_t flags = __float_as_uint(j1.w);
+  const F3 lo = f3(j0), nl = f3(j1), v = e.o - lo;
+  const float len = length(v), D = fmaxf(len, 1e-5f);
+  const F3 ld = len > 0.0f ? v * (1.0f / len) : v, ed = -ld;
+  // E: its inside object and BSDF with the new direction (connectRays)
+  const bool evol = e.contact == kNone;
+  int einside = e.inside;
+  if (!evol) {
+    if (dot(e.n, ed) <= 0.0f) einside = e.contact;
+    else if (dot(e.n, e.pd) <= 0.0f) einside = e.pin;
+    else einside = find_inside(S, e.o, ed, e.contact);
+  }
+  const int eobj = evol ? einside : e.contact;
+  const bool lmed = is_vpm(S, linside), emed = is_vpm(S, einside);
+  const bool aimed = len > 0.0f;  // getCosineTerm: no cosine without a direction
+  const float cosL = aimed && lcontact >= 0 && !is_vpm(S, lcontact) ? fmaxf(fabsf(dot(nl, ld)), kCosMin) : 1.0f;
+  const float cosE = aimed && e.contact >= 0 && !is_vpm(S, e.contact) ? fmaxf(fabsf(dot(e.n, ed)), kCosMin) : 1.0f;
+  F3 col = f3(j2) * decay_of(S, linside, D);
+  col = col * (cosL * cosE / (D * D));
+  col = col * merge_bsdf(S, eobj, evol, e.n, e.pd, ed);
+  col = col * e.thr;
+  const float4 j4 = __ldg(jd + 4);
+  float opf = 1.0f;  // getOriginSampleProbDensity of E from L
+  if (lmed) opf = evol ? p_medium(S.objects[linside], D) : P_surface(S.objects[linside], D);
+  const float vol = evol && einside != kNone ? 4.0f / 3.0f * r : 1.0f;
+  const float area = RX_PI * r * r;
+  float prob = j4.w * j0.w * e.oprob * e.prob;
+  prob *= area;
+  prob *= cosE;
+  prob /= D * D;
+  prob *= opf;
+  prob *= vol;
+  if (!(prob > 0.0f) || !(length(col) > 0.0f)) return F3{0, 0, 0};
+  const bool rl = flags & kJoinRandom, pred = flags & kJoinPred, lvol = lcontact == kNone;
+  float dpf = 1.0f;
+  if (rl) dpf = pred ? merge_pdf(S, lvol ? linside : lcontact, lvol, nl, f3(j4), ld) : cos_lobe_pdf(nl, ld, 1.0f);
+  // every term over pf[ci] pb[ci+1] (join_eval)
+  const float g = 1.0f / (D * D);
+  const float M = dpf * opf * cosE * g * area * norm * vol;
+  float sum = (rl ? 1.0f : 0.0f) + M;
+  if (pred) {
+    const float4 j3 = __ldg(jd + 3);
+    float pb0 = cosL * g * merge_pdf(S, eobj, evol, e.n, e.pd, ed);
+    if (emed) pb0 *= lvol ? p_medium(S.objects[einside], D) : P_surface(S.objects[einside], D);
+    const int lin = __float_as_int(j5.z);
+    const float back = rl ? merge_pdf(S, lvol ? lin : lcontact, lvol, nl, ed, f3(j3)) : 1.0f;
+    sum += pb0 * (back * j2.w + j3.w);
+  }
+  const float pf1 = cosE * g * (rl ? dpf * opf : 1.0f);  // pf[ci+1] / pf[ci]
+  if (e.prand) sum += pf1 * e.pbr;
+  sum += pf1 * merge_pdf(S, evol ? e.pin : e.contact, evol, e.n, ld, e.rd) * e.sea;
+  const float wt = M / sum;
+  return col * ((wt >= 0.0f ? wt : 0.0f) / prob) * (1.0f / norm);
+}
+
+// Merging (colorByMergingPaths, VCMTracer.cpp:566-636), one warp per query of the spatially
+// sorted list: the 32 lanes hash the cells the sphere touches, the warp walks each distinct
+// bucket 128 sorted photons per step (coalesced positions, the strict |p - x| < r test) and
+// puts the photons inside on a list in shared memory; whenever the list holds 32 pairs the
+// lanes evaluate one each (the last ones of a query wait for the next query's, so only the
+// warp's final evaluation has idle lanes). A lane sums its pairs of a query before the
+// image atomics. Queries in spatial order make the warps that run together gather the same
+// photons.
+//
+// The walk and the evaluation were two kernels with a list of all pairs between them
+// (109 M pairs an iteration at 512^2 pixels and 2^20 light paths: 0.9 GB written and read
+// back, one counter that every walking warp waited on, the list's size read by the host
+// and the walk repeated when it had grown), and the evaluation formed both vertices'
+// normals and reversed directions per pair: 14.1 + 3.75 ms (7.5 when the walk repeated)
+// against 6.76 ms here, with 128 registers (bounds of 5 or 6 blocks per SM spill: 7.25,
+// 8.59 ms).
+constexpr int kMergeList = 32 + 128;
+__global__ void __launch_bounds__(128) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
+                                               const unsigned* count, float* img, unsigned long long* merges) {
+  __shared__ uint2 s_list[4][kMergeList];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint2* list = s_list[warp];
   const unsigned lt = (1u << lane) - 1u;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t nq = *count, nw = gridDim.x * 4;
   const float r = P.radius;
-  for (uint32_t j = j0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < j1; j += nw) {
-    {
-      const uint32_t q = __ldg(&qlist[__ldg(&order[j])]);
-      const F3 x = f3(ev[4 * (size_t)q]);  // vertex q % maxv of pixel q / maxv
-      // the cells the sphere touches (as merge_buckets), one per lane; equal buckets are
-      // walked once, by the lowest lane that holds them
-      const int x0 = (int)floorf((x.x - r) / G.cell), y0 = (int)floorf((x.y - r) / G.cell);
-      const int z0 = (int)floorf((x.z - r) / G.cell);
-      const int nx = min((int)floorf((x.x + r) / G.cell), x0 + 2) - x0 + 1;
-      const int ny = min((int)floorf((x.y + r) / G.cell), y0 + 2) - y0 + 1;
-      const int nz = min((int)floorf((x.z + r) / G.cell), z0 + 2) - z0 + 1;
-      const bool cell_lane = lane < nx * ny * nz;
-      unsigned bucket = 0xffffffffu, b0 = 0, b1 = 0;
-      if (cell_lane) {
-        const int cz = lane % nz, cy = (lane / nz) % ny, cx = lane / (nz * ny);
-        bucket = cell_hash(x0 + cx, y0 + cy, z0 + cz, G.mask);
-      }
-      const unsigned peers = __match_any_sync(0xffffffffu, bucket);
-      const bool leader = cell_lane && (unsigned)(__ffs(peers) - 1) == (unsigned)lane;
-      if (leader) {
-        b0 = G.start[bucket];
-        b1 = G.start[bucket + 1];
-      }
-      for (unsigned lead = __ballot_sync(0xffffffffu, leader && b1 > b0); lead; lead &= lead - 1) {
-        const int src = __ffs(lead) - 1;
-        const unsigned r0 = __shfl_sync(0xffffffffu, b0, src), r1 = __shfl_sync(0xffffffffu, b1, src);
-        for (unsigned i0 = r0; i0 < r1; i0 += 128) {
-          bool h[4];
-          unsigned m[4], n = 0;
+  uint32_t fill = 0, cur = 0xffffffffu;
+  unsigned long long total = 0;
+  F3 acc = {0, 0, 0};
+  auto evaluate = [&](uint32_t at) {  // the pair at list entry `at`
+    const uint2 pair = list[at];
+    const EyeSide e = eye[pair.y];
+    if (e.pixel != cur) {
+      if (cur != 0xffffffffu) img_add(img, (int)cur, acc);
+      acc = F3{0, 0, 0};
+      cur = e.pixel;
+    }
+    acc = acc + merge_pair(S, G.join + (size_t)kJoin * pair.x, e, r, P.norm);
+  };
+  for (uint32_t j = blockIdx.x * 4 + warp; j < nq; j += nw) {
+    const F3 x = eye[j].o;
+    // the cells the sphere touches (as merge_buckets), one per lane; equal buckets are
+    // walked once, by the lowest lane that holds them
+    const int x0 = (int)floorf((x.x - r) / G.cell), y0 = (int)floorf((x.y - r) / G.cell);
+    const int z0 = (int)floorf((x.z - r) / G.cell);
+    const int nx = min((int)floorf((x.x + r) / G.cell), x0 + 2) - x0 + 1;
+    const int ny = min((int)floorf((x.y + r) / G.cell), y0 + 2) - y0 + 1;
+    const int nz = min((int)floorf((x.z + r) / G.cell), z0 + 2) - z0 + 1;
+    const bool cell_lane = lane < nx * ny * nz;
+    unsigned bucket = 0xffffffffu, b0 = 0, b1 = 0;
+    if (cell_lane) {
+      const int cz = lane % nz, cy = (lane / nz) % ny, cx = lane / (nz * ny);
+      bucket = cell_hash(x0 + cx, y0 + cy, z0 + cz, G.mask);
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, bucket);
+    const bool leader = cell_lane && (unsigned)(__ffs(peers) - 1) == (unsigned)lane;
+    if (leader) {
+      b0 = G.start[bucket];
+      b1 = G.start[bucket + 1];
+    }
+    for (unsigned lead = __ballot_sync(0xffffffffu, leader && b1 > b0); lead; lead &= lead - 1) {
+      const int src = __ffs(lead) - 1;
+      const unsigned r0 = __shfl_sync(0xffffffffu, b0, src), r1 = __shfl_sync(0xffffffffu, b1, src);
+      for (unsigned i0 = r0; i0 < r1; i0 += 128) {
+        bool h[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const unsigned i = i0 + 32 * u + lane;
-            h[u] = i < r1 && length(x - f3(G.pos[i])) < r;
-          }
+        for (int u = 0; u < 4; u++) {
+          const unsigned i = i0 + 32 * u + lane;
+          h[u] = i < r1 && length(x - f3(__ldg(&G.pos[i]))) < r;
+        }
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            m[u] = __ballot_sync(0xffffffffu, h[u]);
-            n += __popc(m[u]);
-          }
-          if (n == 0) continue;
-          unsigned long long base = 0;
-          if (lane == 0) base = atomicAdd(npairs, (unsigned long long)n);
-          base = __shfl_sync(0xffffffffu, base, 0);
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            if (h[u]) {
-              const unsigned long long slot = base + __popc(m[u] & lt);
-              if (slot < cap) {
-                pair_q[slot] = q;
-                pair_ref[slot] = (int)(i0 + 32 * u + lane);
-              }
-            }
-            base += __popc(m[u]);
-          }
+        for (int u = 0; u < 4; u++) {
+          const unsigned m = __ballot_sync(0xffffffffu, h[u]);
+          if (h[u]) list[fill + __popc(m & lt)] = make_uint2(i0 + 32 * u + lane, j);
+          fill += __popc(m);
+        }
+        __syncwarp();
+        while (fill >= 32) {
+          fill -= 32;
+          total += 32;
+          evaluate(fill + lane);
+          __syncwarp();
         }
       }
     }
   }
+  if ((uint32_t)lane < fill) evaluate(lane);
+  if (cur != 0xffffffffu) img_add(img, (int)cur, acc);
+  total += fill;
+  if (lane == 0 && total) atomicAdd(merges, total);
 }
 
-// One merge pair per lane, kRun consecutive pairs per thread (pairs of one query are
-// appended together, so the eye vertex and its records are loaded once per query and
-// contributions summed per pixel before the image atomics).
-constexpr int kRun = 8;
-__global__ void __launch_bounds__(128) k_merge_eval(DevScene S, VcmParams P, const float4* ev, const MisE* emis,
-                                                    const float4* join, const uint32_t* pair_q, const int* pair_slot,
-                                                    uint32_t npairs, float* img) {
-  uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) * kRun; base < npairs; base += stride * kRun) {
-    F3 acc = {0, 0, 0};
-    uint32_t cur = 0xffffffffu;
-    PV E, pe;
-    MisE me;
-    for (uint32_t j = base; j < base + kRun && j < npairs; j++) {
-      const uint32_t q = pair_q[j];
-      if (q != cur) {
-        if (cur != 0xffffffffu) img_add(img, (int)(cur / P.maxv), acc);
-        acc = {0, 0, 0};
-        cur = q;
-        const uint32_t p = q / P.maxv, k = q % P.maxv;
-        const float4* eb = ev + 4 * ((size_t)p * P.maxv);
-        E = load_pv(eb + 4 * k);
-        pe = load_pv(eb + 4 * (k - 1));
-        me = emis[q];
-      }
-      acc = acc + merge_pair(S, P, join + (size_t)kJoin * pair_slot[j], E, pe, me);
-    }
-    if (cur != 0xffffffffu) img_add(img, (int)(cur / P.maxv), acc);
-  }
-}
-
+constexpr int kRun = 8;  // consecutive pairs per thread of the whole-path check
 // Merge pairs evaluated by the reference's loops over the whole joined path
 // (connectRays, connectColorProb, connectMergeWeight): O(path length) per pair, with the
-// path in a per-thread array. Kept as the check of k_merge_eval (RX_VCM_FULL_PATH_MIS).
+// path in a per-thread array. Kept as the check of k_merge (RX_VCM_FULL_PATH_MIS).
 __global__ void __launch_bounds__(128) k_merge_eval_full(DevScene S, VcmParams P, const float4* lv, const float4* ev,
                                                          const uint32_t* pair_q, const int* pair_ref, uint32_t npairs,
                                                          float* img) {
@@ -1721,8 +1838,8 @@ static VcmParams camera_params(const rx_camera& cam) {
   return P;
 }
 
-// Photons stored in this iteration's grid (the stored count, clipped to the capacity),
-// added to a running total.
+// A count of this iteration (photons stored in the grid, merge queries), clipped to its
+// capacity, added to a running total.
 __global__ void k_count_photons(const unsigned* nph, unsigned cap, unsigned long long* total) {
   *total += (unsigned long long)min(*nph, cap);
 }
@@ -1775,10 +1892,9 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     if ((e = al(29, (size_t)nq * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = al(30, ((size_t)kRayBins + 1024) * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = al(31, 16)) != cudaSuccess) return e;
+    if ((e = al(24, (size_t)nq * sizeof(EyeSide))) != cudaSuccess) return e;  // their eye sides
   }
   const bool full_mis = (opt.flags & RX_VCM_FULL_PATH_MIS) != 0;
-  constexpr uint32_t kMergeCap = 1u << 30;  // merge pairs per evaluation (8 GB of pair list)
-  uint32_t q_chunk = nq;                     // sorted queries per merge walk
   const uint32_t pair_cap = 1u << 27;  // pairs per evaluation window
   uint32_t pair_alloc = 1u << 20;      // grows with demand up to pair_cap
   if ((e = al(17, (size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return e;
@@ -1789,20 +1905,22 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   int grid = c->trace_cfg.sms * 4;
   // shadow rays on the persistent 4-wide walk when the tree fits its stack
   const bool wide_shadow = c->d_bvh4.p && 3 * c->bvh4.max_depth + 1 <= 64;
-  int sub_grid[2] = {0, 0};  // resident blocks of k_sub_run<false>, <true>
+  int sub_grid[2] = {0, 0}, merge_grid = 0;  // resident blocks of k_sub_run<false>, <true>, and of k_merge
   {
     int per = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<false>, 128, 0)) != cudaSuccess) return e;
     sub_grid[0] = c->trace_cfg.sms * std::max(per, 1);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<true>, 128, 0)) != cudaSuccess) return e;
     sub_grid[1] = c->trace_cfg.sms * std::max(per, 1);
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_merge, 128, 0)) != cudaSuccess) return e;
+    merge_grid = c->trace_cfg.sms * std::max(per, 1);
   }
   Event e0, e1, m0, m1;  // render; merge gather of an iteration (with stats)
   if ((e = e0.create()) != cudaSuccess || (e = e1.create()) != cudaSuccess) return e;
   if (stats && ((e = m0.create()) != cudaSuccess || (e = m1.create()) != cudaSuccess)) return e;
   cudaEventRecord(e0, s);
   float radius = opt.radius;
-  unsigned long long merges = 0, queries = 0;
+  unsigned long long merges = 0;
   float merge_ms = 0;
   unsigned nscan = buckets + 1;
   unsigned nblk = (nscan + 1023) / 1024;
@@ -1845,9 +1963,9 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       k_scan_sums<unsigned><<<1, 1024, 0, s>>>(bufs[9].as<unsigned>(), nblk);
       k_scan_add<unsigned><<<nblk, 1024, 0, s>>>(bufs[7].as<unsigned>(), bufs[9].as<unsigned>(), nscan,
                                                   bufs[8].as<unsigned>());
-      k_grid_scatter<<<grid, 256, 0, s>>>(bufs[4].as<unsigned>(), bufs[2].as<float4>(), bufs[3].as<int>(), nph, cap,
-                                          bufs[8].as<unsigned>(), bufs[22].as<float4>(), bufs[5].as<int>(),
-                                          bufs[0].as<float4>(), bufs[19].as<MisL>(), P.maxv, bufs[23].as<float4>());
+      k_grid_scatter<<<grid * 2, 256, 0, s>>>(S, P, bufs[4].as<unsigned>(), bufs[2].as<float4>(), bufs[3].as<int>(), nph,
+                                              cap, bufs[8].as<unsigned>(), bufs[22].as<float4>(), bufs[5].as<int>(),
+                                              bufs[0].as<float4>(), bufs[19].as<MisL>(), bufs[23].as<float4>());
       k_count_photons<<<1, 1, 0, s>>>(nph, cap, ctr + 6);
     }
     cudaMemsetAsync(bufs[10].p, 0, bufs[10].bytes, s);
@@ -1929,39 +2047,10 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       k_merge_queries<<<grid, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[13].as<int>(), qlist, qkey, qhist, qcount);
       scan_bins(qhist, qhist + kRayBins, s);
       k_ray_scatter<<<grid * 2, 256, 0, s>>>(qkey, 0, qcount, qhist, qorder);
-      unsigned nqv = 0;
-      cudaMemcpyAsync(&nqv, qcount, sizeof nqv, cudaMemcpyDeviceToHost, s);
-      if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-      queries += nqv;
-      for (uint32_t j0 = 0; j0 < nqv;) {
-        const uint32_t j1 = (uint32_t)std::min<uint64_t>(nqv, (uint64_t)j0 + q_chunk);
-        unsigned long long* np_dev = ctr + 4;  // [4] pairs of this query range
-        cudaMemsetAsync(np_dev, 0, sizeof(unsigned long long), s);
-        k_merge_walk<<<grid * 2, 256, 0, s>>>(P, bufs[12].as<float4>(), G, qlist, qorder, j0, j1, pair_alloc,
-                                              bufs[17].as<uint32_t>(), bufs[18].as<int>(), np_dev);
-        unsigned long long np = 0;
-        cudaMemcpyAsync(&np, np_dev, sizeof np, cudaMemcpyDeviceToHost, s);
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        if (np > pair_alloc) {  // grow the pair list, or split the query range once it is at its cap
-          if (pair_alloc < kMergeCap) {
-            pair_alloc = (uint32_t)std::min<unsigned long long>(kMergeCap, np + np / 4);
-            if ((e = bufs[17].alloc((size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return e;
-            if ((e = bufs[18].alloc((size_t)pair_alloc * sizeof(int))) != cudaSuccess) return e;
-            continue;
-          }
-          if (j1 - j0 > 1) {
-            q_chunk = (j1 - j0) / 2;
-            continue;
-          }
-          np = pair_alloc;  // one query beyond the cap: its first kMergeCap pairs
-        }
-        merges += np;
-        if (np)
-          k_merge_eval<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), bufs[23].as<float4>(),
-                                                bufs[17].as<uint32_t>(), bufs[18].as<int>(), (uint32_t)np,
-                                                bufs[10].as<float>());
-        j0 = j1;
-      }
+      k_merge_eye<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), qlist, qorder, qcount,
+                                           bufs[24].as<EyeSide>());
+      k_merge<<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
+      k_count_photons<<<1, 1, 0, s>>>(qcount, nq, ctr + 5);
       if (m1) {  // device time of this iteration's merge gather (walk + pair evaluation)
         cudaEventRecord(m1, s);
         if ((e = cudaEventSynchronize(m1)) != cudaSuccess) return e;
@@ -1992,11 +2081,11 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     cudaMemcpy(h, ctr, sizeof h, cudaMemcpyDeviceToHost);
     stats->extension_rays = h[0] + h[1];
     stats->shadow_rays = h[2];
-    stats->merges = merges;
+    stats->merges = merges + h[4];
     stats->paths = (uint64_t)P.n_pixels * done;
     stats->ms = ms;
     stats->merge_ms = merge_ms;
-    stats->merge_queries = queries;
+    stats->merge_queries = h[5];
     stats->photons = h[6];
   }
   return cudaSuccess;
