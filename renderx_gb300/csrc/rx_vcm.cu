@@ -155,7 +155,7 @@ __device__ __forceinline__ PV load_pv(const float4* p) {
 //    subpath alone;
 //  - the techniques at i <= ci-2 add up to pb[ci-1] x (a light-only sum) and those at
 //    i >= ci+2, with the merge at ci+1, to pf[ci+2] x (an eye-only sum), both built once
-//    per subpath by a recursion over its vertices (light_mis, eye_mis);
+//    per subpath by a recursion over its vertices (k_records);
 //  - what is left (C and M at ci-1 and ci, C at ci+1, and the pdfs through the two
 //    changed directions) is evaluated per pair (join_eval).
 // The throughput and probability of connectColorProb split the same way.
@@ -183,137 +183,7 @@ __device__ __forceinline__ PV rev_to(const PV& v, const PV& u) {
   r.inside = u.inside;
   return r;
 }
-__device__ __forceinline__ float seg_len(const PV& a, const PV& b) { return fmaxf(length(b.o - a.o), 1e-5f); }
 __device__ __forceinline__ bool rnd(const PV& v) { return (v.flags & kDirRandom) != 0u; }
-// the merge technique's pdf factors of connectMergeWeight (VCMTracer.cpp:400-409) past pf, pb
-__device__ __forceinline__ double merge_area(double p, const PV& v, float r, float norm) {
-  p *= RX_PI * r * r;
-  if (v.inside != kNone && v.contact == kNone) p *= 4.0 / 3.0 * r;
-  return p * norm;
-}
-
-// Light-subpath records for c = 0 .. n-1, from the stored vertices of one light path
-// (a window of four vertices, c - 2 .. c + 1, in registers).
-__device__ void light_mis(const DevScene& S, const CamDev& cam, const float4* lb, int n, float r, float norm,
-                          bool merges, MisL* out) {
-  PV l2, l1, v = load_pv(lb), nx;  // vertices c - 2, c - 1, c, c + 1
-  double pf = v.oprob, pf_prev = 0.0, sl = 0.0;
-  F3 thr = {1, 1, 1};
-  float prob = 1.0f;
-  for (int c = 0; c < n; c++) {
-    if (c + 1 < n) nx = load_pv(lb + 4 * (c + 1));
-    MisL m;
-    double al = 0.0, tl = 0.0;
-    if (c >= 1) {
-      const PV& a = l1;
-      float d = seg_len(a, v);
-      PV rv = rev_to(v, a);
-      al = cos_term(S, cam, a);
-      al /= (double)d * d;
-      if (rnd(v)) al *= origin_pdf(S, rv, a);
-      tl = rnd(a) && rnd(v) ? pf_prev : 0.0;
-      if (merges && rnd(v)) {
-        double p = pf_prev;
-        if (rnd(a)) p *= c - 1 > 0 ? dir_pdf(S, cam, l2, a, false) : dir_pdf(S, cam, a, a, true);
-        p *= origin_pdf(S, a, v);
-        p *= cos_term(S, cam, rv);
-        p /= (double)d * d;
-        tl += merge_area(p, v, r, norm);
-      }
-    }
-    m.sla = (float)(al * sl / pf);
-    m.tla = (float)(tl / pf);
-    m.prob = prob;
-    m.pad = 0.0f;
-    m.thr = thr;
-    m.pad2 = 0.0f;
-    out[c] = m;
-    if (c + 1 >= n) break;
-    // advance to c + 1
-    float d = seg_len(v, nx);
-    prob *= v.dprob * v.oprob;
-    thr = thr * v.c;
-    thr = thr * decay_of(S, v.inside, d);
-    thr = thr * cos_term(S, cam, v);
-    double pfn = pf * cos_term(S, cam, rev_to(nx, v));
-    pfn /= (double)d * d;
-    if (rnd(v)) {
-      pfn *= c > 0 ? dir_pdf(S, cam, l1, v, false) : dir_pdf(S, cam, v, v, true);
-      pfn *= origin_pdf(S, v, nx);
-    }
-    if (c >= 1) {
-      double g = al;
-      if (rnd(v)) g *= dir_pdf(S, cam, rev_to(nx, v), rev_to(v, l1), false);
-      sl = sl * g + tl;
-    }
-    pf_prev = pf;
-    pf = pfn;
-    l2 = l1;
-    l1 = v;
-    v = nx;
-  }
-}
-
-// Eye-subpath records for k = 0 .. n-1 (k >= 1 are merge vertices); e(k) gives vertex k.
-template <class Get>
-__device__ void eye_mis(const DevScene& S, const CamDev& cam, Get&& e, int n, float r, float norm, bool merges,
-                        MisE* out) {
-  double pb = e(0).oprob, pb_prev = 0.0, u = 0.0;
-  F3 thr = {1, 1, 1};
-  float prob = 1.0f;
-  for (int k = 0; k < n; k++) {
-    const PV v = e(k);
-    MisE m;
-    m.pb = pb;
-    m.pbr = (float)(pb_prev / pb);
-    m.sea = 0.0f;
-    if (k >= 1) {
-      const PV pe = e(k - 1);
-      float d = seg_len(v, pe);
-      double fe = cos_term(S, cam, pe);
-      fe /= (double)d * d;
-      fe *= origin_pdf(S, rev_to(v, pe), pe);
-      double se = u + (merges && k >= 2 && rnd(pe) ? merge_area(pb_prev, pe, r, norm) : 0.0);
-      m.sea = (float)(fe * se / pb);
-    }
-    m.thr = thr;
-    m.prob = prob;
-    out[k] = m;
-    if (k + 1 >= n) break;
-    // advance to k + 1
-    const PV up = e(k + 1);
-    float d = seg_len(v, up);
-    thr = thr * v.c;
-    thr = thr * decay_of(S, v.inside, d);
-    thr = thr * cos_term(S, cam, v);
-    prob *= v.dprob * v.oprob;
-    double pbn = pb * cos_term(S, cam, rev_to(up, v));
-    pbn /= (double)d * d;
-    if (rnd(v)) {
-      pbn *= k > 0 ? dir_pdf(S, cam, e(k - 1), v, false) : dir_pdf(S, cam, v, v, true);
-      pbn *= origin_pdf(S, v, up);
-    }
-    if (k >= 1) {
-      const PV pe = e(k - 1);
-      float dd = seg_len(v, pe);
-      PV rv = rev_to(v, pe);
-      double g = cos_term(S, cam, pe);
-      g /= (double)dd * dd;
-      double opf = origin_pdf(S, rv, pe);
-      if (rnd(v)) {
-        g *= dir_pdf(S, cam, rev_to(up, v), rv, false);
-        g *= opf;
-      }
-      double un = u * g;
-      if (rnd(v) && rnd(pe)) un += pb_prev;
-      if (merges && k >= 2 && rnd(pe)) un += merge_area(g * pb_prev * (rnd(v) ? 1.0 : opf), pe, r, norm);
-      u = un;
-    }
-    pb_prev = pb;
-    pb = pbn;
-  }
-}
-
 // connectRays (MCRenderer.cpp:50-106) for light vertex L (w[ci]) and eye vertex E
 // (w[ci+1]). Lm: the light vertex before L (null when ci = 0); pe: the eye vertex
 // before E (null when E is the camera vertex, t = 1). Where the reference's neighbour
@@ -552,12 +422,246 @@ __global__ void __launch_bounds__(128) k_sub_run(DevScene S, VcmParams P, SubSin
   if (nr) atomicAdd(rays, nr);
 }
 
-// The light subpaths' records, one thread per path, from the stored vertices (apart from
-// the sampling kernel, whose traversal stack and divergent bounce loop would hold them).
-__global__ void __launch_bounds__(128) k_light_mis(DevScene S, VcmParams P, const float4* lv, const int* llen,
-                                                   MisL* lmis) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P.n_light; p += gridDim.x * blockDim.x)
-    light_mis(S, P.cam, lv + 4 * ((size_t)p * P.maxv), llen[p], P.radius, P.norm, !P.bpt, lmis + (size_t)p * P.maxv);
+// bsdf_of and dir_pdf at a vertex whose contact normal `n` is at hand (records and merges):
+// `obj` is the vertex's contact object, or its inside object when it has no contact
+// (`volume`). The pdf of a vertex sampled at random, not of an emission.
+__device__ __forceinline__ F3 merge_bsdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
+  if (obj < 0) return F3{0, 0, 0};
+  const DevObject& ob = S.objects[obj];
+  if (volume) return ob.material == kVPM ? f3v(ob.sigma_s) * hg(ob.g, dot(in, out)) : F3{0, 0, 0};
+  if (ob.material == kEmissive) return dot(n, out) < 0.0f ? F3{0, 0, 0} : f3v(ob.color);
+  F3 f = {0, 0, 0};
+  if (!(dot(n, in) <= 0.0f && dot(n, out) >= 0.0f)) return f;
+  if (ob.material == kDiffuse || ob.material == kPhong)
+    f = f + (ob.material == kPhong ? f3v(ob.diffuse_color) : f3v(ob.color)) * (1.0f / RX_PI);
+  if (ob.material == kGlossy || ob.material == kPhong) {
+    const F3 c = f3v(ob.color), r = n * (-dot(n, in) * 2.0f) + in;
+    const float rw = dot(r, out);
+    if (rw > 0.0f) f = f + c * (maxc(c) * powf(rw, ob.coeff));
+  }
+  return f;
+}
+__device__ __forceinline__ float merge_pdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
+  if (obj < 0) return obj == kCameraObj ? 1.0f : 0.0f;
+  const DevObject& ob = S.objects[obj];
+  if (volume) {
+    if (ob.material != kVPM) return ob.material == kRefractive || ob.material == kReflective ? 1.0f : 0.0f;
+    const float albedo = lum(f3v(ob.sigma_s)) / lum(sigma_t(ob));
+    return albedo * hg(ob.g, dot(normalize(in), out));
+  }
+  switch (ob.material) {
+    case kDiffuse: return maxc(f3v(ob.color)) * cos_lobe_pdf(n, out, 1.0f);
+    case kRefractive:
+    case kReflective: return 1.0f;
+    case kGlossy: return cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff);
+    case kPhong:
+      return (maxc(f3v(ob.diffuse_color)) * cos_lobe_pdf(n, out, 1.0f) +
+              cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff)) / 2.0f;
+    default: return 0.0f;  // emitters, medium boundaries
+  }
+}
+
+__device__ __forceinline__ void img_add(float* img, int pixel, F3 c) {
+  atomicAdd(img + 3 * pixel, c.x);
+  atomicAdd(img + 3 * pixel + 1, c.y);
+  atomicAdd(img + 3 * pixel + 2, c.z);
+}
+
+// ---- subpath records --------------------------------------------------------------------
+// 1 / x in double precision: for x well within single precision's range the
+// single-precision reciprocal and two Newton steps (a double division is three times the
+// FP64 operations, and the FP64 pipe is what bounds the records), else the division.
+__device__ __forceinline__ double rcp64(double x) {
+  if (!(x > 1e-30 && x < 1e30)) return 1.0 / x;
+  double y = (double)(1.0f / (float)x);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+// Ray::getCosineTerm of a vertex with contact normal `n` along `d`.
+__device__ __forceinline__ float cos_at(const DevScene& S, int contact, F3 n, F3 d) {
+  const bool has_cos = contact == kCameraObj || (contact >= 0 && !is_vpm(S, contact));
+  return has_cos && length(d) > 0.5f ? fmaxf(fabsf(dot(n, d)), kCosMin) : 1.0f;
+}
+
+// The light (MisL) or eye (MisE) records of every stored subpath, a subpath per lane; a lane
+// whose subpath has ended takes the next one of the warp's share, so lanes stay busy. Each
+// step of the loop writes one vertex's record and forms what the edge to the next vertex
+// needs once: its normal, cosines, direction pdfs and transmittance pdfs, which the next
+// steps carry along. The pdf chains of connectMergeWeight (VCMTracer.cpp:321-428) are kept
+// as ratios of neighbouring vertices (pf[c+1] / pf[c] is the product of one edge's factors),
+// so the partial sums come already divided by the chain: per edge one reciprocal in double
+// instead of five divisions. At 2^20 light paths through the medium scene 0.38 ms against
+// 2.12 for a subpath per thread with the chains themselves (FP64 pipe 74% busy at 7.8 of 32
+// lanes); 512^2 eye paths 0.19 against 0.43.
+//
+// Light, at vertex c (a = c - 1): sl / pf[c] = s:  sla = al s,  tla = tl / pf[c],
+//   s <- (s al back + tla) pf[c] / pf[c+1].
+// Eye, at vertex k (a = k - 1): u / pb[k-1] = s:  sea = fe (s + M) pb[k-1] / pb[k],
+//   s <- (s g + C + M g) pb[k-1] / pb[k].
+// The light side also lists the vertices that can take part in a connection (`lmask`: random,
+// not on an emitter past the light's own vertex). The eye side adds the s = 0 technique (the
+// eye path ends on an emitter and the reference's mustUsePT holds: VCM, no interior vertex
+// sampled at random, weight pb[0] / (pb[0] + the two-vertex connection);
+// BidirectionalPathTracer, no two consecutive random vertices, weight pb[0] / pb[0]) and
+// writes each pixel's masks and number of connections.
+template <bool EYE>
+__global__ void __launch_bounds__(128) k_records(DevScene S, VcmParams P, const float4* __restrict__ verts,
+                                                 const int* __restrict__ lens, MisL* lmis, MisE* emis, uint32_t* lmask,
+                                                 uint2* cmask, unsigned long long* ccount, float* img) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = EYE ? P.n_pixels : P.n_light, nw = gridDim.x * 4, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const uint32_t per = (n + nw - 1) / nw, end = min(n, (w + 1) * per);
+  uint32_t next = min(n, w * per);
+  const bool merges = !P.bpt;
+  const double area = (double)(RX_PI * P.radius * P.radius) * P.norm, varea = area * (4.0 / 3.0 * P.radius);
+  bool active = false;
+  uint32_t p = 0, mask = 0;
+  int c = 0, len = 0;
+  const float4* vb = verts;
+  PV v{}, a{};
+  F3 nv{}, rd{}, thr{};  // v's normal; direction v -> a
+  float prob = 1.0f, cosA = 1.0f, opVA = 1.0f, opAV = 1.0f;
+  double id2 = 0.0, inv = 0.0, s = 0.0, pb = 0.0;  // 1 / |v - a|^2; chain ratio a / v; partial sum
+  F3 acc{};
+  bool rand_interior = false, rand_pair = false, first_rand = false, open = true;
+  while (true) {
+    const unsigned want = __ballot_sync(FULL, !active);
+    if (want && next < end) {
+      if (!active) {
+        p = next + __popc(want & ((1u << lane) - 1u));
+        if (p < end) {
+          active = true;
+          len = lens[p];
+          vb = verts + 4 * ((size_t)p * P.maxv);
+          v = load_pv(vb);
+          nv = contact_normal(S, P.cam, v);
+          c = 0;
+          mask = 0;
+          thr = F3{1, 1, 1};
+          prob = 1.0f;
+          s = inv = 0.0;
+          pb = v.oprob;
+          acc = F3{0, 0, 0};
+          rand_interior = rand_pair = first_rand = false;
+          open = true;
+        }
+      }
+      next += __popc(want);
+    }
+    if (!__any_sync(FULL, active)) break;
+    if (!active) continue;
+    const bool rv = rnd(v), ra = c >= 1 && rnd(a);
+    const double fe = cosA * id2;  // (c >= 1)
+    double al = 0.0, t = 0.0, M = 0.0;
+    if constexpr (EYE) {
+      MisE m;
+      m.pb = pb;
+      m.pbr = (float)inv;
+      M = merges && c >= 2 && ra ? (a.inside != kNone && a.contact == kNone ? varea : area) : 0.0;
+      m.sea = c >= 1 ? (float)(fe * opVA * (s + M) * inv) : 0.0f;
+      m.thr = thr;
+      m.prob = prob;
+      emis[(size_t)p * P.maxv + c] = m;
+      const bool emit = is_emissive(S, v.contact);
+      if (rv && !emit) mask |= 1u << c;
+      if (c == 0) first_rand = rv;
+      if (c >= 1) rand_pair |= ra && rv;  // pairs within e[0..c]
+      if (c >= 1 && open) {               // s = 0 with t = c + 1 (interior e[1..c-1], pairs within e[0..c])
+        if (P.bpt ? rand_pair : rand_interior) {
+          open = false;
+        } else if (emit) {
+          const F3 col = v.c * thr;
+          const float pr = (v.dprob * v.oprob) * prob;
+          if (pr > 0.0f && length(col) > 0.0f) {
+            float wt = pb > 0.0 && pb < INFINITY ? 1.0f : 0.0f;      // pb[0] / pb[0]
+            if (!P.bpt && wt > 0.0f && c == 1 && rv && first_rand) {  // pb[0] / (pb[0] + pf[0] pb[1])
+              const float res = 1.0f / (1.0f + v.oprob * m.pbr);
+              wt = res >= 0.0f ? res : 0.0f;
+            }
+            const F3 add = col * (wt / pr);
+            if (length(add) > 0.0f) acc = acc + add;
+          }
+        }
+      }
+      if (c >= 1) rand_interior |= rv;  // e[c] is interior for every longer path
+    } else {
+      if (c >= 1) {
+        al = rv ? fe * opVA : fe;
+        if (ra && rv) t = inv;
+        if (merges && rv) t += (v.inside != kNone && v.contact == kNone ? varea : area) * (ra ? 1.0f : opAV);
+      }
+      MisL m;
+      m.sla = (float)(al * s);
+      m.tla = (float)t;
+      m.prob = prob;
+      m.pad = 0.0f;
+      m.thr = thr;
+      m.pad2 = 0.0f;
+      lmis[(size_t)p * P.maxv + c] = m;
+      if (rv && (c == 0 || !is_emissive(S, v.contact))) mask |= 1u << c;
+    }
+    if (c + 1 >= len) {  // the subpath's last vertex
+      if constexpr (EYE) {
+        if (acc.x != 0.0f || acc.y != 0.0f || acc.z != 0.0f) img_add(img, (int)p, acc);
+        const uint32_t lm = lmask[p % P.n_light];
+        cmask[p] = make_uint2(mask, lm);
+        ccount[p] = (unsigned long long)(__popc(mask) * __popc(lm));
+      } else {
+        lmask[p] = mask;
+      }
+      active = false;
+      continue;
+    }
+    // the edge to the next vertex
+    const PV x = load_pv(vb + 4 * (c + 1));
+    const F3 nx = contact_normal(S, P.cam, x), e = v.o - x.o;
+    const float el = length(e), d = fmaxf(el, 1e-5f);
+    const F3 xd = el > 0.0f ? e * (1.0f / el) : e;  // x -> v
+    const float cosV = cos_at(S, v.contact, nv, v.d), cosR = cos_at(S, x.contact, nx, xd);
+    const int obj = v.contact != kNone ? v.contact : v.inside;
+    float dp = 1.0f, opVX = 1.0f, opXV = 1.0f, back = 1.0f;
+    if (is_vpm(S, v.inside)) {
+      const DevObject& ob = S.objects[v.inside];
+      const float ps = P_surface(ob, d), pm = p_medium(ob, d);
+      opVX = x.contact != kNone ? ps : pm;
+      opXV = v.contact != kNone ? ps : pm;
+    }
+    const bool vol = v.contact == kNone;
+    if (rv) {
+      dp = c > 0 ? merge_pdf(S, obj, vol, nv, a.d, v.d)
+                 : (v.contact == kCameraObj ? 1.0f : cos_lobe_pdf(nv, v.d, 1.0f));
+      if (c > 0) back = merge_pdf(S, vol ? a.inside : v.contact, vol, nv, xd, rd);
+    }
+    thr = thr * v.c;
+    thr = thr * decay_of(S, v.inside, d);
+    thr = thr * cosV;
+    prob *= v.dprob * v.oprob;
+    const double d2 = (double)d * d, nid2 = rcp64(d2);
+    double f = cosR;  // pf[c+1] / pf[c] (pb for the eye side) times d^2
+    if (rv) f *= (double)dp * opVX;
+    if constexpr (EYE) {
+      if (c >= 1) {
+        double g = fe;
+        if (rv) g *= (double)back * opVA;
+        s = (s * g + (rv && ra ? 1.0 : 0.0) + M * g * (rv ? 1.0f : opVA)) * inv;
+      }
+      pb *= f * nid2;
+    } else if (c >= 1) {
+      s = s * (rv ? al * back : al) + t;
+    }
+    inv = d2 * rcp64(f);
+    if (!EYE) s *= inv;
+    id2 = nid2;
+    cosA = cosV;
+    opVA = opXV;
+    opAV = opVX;
+    rd = xd;
+    a = v;
+    v = x;
+    nv = nx;
+    c++;
+  }
 }
 
 // ---- hash grid ---------------------------------------------------------------------------
@@ -786,78 +890,14 @@ __device__ __forceinline__ void trans_to_pixel(const CamDev& c, F3 point, float&
   py = c.height / 2.0f - dot(v, c.up) * ratio - 0.5f;
 }
 
-__device__ __forceinline__ void img_add(float* img, int pixel, F3 c) {
-  atomicAdd(img + 3 * pixel, c.x);
-  atomicAdd(img + 3 * pixel + 1, c.y);
-  atomicAdd(img + 3 * pixel + 2, c.z);
-}
-
 // ---- eye subpaths and connections ---------------------------------------------------------
 // colorByConnectingPaths (VCMTracer.cpp:430-562) joins every light vertex ci of the
 // pixel's light path with every eye vertex k (s = ci + 1, t = k + 1), plus the pure
-// eye path (s = 0). k_sub_run samples and stores the eye subpath; k_eye_post
+// eye path (s = 0). k_sub_run samples and stores the eye subpath; k_records
 // builds its records, adds the s = 0 technique, and lists which vertices can take part
 // in a connection (sampled
 // at random, not on an emitter past the light's own vertex); the (k, ci) pairs are then
 // evaluated one per lane with their shadow rays (k_conn_eval).
-
-// Per pixel, from its stored eye subpath: the records, the s = 0 technique (the eye
-// path ends on an emitter and the reference's mustUsePT holds: VCM, no interior vertex
-// sampled at random, weight pb[0] / (pb[0] + the two-vertex connection);
-// BidirectionalPathTracer, no two consecutive random vertices, weight pb[0] / pb[0]),
-// and the lists of eye and light vertices that can take part in a connection.
-__global__ void __launch_bounds__(128) k_eye_post(DevScene S, VcmParams P, const float4* lv, const int* llen,
-                                                  const float4* ev, const int* elen, MisE* emis, uint2* cmask,
-                                                  unsigned long long* ccount, float* img) {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P.n_pixels; p += gridDim.x * blockDim.x) {
-    const float4* eb = ev + 4 * ((size_t)p * P.maxv);
-    const int ne = elen[p];
-    MisE* me = emis + (size_t)p * P.maxv;
-    eye_mis(S, P.cam, [&](int k) { return load_pv(eb + 4 * k); }, ne, P.radius, P.norm, !P.bpt, me);
-    F3 acc = {0, 0, 0};
-    uint32_t em = 0;
-    bool rand_interior = false, rand_pair = false, prev_rand = false, first_rand = false, open = true;
-    for (int k = 0; k < ne; k++) {
-      const PV v = load_pv(eb + 4 * k);
-      const bool rv = rnd(v);
-      if (k == 0) first_rand = rv;
-      if (k >= 1) rand_pair |= prev_rand && rv;  // pairs within e[0..k]
-      if (rv && !is_emissive(S, v.contact)) em |= 1u << k;
-      if (k >= 1 && open) {  // s = 0 with t = k + 1 (interior e[1..k-1], pairs within e[0..k])
-        if (P.bpt ? rand_pair : rand_interior) {
-          open = false;
-        } else if (is_emissive(S, v.contact)) {
-          const MisE m = me[k];
-          F3 col = v.c * m.thr;
-          float prob = (v.dprob * v.oprob) * m.prob;
-          if (prob > 0.0f && length(col) > 0.0f) {
-            float wt = m.pb > 0.0 && m.pb < INFINITY ? 1.0f : 0.0f;      // pb[0] / pb[0]
-            if (!P.bpt && wt > 0.0f && k == 1 && rv && first_rand) {  // pb[0] / (pb[0] + pf[0] pb[1])
-              float res = 1.0f / (1.0f + v.oprob * m.pbr);
-              wt = res >= 0.0f ? res : 0.0f;
-            }
-            F3 c = col * (wt / prob);
-            if (length(c) > 0.0f) acc = acc + c;
-          }
-        }
-      }
-      if (k >= 1) rand_interior |= rv;  // e[k] is interior for every longer path
-      prev_rand = rv;
-    }
-    img_add(img, (int)p, acc);
-    uint32_t lm = 0;
-    const uint32_t lp = p % P.n_light;
-    const int nl = llen[lp];
-    for (int ci = 0; ci < nl; ci++) {
-      float4 t4 = lv[4 * ((size_t)lp * P.maxv + ci) + 3];
-      int contact = __float_as_int(t4.x);
-      uint32_t flags = __float_as_uint(t4.w);
-      if ((flags & kDirRandom) && (ci == 0 || !is_emissive(S, contact))) lm |= 1u << ci;
-    }
-    cmask[p] = make_uint2(em, lm);
-    ccount[p] = (unsigned long long)(__popc(em) * __popc(lm));
-  }
-}
 
 // Pairs [win0, win0 + cap) of the scanned order: pixel and eye vertex (q = p * maxv + k)
 // and light vertex of each.
@@ -1013,12 +1053,11 @@ __global__ void __launch_bounds__(128) k_shadow_thread(DevScene S, const ShadowQ
 
 // Per pixel: the eye subpath and colorByConnectingPaths by the reference's loops over each
 // whole joined path, a shadow ray per connection in the same thread. Kept as the check of
-// k_sub_run + k_eye_post + k_conn_eval (RX_VCM_FULL_PATH_MIS, which also samples the
+// k_sub_run + k_records + k_conn_eval (RX_VCM_FULL_PATH_MIS, which also samples the
 // light subpaths one per thread, k_vcm_light: the same random numbers, so the same
 // subpaths as k_sub_run).
 __global__ void __launch_bounds__(128) k_vcm_eye_full(DevScene S, VcmParams P, const float4* lv, const int* llen,
-                                                 float4* ev, int* elen, MisE* emis, float* img,
-                                                 unsigned long long* rays) {
+                                                 float4* ev, int* elen, float* img, unsigned long long* rays) {
   uint32_t stride = gridDim.x * blockDim.x;
   unsigned long long nrays = 0, nshadow = 0;
   const float r = P.radius;
@@ -1032,7 +1071,6 @@ __global__ void __launch_bounds__(128) k_vcm_eye_full(DevScene S, VcmParams P, c
     nrays += (unsigned long long)ne;
     for (int k = 0; k < ne; k++) store_pv(ev + 4 * ((size_t)p * P.maxv + k), eye[k]);
     elen[p] = ne;
-    eye_mis(S, P.cam, [&](int k) { return eye[k]; }, ne, r, P.norm, !P.bpt, emis + (size_t)p * P.maxv);
     F3 acc = {0, 0, 0};
     uint32_t lp = p % P.n_light;
     int nl = llen[lp];
@@ -1264,44 +1302,6 @@ __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, cons
     e.prand = rnd(pe) ? 1u : 0u;
     e.pixel = q / P.maxv;
     out[j] = e;
-  }
-}
-
-// bsdf_of and dir_pdf at a merge's vertices, whose contact normal `n` is at hand: `obj` is
-// the vertex's contact object, or its inside object when it has no contact (`volume`).
-__device__ __forceinline__ F3 merge_bsdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
-  if (obj < 0) return F3{0, 0, 0};
-  const DevObject& ob = S.objects[obj];
-  if (volume) return ob.material == kVPM ? f3v(ob.sigma_s) * hg(ob.g, dot(in, out)) : F3{0, 0, 0};
-  if (ob.material == kEmissive) return dot(n, out) < 0.0f ? F3{0, 0, 0} : f3v(ob.color);
-  F3 f = {0, 0, 0};
-  if (!(dot(n, in) <= 0.0f && dot(n, out) >= 0.0f)) return f;
-  if (ob.material == kDiffuse || ob.material == kPhong)
-    f = f + (ob.material == kPhong ? f3v(ob.diffuse_color) : f3v(ob.color)) * (1.0f / RX_PI);
-  if (ob.material == kGlossy || ob.material == kPhong) {
-    const F3 c = f3v(ob.color), r = n * (-dot(n, in) * 2.0f) + in;
-    const float rw = dot(r, out);
-    if (rw > 0.0f) f = f + c * (maxc(c) * powf(rw, ob.coeff));
-  }
-  return f;
-}
-__device__ __forceinline__ float merge_pdf(const DevScene& S, int obj, bool volume, F3 n, F3 in, F3 out) {
-  if (obj < 0) return 0.0f;
-  const DevObject& ob = S.objects[obj];
-  if (volume) {
-    if (ob.material != kVPM) return ob.material == kRefractive || ob.material == kReflective ? 1.0f : 0.0f;
-    const float albedo = lum(f3v(ob.sigma_s)) / lum(sigma_t(ob));
-    return albedo * hg(ob.g, dot(normalize(in), out));
-  }
-  switch (ob.material) {
-    case kDiffuse: return maxc(f3v(ob.color)) * cos_lobe_pdf(n, out, 1.0f);
-    case kRefractive:
-    case kReflective: return 1.0f;
-    case kGlossy: return cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff);
-    case kPhong:
-      return (maxc(f3v(ob.diffuse_color)) * cos_lobe_pdf(n, out, 1.0f) +
-              cos_lobe_pdf(n * (-dot(n, in) * 2.0f) + in, out, ob.coeff)) / 2.0f;
-    default: return 0.0f;  // emitters, medium boundaries
   }
 }
 
@@ -1884,6 +1884,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   if ((e = al(19, (size_t)P.n_light * P.maxv * sizeof(MisL))) != cudaSuccess) return e;         // light MIS records
   if ((e = al(20, (size_t)P.n_pixels * P.maxv * sizeof(MisE))) != cudaSuccess) return e;        // eye MIS records
   if ((e = al(21, (size_t)P.n_pixels * sizeof(uint2))) != cudaSuccess) return e;                // connection masks
+  if ((e = al(25, (size_t)P.n_light * sizeof(uint32_t))) != cudaSuccess) return e;              // light masks
   if ((e = al(22, (size_t)cap * sizeof(float4))) != cudaSuccess) return e;                      // sorted photon positions
   if ((e = al(23, (size_t)cap * kJoin * sizeof(float4))) != cudaSuccess) return e;              // photon join data
   if (!P.bpt) {  // merge queries in spatial order: list, keys, sorted order, key counts, count
@@ -1905,7 +1906,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   int grid = c->trace_cfg.sms * 4;
   // shadow rays on the persistent 4-wide walk when the tree fits its stack
   const bool wide_shadow = c->d_bvh4.p && 3 * c->bvh4.max_depth + 1 <= 64;
-  int sub_grid[2] = {0, 0}, merge_grid = 0;  // resident blocks of k_sub_run<false>, <true>, and of k_merge
+  int sub_grid[2] = {0, 0}, merge_grid = 0, rec_grid[2] = {0, 0};  // resident blocks: k_sub_run<false>, <true>; k_merge; k_records
   {
     int per = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<false>, 128, 0)) != cudaSuccess) return e;
@@ -1914,6 +1915,10 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     sub_grid[1] = c->trace_cfg.sms * std::max(per, 1);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_merge, 128, 0)) != cudaSuccess) return e;
     merge_grid = c->trace_cfg.sms * std::max(per, 1);
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_records<false>, 128, 0)) != cudaSuccess) return e;
+    rec_grid[0] = c->trace_cfg.sms * std::max(per, 1);
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_records<true>, 128, 0)) != cudaSuccess) return e;
+    rec_grid[1] = c->trace_cfg.sms * std::max(per, 1);
   }
   Event e0, e1, m0, m1;  // render; merge gather of an iteration (with stats)
   if ((e = e0.create()) != cudaSuccess || (e = e1.create()) != cudaSuccess) return e;
@@ -1951,7 +1956,8 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
                                        bufs[3].as<int>(), nph, cap, ctr);
     else
       subpaths(true);
-    k_light_mis<<<grid, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[19].as<MisL>());
+    k_records<false><<<rec_grid[0], 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[19].as<MisL>(),
+                                                 nullptr, bufs[25].as<uint32_t>(), nullptr, nullptr, nullptr);
     const float cell = 2.0f * radius;
     Grid G{cell, buckets - 1, bufs[7].as<unsigned>(), bufs[22].as<float4>(), bufs[5].as<int>(), bufs[23].as<float4>()};
     if (!P.bpt) {  // the photon grid
@@ -1992,12 +1998,12 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     unsigned long long total = 0;
     if (full_mis) {
       k_vcm_eye_full<<<grid, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[12].as<float4>(),
-                                          bufs[13].as<int>(), bufs[20].as<MisE>(), bufs[10].as<float>(), ctr + 1);
+                                          bufs[13].as<int>(), bufs[10].as<float>(), ctr + 1);
     } else {
       subpaths(false);
-      k_eye_post<<<grid * 2, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[12].as<float4>(),
-                                          bufs[13].as<int>(), bufs[20].as<MisE>(), bufs[21].as<uint2>(), qc,
-                                          bufs[10].as<float>());
+      k_records<true><<<rec_grid[1], 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[13].as<int>(), nullptr,
+                                                  bufs[20].as<MisE>(), bufs[25].as<uint32_t>(), bufs[21].as<uint2>(), qc,
+                                                  bufs[10].as<float>());
       if ((e = scan_total(P.n_pixels, total)) != cudaSuccess) return e;
       // the shadow-ray queue: at most one ray per connection of a window
       const size_t sq_bytes = (size_t)std::min<unsigned long long>(pair_alloc, std::max(total, 1ull)) * sizeof(ShadowQ);
