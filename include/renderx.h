@@ -217,6 +217,8 @@ typedef struct rx_render_stats {
 /* Replaces the process-global GPU state of IntersectionGPU::init
  * (reference src/IntersectionGPU.cpp:16-44). */
 rx_status rx_create(rx_context** out, int device);
+/* A context keeps the device buffers of its renders between calls, at most 8 GiB; they go
+ * with it. */
 void rx_destroy(rx_context* ctx);
 const char* rx_last_error(const rx_context* ctx);
 /* Build identification string (kernels, architecture). */

@@ -19,6 +19,14 @@ rx_status upload(rx_context* c, DevBuf& b, const void* src, size_t bytes, const 
   return c->cuda(cudaMemcpy(b.p, src, bytes, cudaMemcpyHostToDevice), what);
 }
 
+// The mean of a device film of sums (`n` samples over all pixels) to the caller's buffer.
+rx_status mean_to_host(rx_context* c, double* film, size_t pixels, uint64_t n, double* out) {
+  rx_status s = c->cuda(rx::film_mean(film, pixels, n, c->stream), "film mean");
+  if (s != RX_OK) return s;
+  s = c->cuda(cudaMemcpyAsync(out, film, pixels * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "film copy");
+  return s != RX_OK ? s : c->cuda(cudaStreamSynchronize(c->stream), "film copy");
+}
+
 }  // namespace
 
 extern "C" {
@@ -71,6 +79,7 @@ void rx_destroy(rx_context* c) {
     for (cudaEvent_t e : c->timing_ev) cudaEventDestroy(e);
     rx::guide_free(c->guide);
     c->guide = nullptr;
+    c->ws.trim(0);
     if (c->stream) cudaStreamDestroy(c->stream);
     for (auto s : c->copy_stream)
       if (s) cudaStreamDestroy(s);
@@ -413,28 +422,22 @@ rx_status rx_render_pt(rx_context* c, const rx_camera* cam, const rx_pt_options*
     if (!rx::guide_ready(c->guide)) return c->fail(RX_ERR_STATE, "guided rendering needs rx_guide_init");
   }
   DeviceGuard g(c->device);
-  size_t np = (size_t)cam->width * cam->height;
-  DevBuf sum, sq;
+  const size_t np = (size_t)cam->width * cam->height, film_bytes = np * 3 * sizeof(double);
+  rx::Workspace::Frame frame(c->ws);
+  rx::WsBuf sum, sq;
   rx_status s;
-  if ((s = c->cuda(sum.alloc(np * 3 * sizeof(double)), "film")) != RX_OK) return s;
-  if (film_sq && (s = c->cuda(sq.alloc(np * 3 * sizeof(double)), "film")) != RX_OK) return s;
-  cudaMemsetAsync(sum.p, 0, sum.bytes, c->stream);
-  if (film_sq) cudaMemsetAsync(sq.p, 0, sq.bytes, c->stream);
+  if ((s = c->cuda(sum.alloc(c->ws, film_bytes), "film")) != RX_OK) return s;
+  if (film_sq && (s = c->cuda(sq.alloc(c->ws, film_bytes), "film")) != RX_OK) return s;
+  cudaMemsetAsync(sum.p, 0, film_bytes, c->stream);
+  if (film_sq) cudaMemsetAsync(sq.p, 0, film_bytes, c->stream);
   rx_render_stats st{};
   if ((s = c->cuda(rx::render_pt(c, *cam, *opts, sum.as<double>(), film_sq ? sq.as<double>() : nullptr, &st, c->stream),
                    "render_pt")) != RX_OK)
     return s;
   // paths run sample-major: with st.paths done, pixel q holds done / np samples, one
   // more when q < done % np (every pixel holds spp when the render completed)
-  const uint64_t done = st.paths;
-  auto count = [&](size_t q) { return (double)(done / np + (q < done % np ? 1 : 0)); };
-  std::vector<double> h(np * 3);
-  if ((s = c->cuda(cudaMemcpy(h.data(), sum.p, sum.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
-  for (size_t k = 0; k < h.size(); k++) film_rgb[k] = count(k / 3) > 0 ? h[k] / count(k / 3) : 0.0;
-  if (film_sq) {
-    if ((s = c->cuda(cudaMemcpy(h.data(), sq.p, sq.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
-    for (size_t k = 0; k < h.size(); k++) film_sq[k] = count(k / 3) > 0 ? h[k] / count(k / 3) : 0.0;
-  }
+  if ((s = mean_to_host(c, sum.as<double>(), np, st.paths, film_rgb)) != RX_OK) return s;
+  if (film_sq && (s = mean_to_host(c, sq.as<double>(), np, st.paths, film_sq)) != RX_OK) return s;
   if (stats) *stats = st;
   return RX_OK;
 }
@@ -468,9 +471,10 @@ rx_status rx_render_pt_batch(rx_context* c, const rx_batch_item* items, uint32_t
     pixels += (uint64_t)cam.width * cam.height;
   }
   DeviceGuard g(c->device);
-  DevBuf film;
+  rx::Workspace::Frame frame(c->ws);
+  rx::WsBuf film;
   rx_status s;
-  if ((s = c->cuda(film.alloc(pixels * 3 * sizeof(double)), "film")) != RX_OK) return s;
+  if ((s = c->cuda(film.alloc(c->ws, pixels * 3 * sizeof(double)), "film")) != RX_OK) return s;
   cudaMemsetAsync(film.p, 0, film.bytes, c->stream);
   rx::PtRun run;
   run.paths_per_pass = opts ? opts->paths_per_pass : 0;
@@ -481,12 +485,28 @@ rx_status rx_render_pt_batch(rx_context* c, const rx_batch_item* items, uint32_t
   if ((s = c->cuda(rx::render_pt_jobs(c, jobs.data(), (int)n, run, film.as<double>(), nullptr, &st, &shape, c->stream),
                    "render_pt_batch")) != RX_OK)
     return s;
-  std::vector<double> h(pixels * 3);
-  if ((s = c->cuda(cudaMemcpy(h.data(), film.p, film.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
-  for (uint32_t k = 0; k < n; k++) {
-    size_t np = (size_t)items[k].camera.width * items[k].camera.height * 3;
-    const double* src = h.data() + jobs[k].film_base * 3;
-    for (size_t q = 0; q < np; q++) items[k].film_rgb[q] = src[q] / items[k].options.spp;
+  if (pixels >= 1024 * (uint64_t)n) {  // 24 KB a film or more: divide on the device, copy each film
+    for (uint32_t k = 0; k < n; k++) {
+      const uint64_t np = (uint64_t)items[k].camera.width * items[k].camera.height;
+      double* f = film.as<double>() + jobs[k].film_base * 3;
+      if ((s = c->cuda(rx::film_mean(f, np, np * items[k].options.spp, c->stream), "film mean")) != RX_OK) return s;
+    }
+    for (uint32_t k = 0; k < n; k++) {
+      const size_t bytes = (size_t)items[k].camera.width * items[k].camera.height * 3 * sizeof(double);
+      if ((s = c->cuda(cudaMemcpyAsync(items[k].film_rgb, film.as<double>() + jobs[k].film_base * 3, bytes,
+                                       cudaMemcpyDeviceToHost, c->stream),
+                       "film copy")) != RX_OK)
+        return s;
+    }
+    if ((s = c->cuda(cudaStreamSynchronize(c->stream), "film copy")) != RX_OK) return s;
+  } else {  // many tiny films: one copy
+    std::vector<double> h(pixels * 3);
+    if ((s = c->cuda(cudaMemcpy(h.data(), film.p, film.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
+    for (uint32_t k = 0; k < n; k++) {
+      size_t np = (size_t)items[k].camera.width * items[k].camera.height * 3;
+      const double* src = h.data() + jobs[k].film_base * 3;
+      for (size_t q = 0; q < np; q++) items[k].film_rgb[q] = src[q] / items[k].options.spp;
+    }
   }
   if (opts) {
     opts->chosen_blocks_per_sm = shape.blocks_per_sm;
@@ -510,16 +530,15 @@ static rx_status render_bidirectional(rx_context* c, const rx_camera* cam, const
   if (c->scene.num_lights == 0) return c->fail(RX_ERR_INVALID, "vertex connection and merging needs an emitter");
   DeviceGuard g(c->device);
   size_t np = (size_t)cam->width * cam->height;
-  DevBuf film;
+  rx::Workspace::Frame frame(c->ws);
+  rx::WsBuf film;
   rx_status s;
-  if ((s = c->cuda(film.alloc(np * 3 * sizeof(double)), "film")) != RX_OK) return s;
+  if ((s = c->cuda(film.alloc(c->ws, np * 3 * sizeof(double)), "film")) != RX_OK) return s;
   cudaMemsetAsync(film.p, 0, film.bytes, c->stream);
   rx_render_stats st{};
   if ((s = c->cuda(rx::render_vcm(c, *cam, *opts, film.as<double>(), &st, c->stream), "render_vcm")) != RX_OK) return s;
-  std::vector<double> h(np * 3);
-  if ((s = c->cuda(cudaMemcpy(h.data(), film.p, film.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
-  const double iters = (double)(st.paths / np);  // iterations done (fewer under a time budget)
-  for (size_t k = 0; k < h.size(); k++) film_rgb[k] = h[k] / iters;
+  // st.paths = pixels x iterations done (fewer under a time budget)
+  if ((s = mean_to_host(c, film.as<double>(), np, st.paths, film_rgb)) != RX_OK) return s;
   if (stats) *stats = st;
   return RX_OK;
 }
@@ -556,16 +575,15 @@ rx_status rx_render_pm(rx_context* c, const rx_camera* cam, const rx_pm_options*
   if (c->scene.num_lights == 0) return c->fail(RX_ERR_INVALID, "photon mapping needs an emitter");
   DeviceGuard g(c->device);
   size_t np = (size_t)cam->width * cam->height;
-  DevBuf film;
+  rx::Workspace::Frame frame(c->ws);
+  rx::WsBuf film;
   rx_status s;
-  if ((s = c->cuda(film.alloc(np * 3 * sizeof(double)), "film")) != RX_OK) return s;
+  if ((s = c->cuda(film.alloc(c->ws, np * 3 * sizeof(double)), "film")) != RX_OK) return s;
   cudaMemsetAsync(film.p, 0, film.bytes, c->stream);
   rx_render_stats st{};
   if ((s = c->cuda(rx::render_pm(c, *cam, *opts, film.as<double>(), &st, c->stream), "render_pm")) != RX_OK) return s;
-  std::vector<double> h(np * 3);
-  if ((s = c->cuda(cudaMemcpy(h.data(), film.p, film.bytes, cudaMemcpyDeviceToHost), "film copy")) != RX_OK) return s;
-  const double iters = (double)(st.paths / np);  // iterations done (fewer under a time budget)
-  for (size_t k = 0; k < h.size(); k++) film_rgb[k] = h[k] / iters;
+  // st.paths = pixels x iterations done (fewer under a time budget)
+  if ((s = mean_to_host(c, film.as<double>(), np, st.paths, film_rgb)) != RX_OK) return s;
   if (stats) *stats = st;
   return RX_OK;
 }

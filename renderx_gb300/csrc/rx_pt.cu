@@ -717,16 +717,28 @@ __global__ void k_net_pad(int nnet, unsigned* ncount, const uint32_t* seg, int* 
 // -------------------------------------------------------------------------------------
 // Host driver
 // -------------------------------------------------------------------------------------
-static cudaError_t alloc_soa(PathSoA& s, std::vector<DevBuf>& bufs, size_t n) {
+static cudaError_t alloc_soa(PathSoA& s, Workspace& ws, size_t n) {
   size_t sizes[6] = {16, 16, 16, 16, 16, 8};
   void** ptrs[6] = {(void**)&s.o, (void**)&s.d, (void**)&s.T, (void**)&s.L, (void**)&s.info, (void**)&s.id};
   for (int k = 0; k < 6; k++) {
-    bufs.emplace_back();
-    cudaError_t e = bufs.back().alloc(sizes[k] * n);
+    cudaError_t e = ws.alloc(sizes[k] * n, ptrs[k]);
     if (e != cudaSuccess) return e;
-    *ptrs[k] = bufs.back().p;
   }
   return cudaSuccess;
+}
+
+// The divisions run where the sums are: on the host they cost a 1024^2 frame milliseconds.
+__global__ void k_film_mean(double* film, uint64_t pixels, uint64_t n) {
+  const uint64_t each = n / pixels, more = n % pixels, stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < 3 * pixels; k += stride) {
+    const uint64_t cnt = each + (k / 3 < more ? 1 : 0);
+    film[k] = cnt ? film[k] / (double)cnt : 0.0;
+  }
+}
+cudaError_t film_mean(double* film, uint64_t pixels, uint64_t n, cudaStream_t s) {
+  if (pixels == 0) return cudaSuccess;
+  k_film_mean<<<(unsigned)std::min<uint64_t>((3 * pixels + 255) / 256, 2048), 256, 0, s>>>(film, pixels, n);
+  return cudaGetLastError();
 }
 
 PtParams make_pt_params(const rx_context* c, const rx_camera& cam, const rx_pt_options& opt) {
@@ -934,12 +946,12 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
   const uint32_t slots = (uint32_t)slots64;
   const int sms = c->trace_cfg.sms;
 
-  std::vector<DevBuf> bufs;
+  Workspace::Frame frame(c->ws);
   cudaError_t e;
   auto alloc = [&](size_t bytes) -> void* {
-    bufs.emplace_back();
-    if ((e = bufs.back().alloc(bytes)) != cudaSuccess) return nullptr;
-    return bufs.back().p;
+    void* p = nullptr;
+    if ((e = c->ws.alloc(bytes, &p)) != cudaSuccess) return nullptr;
+    return p;
   };
   auto upload = [&](const void* src, size_t bytes) -> void* {
     void* p = alloc(bytes);
@@ -963,8 +975,8 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
     W.L.quota = d_quota;
     cudaMemsetAsync(W.L.taken, 0, (size_t)nj * 8, s);
   }
-  if ((e = alloc_soa(W.A, bufs, slots)) != cudaSuccess) return e;
-  if ((e = alloc_soa(W.B, bufs, slots)) != cudaSuccess) return e;
+  if ((e = alloc_soa(W.A, c->ws, slots)) != cudaSuccess) return e;
+  if ((e = alloc_soa(W.B, c->ws, slots)) != cudaSuccess) return e;
   if (!(W.hit = static_cast<int2*>(alloc(slots * sizeof(int2))))) return e;
   if (!(W.ctr = static_cast<unsigned long long*>(alloc(64 * sizeof(unsigned long long))))) return e;
   W.cnt = reinterpret_cast<unsigned*>(W.ctr + 8);

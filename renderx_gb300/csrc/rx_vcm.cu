@@ -1858,9 +1858,10 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   const unsigned cap = P.bpt ? 1u : P.n_light * P.maxv;  // photon capacity (none without merging)
   unsigned buckets = 1u << 16;
   while (buckets < cap && buckets < (1u << 26)) buckets <<= 1;
-  std::vector<DevBuf> bufs(33);
+  Workspace::Frame frame(c->ws);
+  std::vector<WsBuf> bufs(33);
   cudaError_t e;
-  auto al = [&](int k, size_t bytes) { return bufs[k].alloc(bytes); };
+  auto al = [&](int k, size_t bytes) { return bufs[k].alloc(c->ws, bytes); };
   if ((e = al(26, 16)) != cudaSuccess) return e;  // subpath cursors
   if ((e = al(0, (size_t)P.n_light * P.maxv * 4 * sizeof(float4))) != cudaSuccess) return e;  // light vertices
   if ((e = al(1, (size_t)P.n_light * sizeof(int))) != cudaSuccess) return e;
@@ -1990,8 +1991,8 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       total = tail[0] + tail[1];
       if (err == cudaSuccess && total > pair_alloc && pair_alloc < pair_cap) {
         pair_alloc = (uint32_t)std::min<unsigned long long>(pair_cap, std::max<unsigned long long>(total, 2ull * pair_alloc));
-        if ((err = bufs[17].alloc((size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return err;
-        err = bufs[18].alloc((size_t)pair_alloc * sizeof(int));
+        if ((err = al(17, (size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return err;
+        err = al(18, (size_t)pair_alloc * sizeof(int));
       }
       return err;
     };
@@ -2007,7 +2008,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       if ((e = scan_total(P.n_pixels, total)) != cudaSuccess) return e;
       // the shadow-ray queue: at most one ray per connection of a window
       const size_t sq_bytes = (size_t)std::min<unsigned long long>(pair_alloc, std::max(total, 1ull)) * sizeof(ShadowQ);
-      if (bufs[32].bytes < sq_bytes && (e = bufs[32].alloc(sq_bytes)) != cudaSuccess) return e;
+      if (bufs[32].bytes < sq_bytes && (e = al(32, sq_bytes)) != cudaSuccess) return e;
       unsigned* sq_n = reinterpret_cast<unsigned*>(ctr + 13);
       unsigned long long* sq_cursor = ctr + 12;
       for (unsigned long long w0 = 0; w0 < total; w0 += pair_alloc) {
@@ -2115,9 +2116,10 @@ cudaError_t render_pm(rx_context* c, const rx_camera& cam, const rx_pm_options& 
   unsigned buckets = 1u << 16;
   while (buckets < cap && buckets < (1u << 26)) buckets <<= 1;
   const unsigned nscan = buckets + 1, nblk = (nscan + 1023) / 1024;
-  std::vector<DevBuf> bufs(12);
+  Workspace::Frame frame(c->ws);
+  std::vector<WsBuf> bufs(12);
   cudaError_t e;
-  auto al = [&](int k, size_t bytes) { return bufs[k].alloc(bytes); };
+  auto al = [&](int k, size_t bytes) { return bufs[k].alloc(c->ws, bytes); };
   if ((e = al(0, (size_t)cap * sizeof(float4))) != cudaSuccess) return e;            // photon positions (+ type)
   if ((e = al(1, (size_t)cap * kPmData * sizeof(float4))) != cudaSuccess) return e;  // photon rays, powers
   if ((e = al(2, (size_t)cap * sizeof(unsigned))) != cudaSuccess) return e;          // bucket keys

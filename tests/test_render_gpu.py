@@ -116,3 +116,53 @@ def test_baseline_roulette_mode_converges_to_the_same_image():
     seb = np.sqrt(np.maximum(sb - b * b, 0) / 4096)
     _, bad = compare(a, sea, b, seb)
     assert bad.mean() < 0.02
+
+
+def test_renders_share_the_workspace():
+    """Renders of different sizes and kinds in turn on one context, one of them from another
+    one's snapshot callback, each equal to the same render on a context of its own."""
+    sc = scenes.medium_scene(48, 40)
+    calls = [lambda c: c.render_pt(sc.camera, 3, max_depth=6, seed=3, want_sq=True)[:2],
+             lambda c: c.render_pt(scenes.cornell_camera(7, 5), 2, max_depth=4, seed=4, nee=True)[:1],
+             lambda c: c.render_bpt(sc.camera, 1, max_depth=6, seed=5)[:1],
+             lambda c: c.render_vcm(sc.camera, 2, 0.2, max_depth=6, seed=6)[:1],
+             lambda c: c.render_pm(sc.camera, 1, 0.2, max_depth=6, seed=7)[:1],
+             lambda c: [f for f in c.render_pt_batch([(c, scenes.cornell_camera(w, 9), dict(spp=2, seed=w)) for w in (3, 40)])[0]]]
+
+    def context():
+        c = rx.Context(0)
+        c.set_scene(sc)
+        c.build_accel()
+        return c
+
+    alone = []
+    for call in calls:
+        with context() as c:
+            alone.append(call(c))
+    got = []
+    with context() as c:
+        def check(k):
+            for a, b in zip(call_of(k), alone[k]):
+                # FP32 image atomics of the bidirectional estimators: their order alone
+                np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-6 * b.max())
+
+        def call_of(k):
+            return calls[k](c)
+
+        for k in (3, 0, 1, 2, 4, 5, 3, 1, 5, 0):
+            check(k)
+
+        busy = []
+
+        def nested(_t, _n, _film):  # the inner render's own snapshots come here too
+            if not busy:
+                busy.append(True)
+                got.append(calls[3](c)[0])
+
+        c.set_snapshots(1e-9, nested)
+        outer = c.render_pt(sc.camera, 4, max_depth=6, seed=8, paths_per_pass=1000)[0]
+        c.set_snapshots(0.0)
+        assert len(got) >= 1
+        np.testing.assert_allclose(got[0], alone[3][0], rtol=1e-5, atol=1e-6 * alone[3][0].max())
+        plain = c.render_pt(sc.camera, 4, max_depth=6, seed=8, paths_per_pass=1000)[0]
+        np.testing.assert_allclose(outer, plain, rtol=1e-9)
