@@ -138,6 +138,47 @@ __global__ void __launch_bounds__(128, 8) k_trace_persistent4(DevAccel A, const 
   walk_wide<4, kShort, 64>(A, A.bvh4, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, counters);
 }
 
+// A batch that the GPU holds at once: one launch, a ray per lane, the winner's visibility
+// check and (rarely) the re-walk by the lane that walked, after its warp's walks. The five
+// launches of a larger batch (two clears, walk, check, re-walk) cost a small one more than
+// its rays do: 1,000 rays 26.5 -> 10.3 us over 36 triangles and 58.6 -> 30.7 over 256 K,
+// 100,003 rays 68.9 -> 50.5 us over 25 K triangles.
+//  * Up to kOnceRays rays per SM, one resident lane each (eight blocks of 128). Beyond that
+//    the persistent walk's refills win on large scenes: 262,000 rays over 256 K triangles
+//    146.5 us against 150.2 (155,000: 112.3 against 96.3).
+//  * A warp takes 2^lanes_log2 rays, as few as keep kOnceWarps warps per SM busy, since the
+//    lanes of a warp wait for its longest walk: 3,000 rays over 256 K triangles 36.9 us
+//    against 49.1 in full warps. With 32 or 64 warps per SM before the warps fill, 30,000
+//    rays over 25 K triangles take 45.1 and 57.5 us against 41.0 with 16.
+constexpr uint32_t kOnceRays = 1024, kOnceWarps = 16;
+struct OnceLane : HitLane {
+  __device__ void end() {}
+};
+__global__ void __launch_bounds__(128, 8) k_trace_once(DevAccel A, const rx_ray* __restrict__ rays, uint32_t n,
+                                                       int lanes_log2, int32_t* __restrict__ out_tid,
+                                                       float* __restrict__ out_dist,
+                                                       unsigned long long* __restrict__ counters) {
+  const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t i = lane < (1u << lanes_log2) ? (warp << lanes_log2) + lane : kNoRay;
+  OnceLane L{{A, rays, n, nullptr, nullptr, nullptr, nullptr, nullptr, A.bvh4}};
+  walk_persistent<4, 16, 64, true>(L, nullptr, i);
+  if (i >= n) return;
+  HitResult h = L.best;
+  unsigned n_exact = 0;
+  if (h.hit) {
+    const float4* rp = reinterpret_cast<const float4*>(rays + i);
+    const F3 o = f3(__ldg(rp)), d = f3(__ldg(rp + 1));
+    const bool zd = (d.x == 0.0f) | (d.y == 0.0f) | (d.z == 0.0f);
+    if (!ref_visible(A, h.leaf, o, d, safe_inv(d), zd, &n_exact)) {
+      h = trace_ref_exact<true>(A, o, d, &n_exact);
+      atomicAdd(&counters[2], 1ull);
+    }
+  }
+  out_tid[i] = h.hit ? h.tid : -1;
+  out_dist[i] = h.hit ? h.t : -1.0f;
+  if (n_exact) atomicAdd(&counters[1], (unsigned long long)n_exact);
+}
+
 // 8-wide walk: 256-byte nodes; at most 7 stack entries per level of a tree shallower
 // than 12 levels.
 template <int kShort>
@@ -485,13 +526,25 @@ cudaError_t launch_trace_closest(const DevAccel& A, const rx_ray* rays, uint32_t
                                  uint32_t* queue, unsigned long long* counters, const TraceConfig& cfg,
                                  cudaStream_t s, const cudaEvent_t* ev, bool bin) {
   if (n == 0) return cudaSuccess;
+  const bool walk4 = A.bvh4 && 3 * A.bvh4_depth + 1 <= 64;  // the 4-wide walk's stack bound
+  const bool binned = bin && cfg.variant != 0 && cfg.bin_min && n >= cfg.bin_min;
+  if (cfg.variant == 4 && walk4 && cfg.check_thread && !binned && n <= (uint32_t)cfg.sms * kOnceRays) {
+    int lanes_log2 = 0;
+    while (lanes_log2 < 5 && ((uint64_t)cfg.sms * kOnceWarps << lanes_log2) < n) lanes_log2++;
+    if (ev) cudaEventRecord(ev[0], s);
+    const uint32_t warps = (n + (1u << lanes_log2) - 1) >> lanes_log2;
+    k_trace_once<<<(warps + 3) / 4, 128, 0, s>>>(A, rays, n, lanes_log2, tid, dist, counters);
+    if (ev)
+      for (int k = 1; k < 4; k++) cudaEventRecord(ev[k], s);
+    return cudaGetLastError();
+  }
   cudaMemsetAsync(counters, 0, sizeof(unsigned long long), s);  // eager queue length
   uint32_t* hit_leaf = queue;  // scratch: n entries of winners' reference leaves
   uint32_t* eager = queue + n;  // then up to n queued rays
   if (cfg.variant != 0) cudaMemsetAsync(counters + 4, 0, sizeof(unsigned long long), s);  // batch cursor
   const uint32_t* order = nullptr;
   int4* slot_rec = nullptr;
-  if (bin && cfg.variant != 0 && cfg.bin_min && n >= cfg.bin_min) {
+  if (binned) {
     uint32_t* keys = queue + 2 * (size_t)n;
     uint32_t* perm = queue + 3 * (size_t)n;
     uint32_t* hist = queue + 8 * (size_t)n;
@@ -514,7 +567,6 @@ cudaError_t launch_trace_closest(const DevAccel& A, const rx_ray* rays, uint32_t
     blocks = blocks < need ? blocks : need;
     // the walk's stack lives in local memory: the shallower one when the BVH allows
     const bool shallow = cfg.walk_stack != 64 && A.bvh_depth < 32;
-    const bool walk4 = A.bvh4 && 3 * A.bvh4_depth + 1 <= 64;  // the 4-wide walk's stack bound
     const bool walk8 = A.bvh8 && 7 * A.bvh8_depth + 1 <= 80;  // the 8-wide walk's
     if ((cfg.variant == 5 && walk8) || (cfg.variant == 4 && !walk4 && walk8))
       k_trace_persistent8<16><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);

@@ -39,8 +39,10 @@
 
 namespace rx {
 
-template <int W, int kShort, int kStack, class Lane>
-__device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cursor) {
+// kOnce: one ray per lane, `once` (kNoRay: none); no refills and no cursor.
+constexpr uint32_t kNoRay = 0xffffffffu;
+template <int W, int kShort, int kStack, bool kOnce = false, class Lane>
+__device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cursor, uint32_t once = kNoRay) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int DONE = INT_MIN;
   constexpr int kShortN = kShort > 0 ? kShort : 1;
@@ -69,10 +71,10 @@ __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cur
     if (want) {
       const int leader = __ffs(want) - 1;
       unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(cursor, (unsigned long long)__popc(want));
+      if (!kOnce && lane == leader) base = atomicAdd(cursor, (unsigned long long)__popc(want));
       base = __shfl_sync(FULL, base, leader);
       if (!active && !exhausted) {
-        const unsigned long long r = base + __popc(want & ((1u << lane) - 1));
+        const unsigned long long r = kOnce ? once : base + __popc(want & ((1u << lane) - 1));
         if (r < 0xffffffffull && L.begin((uint32_t)r, o, d)) {
           inv = safe_inv(d);
           ood = {o.x * inv.x, o.y * inv.y, o.z * inv.z};
@@ -179,6 +181,7 @@ __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cur
     if (active && cur == DONE) {
       L.end();
       active = false;
+      exhausted = kOnce;
     }
   }
 }
