@@ -800,7 +800,7 @@ struct Wave {
   const guide::RecSeg* segs;
   int steps;                // Adam steps per training pass (the most any network takes)
   uint32_t batch_max;
-  unsigned *ncount, *cursor;  // grouped inference sort (nnet > 1)
+  unsigned *ncount, *cursor;  // grouped inference sort (nr > 1)
   uint32_t* seg;
   int* rows;
 };
@@ -1004,7 +1004,7 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
     for (int k = 0; k < nj; k++) sc[k] = recs[k].S;
     if (!(W.scenes = static_cast<const DevScene*>(upload(sc.data(), sizeof(DevScene) * nj)))) return e;
     if (!(W.lobes = static_cast<float*>(alloc((size_t)slots * guide::kLobeStride * sizeof(float))))) return e;
-    if (nnet > 1) {
+    if (nj > 1) {  // grouped inference (enqueue_infer), with one network too
       if (!(W.ncount = static_cast<unsigned*>(alloc((size_t)nnet * 4)))) return e;
       if (!(W.cursor = static_cast<unsigned*>(alloc((size_t)nnet * 4)))) return e;
       if (!(W.seg = static_cast<uint32_t*>(alloc((size_t)(nnet + 1) * 4)))) return e;
