@@ -6,7 +6,7 @@
 // Stages per bounce, each a grid-stride kernel whose work count lives in device memory
 // (no host round trip inside a pass): extend (closest legal hit), shade (one scatter of
 // the reference's bounce loop through rx_material.cuh, emission, next-event estimation
-// with an inline shadow ray, Russian roulette) with queue compaction by warp ballot +
+// with its visibility rays queued, Russian roulette) with queue compaction by warp ballot +
 // one atomic per warp. Film accumulation is FP64.
 #include <algorithm>
 #include <chrono>
@@ -187,54 +187,140 @@ __global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, P
   }
 }
 
+// The next-event estimation's visibility rays of one bounce (PathTracerTest), queued by
+// k_shade and traced with the next extension rays: tracing them inline kept 9 of k_shade's
+// 32 lanes busy. A record holds the ray and the path's radiance with the light's
+// contribution (`lit`); a path that goes on already holds the radiance without it, one that
+// ended at the vertex has it in `dark` and reaches the film when the ray is traced.
+struct ShadowSoA {
+  float4* o;     // origin, w = length
+  float4* d;     // direction, w = contact object
+  float4* lit;   // radiance if nothing blocks the ray, w = inside object
+  float4* dark;  // ended paths: radiance if blocked; w = scene
+  int2* to;      // x: the path's slot in the next queue, -1: ended; y: pixel
+};
+
+__device__ __forceinline__ void film_add(double* sum, double* sq, size_t pixel, F3 L) {
+  // a sample that is not finite is dropped: it comes from a direction the 24-bit
+  // generator draws with probability density zero (a cosine lobe's pole at
+  // u = 0), where the reference's arithmetic divides by zero; one such sample
+  // would poison a pixel's FP64 sum at very high sample counts
+  if (!(isfinite(L.x) && isfinite(L.y) && isfinite(L.z)) || (L.x == 0.0f && L.y == 0.0f && L.z == 0.0f)) return;
+  double* s = sum + 3 * pixel;
+  atomicAdd(s, (double)L.x);
+  atomicAdd(s + 1, (double)L.y);
+  atomicAdd(s + 2, (double)L.z);
+  if (sq) {
+    double* q = sq + 3 * pixel;
+    atomicAdd(q, (double)L.x * L.x);
+    atomicAdd(q + 1, (double)L.y * L.y);
+    atomicAdd(q + 2, (double)L.z * L.z);
+  }
+}
+
+// A traced visibility ray's path: its radiance in the queue S, or in the film if it ended.
+__device__ __forceinline__ void shadow_done(const SceneRec* R, const PathSoA& S, const ShadowSoA& Q, uint32_t i,
+                                            bool blocked, double* film, double* sq) {
+  const int2 to = Q.to[i];
+  if (to.x >= 0) {
+    if (!blocked) S.L[to.x] = make_float4(Q.lit[i].x, Q.lit[i].y, Q.lit[i].z, 0.0f);
+  } else {
+    const float4 dark = Q.dark[i];
+    film_add(film, sq, (size_t)(R[__float_as_int(dark.w)].film_base + (uint32_t)to.y), blocked ? f3(dark) : f3(Q.lit[i]));
+  }
+}
+
 // The extension rays' lanes for walk_persistent (kWalk4P): path `order[r]` (binned
 // order) or r of the queue, its scene's 4-wide BVH, the closest legal hit
 // (NoSelfIntersectionCondition through leaf_test, as trace_cond4); the answer to hit[].
+// SHADOW: rays n .. n + m - 1 are the last bounce's visibility rays (any legal hit shorter
+// than the connection).
+template <bool SHADOW>
 struct ExtendLane {
   const SceneRec* R;
   PathSoA S;
-  uint32_t n;
+  uint32_t n, m;
   const uint32_t* __restrict__ order;
   int2* hit;
+  ShadowSoA Q;
+  double *film, *sq;
   const DevScene* sc = nullptr;
   uint32_t i = 0;
   int contact = kNone, inside = kNone;
-  bool cond = false;
+  bool cond = false, shadow = false;
   PHit best{-1, INFINITY};
 
   __device__ bool begin(uint32_t r, F3& o, F3& d) {
-    if (r >= n) return false;
-    i = order ? __ldg(&order[r]) : r;
-    const float4 o4 = S.o[i], d4 = S.d[i];
-    const int4 inf = S.info[i];
-    const bool camera = (inf.w & 255) == 0;  // the camera ray's first query has no condition
-    sc = &R[(uint32_t)inf.w >> 16].S;
-    contact = camera ? kNone : inf.y;
-    inside = camera ? kNone : inf.z;
-    cond = !(contact == kNone && inside == kNone);
+    if (r >= n + m) return false;
     best = PHit{-1, INFINITY};
-    o = f3(o4);
-    d = f3(d4);
+    shadow = SHADOW && r >= n;
+    if (SHADOW && shadow) {
+      i = r - n;
+      const float4 o4 = Q.o[i], d4 = Q.d[i];
+      sc = &R[__float_as_int(Q.dark[i].w)].S;
+      contact = __float_as_int(d4.w);
+      inside = __float_as_int(Q.lit[i].w);
+      best.t = o4.w;
+      o = f3(o4);
+      d = f3(d4);
+    } else {
+      i = order ? __ldg(&order[r]) : r;
+      const float4 o4 = S.o[i], d4 = S.d[i];
+      const int4 inf = S.info[i];
+      const bool camera = (inf.w & 255) == 0;  // the camera ray's first query has no condition
+      sc = &R[(uint32_t)inf.w >> 16].S;
+      contact = camera ? kNone : inf.y;
+      inside = camera ? kNone : inf.z;
+      o = f3(o4);
+      d = f3(d4);
+    }
+    cond = !(contact == kNone && inside == kNone);
     return true;
   }
   __device__ const float4* nodes() const { return sc->accel.bvh4; }
   __device__ float limit() const { return best.t; }
   __device__ void leaf(int first, int count, F3 o, F3 d) {
-    leaf_test<false>(*sc, first, count, o, d, cond, contact, inside, best);
+    if (SHADOW && shadow) {  // any hit: every remaining box is pruned
+      if (leaf_test<true, true>(*sc, first, count, o, d, cond, contact, inside, best)) best.t = -INFINITY;
+    } else {
+      leaf_test<false>(*sc, first, count, o, d, cond, contact, inside, best);
+    }
   }
-  __device__ void end() { hit[i] = make_int2(best.tid, __float_as_int(best.t)); }
+  __device__ void end() {
+    if (SHADOW && shadow) shadow_done(R, S, Q, i, best.tid >= 0, film, sq);
+    else hit[i] = make_int2(best.tid, __float_as_int(best.t));
+  }
 };
 
 // Closest legal hit of each live path's ray on persistent warps (kWalk4P): the same
 // answers as k_extend<kWalk4S>, with lanes refilled from `cursor` (zero at launch)
-// instead of each thread walking its share of the queue to the end.
+// instead of each thread walking its share of the queue to the end. SHADOW: and the
+// visibility rays of the bounce before. rays[0], rays[1] count both.
+template <bool SHADOW>
 __global__ void __launch_bounds__(128, 8) k_extend_p(const SceneRec* R, PathSoA S, const unsigned* count,
-                                                     const uint32_t* __restrict__ order, int2* hit,
+                                                     const uint32_t* __restrict__ order, int2* hit, ShadowSoA Q,
+                                                     const unsigned* scount, double* film, double* sq,
                                                      unsigned long long* rays, unsigned long long* cursor) {
-  const uint32_t n = *count;
-  ExtendLane L{R, S, n, order, hit};
+  const uint32_t n = *count, m = SHADOW ? *scount : 0u;
+  ExtendLane<SHADOW> L{R, S, n, m, order, hit, Q, film, sq};
   walk_persistent<4, kShortStack, 64>(L, cursor);
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(rays, (unsigned long long)n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    atomicAdd(rays, (unsigned long long)n);
+    if (SHADOW && m) atomicAdd(rays + 1, (unsigned long long)m);
+  }
+}
+// The visibility rays of a bounce one per thread (the other walk shapes).
+template <int STACK>
+__global__ void __launch_bounds__(128) k_shadow(const SceneRec* R, PathSoA S, ShadowSoA Q, const unsigned* scount,
+                                                double* film, double* sq, unsigned long long* rays) {
+  const uint32_t m = *scount;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+    const float4 o = Q.o[i], d = Q.d[i];
+    const PHit h = trace_walk<true, STACK, true>(R[__float_as_int(Q.dark[i].w)].S, f3(o), f3(d), o.w, __float_as_int(d.w),
+                                           __float_as_int(Q.lit[i].w));
+    shadow_done(R, S, Q, i, h.tid >= 0, film, sq);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && m) atomicAdd(rays + 1, (unsigned long long)m);
 }
 // Bin keys of the live paths' next rays (counting sort input; rx_bin.cuh).
 __global__ void k_path_keys(const SceneRec* R, PathSoA S, const unsigned* count, uint32_t* keys, uint32_t* hist) {
@@ -267,25 +353,14 @@ __global__ void __launch_bounds__(128) k_extend(const SceneRec* R, PathSoA S, co
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(rays, (unsigned long long)n);
 }
 
-__device__ __forceinline__ void film_add(double* sum, double* sq, int pixel, F3 L) {
-  double* s = sum + 3 * (size_t)pixel;
-  atomicAdd(s, (double)L.x);
-  atomicAdd(s + 1, (double)L.y);
-  atomicAdd(s + 2, (double)L.z);
-  if (sq) {
-    double* q = sq + 3 * (size_t)pixel;
-    atomicAdd(q, (double)L.x * L.x);
-    atomicAdd(q + 1, (double)L.y * L.y);
-    atomicAdd(q + 2, (double)L.z * L.z);
-  }
-}
-
 // PathTracerTest::colorByConnectingLights (src/PathTracerTest.cpp:88-136) at vertex `v`
 // (the ray leaving it), reached by `in`: a light point by area, two-sided emission,
-// balance-heuristic weight against the BSDF's sampling pdf.
-template <int STACK>
-__device__ F3 connect_light(const DevScene& SC, const CamDev& cam, const PV& in, const PV& v, Rng& rng,
-                            unsigned& shadows) {
+// balance-heuristic weight against the BSDF's sampling pdf. Returns the contribution when
+// nothing lies between (testVisibility, still to be traced: direction `dir` and distance
+// `len` from v); no ray is asked for (false) where it is zero.
+__device__ __forceinline__ bool connect_light(const DevScene& SC, const CamDev& cam, const PV& in, const PV& v, Rng& rng,
+                                              F3& add, F3& dir, float& len) {
+  add = F3{0, 0, 0};
   float ru = rng.next() * SC.light_area;
   int lo = 0, hi = (int)SC.num_lights - 1;
   while (lo < hi) {
@@ -305,20 +380,20 @@ __device__ F3 connect_light(const DevScene& SC, const CamDev& cam, const PV& in,
   PV out = v;
   out.d = -ld;
   F3 f = bsdf_of(SC, cam, in, out);
-  if (lum(f) < 1e-7f) return {0, 0, 0};
+  if (lum(f) < 1e-7f) return false;
   F3 nl = world_normal(lg, SC.objects[lg.obj].has_normals, xl);
   float cos_l = fminf(fabsf(dot(nl, ld)), 1.0f);
-  if (cos_l < 1e-6f) return {0, 0, 0};
+  if (cos_l < 1e-6f) return false;
   float cos_s = 1.0f;
   if (v.contact != kNone) cos_s = fminf(fabsf(dot(contact_normal(SC, cam, v), out.d)), 1.0f);
   float bpdf = dir_pdf(SC, cam, in, out, false);
-  shadows++;
-  PHit sh = trace_walk<true, STACK>(SC, v.o, out.d, dist - 1e-5f, v.contact, v.inside);  // testVisibility
-  if (sh.tid >= 0) return {0, 0, 0};
   float pdfa = 1.0f / SC.light_area;
   float pdfw = pdfa * dist * dist / cos_l;
   float mis = pdfw / (pdfw + bpdf);
-  return f3v(SC.objects[lg.obj].color) * f * (cos_l * cos_s / (pdfa * dist * dist) * mis);
+  add = f3v(SC.objects[lg.obj].color) * f * (cos_l * cos_s / (pdfa * dist * dist) * mis);
+  dir = out.d;
+  len = dist - 1e-5f;
+  return true;
 }
 
 // Guided sampling state of a wavefront (all null / zero when guiding is off). A scene's
@@ -405,16 +480,16 @@ static __device__ PV scatter_guided(const DevScene& S, const PV& in, Hit3 h, boo
   return o;
 }
 
-// One bounce of MCRenderer::samplePathIter plus the estimator's bookkeeping.
-template <int STACK>
+// One bounce of MCRenderer::samplePathIter plus the estimator's bookkeeping. NEE: some scene
+// is a PathTracerTest (its visibility rays go to Q); GUIDE: some scene has a network.
+template <bool NEE, bool GUIDE>
 __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassState* ps, PathSoA S,
                                                const unsigned* count, const int2* hit, PathSoA N, unsigned* next_count,
-                                               double* film_sum, double* film_sq, unsigned long long* shadow_rays,
+                                               double* film_sum, double* film_sq, ShadowSoA Q, unsigned* scount,
                                                GuideIO G) {
   uint32_t n = *count;
   uint32_t stride = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
-  unsigned shadows = 0;
   // every lane of a warp walks the same number of iterations (ballots need all 32)
   uint32_t nwarp_iter = (n + stride - 1) / stride;
   for (uint32_t it = 0; it < nwarp_iter; it++) {
@@ -428,6 +503,10 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
     bool rec = false;  // a guided vertex whose path continues: a training record
     uint32_t sc = 0;
     uint32_t local = 0;  // the path's slot in the pass's generation order
+    bool pend = false;   // a visibility ray decides between the radiances `lit` and L
+    F3 lit{}, sdir{};
+    float slen = 0.0f;
+    uint32_t next_slot = 0xffffffffu;
     if (i < n) {
       float4 o4 = S.o[i], d4 = S.d[i], T4 = S.T[i], L4 = S.L[i];
       inf = S.info[i];
@@ -448,7 +527,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
       cur.flags = (depth == 0 || !last_spec) ? kDirRandom : 0u;  // the camera ray is RANDOM
       int2 h = hit[i];
       Rng rng(P.seed, pid & kPidMask, 16u + 32u * (uint32_t)depth);
-      const int net = G.nets ? R[sc].net : -1;
+      const int net = GUIDE ? R[sc].net : -1;
       const bool training = net >= 0 && G.recs && ps->pass < G.nets[net].train;
       bool done = true;
       if (h.x >= 0) {  // a ray that hits nothing ends the path (samplePathIter's termRay)
@@ -466,7 +545,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
         float dist = length(nx.o - cur.o);
         bool killed = length(nx.d) < 0.5f;
         bool capped = !killed && depth + 1 > (int)P.max_depth;
-        if (!P.nee) {
+        if (!NEE || !P.nee) {
           // PathTracer.cpp:48-60: colour/directionProb/originProb of every ray, cosine
           // and transmittance of every ray but the last
           T = T * decay_of(SC, cur.inside, dist);
@@ -492,7 +571,12 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
           }
           L = L + T * f3v(SC.objects[nx.contact].color) * mis;
         } else if (!capped) {
-          if ((nx.flags & kDirRandom) && SC.num_lights > 0) L = L + T * connect_light<STACK>(SC, P.cam, cur, nx, rng, shadows);
+          if ((nx.flags & kDirRandom) && SC.num_lights > 0) {
+            F3 add;
+            pend = connect_light(SC, P.cam, cur, nx, rng, add, sdir, slen);
+            lit = L + T * add;
+            L = L + T * F3{0, 0, 0};
+          }
           if (!killed) {
             T = T * (nx.c * (cos_term(SC, P.cam, nx) / nx.dprob));
             T = T * decay_of(SC, cur.inside, fmaxf(dist, 1e-5f));
@@ -501,13 +585,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
         }
       }
       if (done) {
-        // a sample that is not finite is dropped: it comes from a direction the 24-bit
-        // generator draws with probability density zero (a cosine lobe's pole at
-        // u = 0), where the reference's arithmetic divides by zero; one such sample
-        // would poison a pixel's FP64 sum at very high sample counts
-        const bool finite = isfinite(L.x) && isfinite(L.y) && isfinite(L.z);
-        if (finite && (L.x != 0.0f || L.y != 0.0f || L.z != 0.0f))
-          film_add(film_sum, film_sq, (int)(R[sc].film_base + (uint32_t)inf.x), L);
+        if (!pend) film_add(film_sum, film_sq, (size_t)(R[sc].film_base + (uint32_t)inf.x), L);
         if (training && G.lpath) G.lpath[local] = make_float4(L.x, L.y, L.z, 0.0f);
       } else {
         cont = true;
@@ -541,6 +619,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
       base = __shfl_sync(0xffffffffu, base, leader);
       if (cont) {
         uint32_t j = base + __popc(m & ((1u << lane) - 1));
+        next_slot = j;
         N.o[j] = make_float4(nx.o.x, nx.o.y, nx.o.z, nx.dprob);
         N.d[j] = make_float4(nx.d.x, nx.d.y, nx.d.z, 0.0f);
         N.T[j] = make_float4(T.x, T.y, T.z, 0.0f);
@@ -550,17 +629,33 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
         N.id[j] = pid;
       }
     }
+    if constexpr (NEE) {
+      const unsigned sm = __ballot_sync(0xffffffffu, pend);
+      if (sm) {
+        unsigned base = 0;
+        const int leader = __ffs(sm) - 1;
+        if (lane == leader) base = atomicAdd(scount, (unsigned)__popc(sm));
+        base = __shfl_sync(0xffffffffu, base, leader);
+        if (pend) {
+          const uint32_t j = base + __popc(sm & ((1u << lane) - 1));
+          Q.o[j] = make_float4(nx.o.x, nx.o.y, nx.o.z, slen);
+          Q.d[j] = make_float4(sdir.x, sdir.y, sdir.z, __int_as_float(nx.contact));
+          Q.lit[j] = make_float4(lit.x, lit.y, lit.z, __int_as_float(nx.inside));
+          Q.dark[j] = make_float4(L.x, L.y, L.z, __int_as_float((int)sc));
+          Q.to[j] = make_int2((int)next_slot, inf.x);
+        }
+      }
+    }
   }
-  for (int s2 = 16; s2 > 0; s2 >>= 1) shadows += __shfl_xor_sync(0xffffffffu, shadows, s2);
-  if (lane == 0 && shadows) atomicAdd(shadow_rays, (unsigned long long)shadows);
 }
 
-// The next queue's length, and the extension walk's refill cursor for the next bounce
+// The next queue's length, the extension walk's refill cursor for the next bounce
 // (kWalk4P: every k_extend_p launch of a pass is followed by this one, so the cursor is
-// zero when the next starts).
-__global__ void k_zero(unsigned* p, unsigned long long* cursor) {
+// zero when the next starts) and the number of visibility rays.
+__global__ void k_zero(unsigned* p, unsigned long long* cursor, unsigned* scount) {
   *p = 0;
   *cursor = 0ull;
+  *scount = 0;
 }
 __global__ void k_advance(PassState* ps) {
   ps->base += ps->per_pass;
@@ -779,8 +874,9 @@ struct Wave {
   PassState* ps;
   PathSoA A, B;
   int2* hit;
+  ShadowSoA Q;              // visibility rays of a bounce (null without next-event estimation)
   unsigned long long* ctr;  // [0] extension rays, [1] shadow rays
-  unsigned* cnt;            // [0], [1] queue lengths, [2] raw training records
+  unsigned* cnt;            // [0], [1] queue lengths, [2] raw training records, [3] visibility rays
   double *film, *sq;
   uint32_t loops;           // bounce stages per pass (max depth cap + 1)
   uint32_t *keys, *order, *hist;  // ray binning of bounce rays (null: off)
@@ -839,19 +935,34 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   if (W.recs) k_records_begin<<<1, 256, 0, s>>>(W.nets, W.nnet, W.ps, W.cnt + 2, W.net_count);
   k_generate<<<grid, 256, 0, s>>>(W.R, W.nr, W.ps, W.L, W.A, W.cnt);
   const GuideIO G{W.nets, W.lobes, W.recs, W.cnt + 2, W.rec_cap, W.lpath};
+  const bool nee = W.Q.o != nullptr;
+  unsigned* scnt = W.cnt + 3;
   PathSoA cur = W.A, nxt = W.B;
   unsigned *cc = W.cnt, *cn = W.cnt + 1;
+  // the extension rays of a queue, and the visibility rays of the bounce before
+  auto extend = [&](const PathSoA& q, const unsigned* count, const uint32_t* order) {
+    if constexpr (STACK == kWalk4P) {  // persistent: the blocks that stay resident (8 per SM)
+      auto k = nee ? k_extend_p<true> : k_extend_p<false>;
+      k<<<W.sms * 8, 128, 0, s>>>(W.R, q, count, order, W.hit, W.Q, scnt, W.film, W.sq, W.ctr, W.ctr + kExtendCursor);
+    } else {
+      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, count, order, W.hit, W.ctr);
+      if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, scnt, W.film, W.sq, W.ctr);
+    }
+  };
   for (uint32_t d = 0; d < W.loops; d++) {
     const uint32_t* order = d > 0 ? enqueue_binning(W, cur, cc, grid, s) : nullptr;
-    if constexpr (STACK == kWalk4P)  // persistent: the blocks that stay resident (8 per SM)
-      k_extend_p<<<W.sms * 8, 128, 0, s>>>(W.R, cur, cc, order, W.hit, W.ctr, W.ctr + kExtendCursor);
-    else
-      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, cur, cc, order, W.hit, W.ctr);
+    extend(cur, cc, order);
     if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, cc, grid, s);
-    k_zero<<<1, 1, 0, s>>>(cn, W.ctr + kExtendCursor);
-    k_shade<STACK><<<grid, 128, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.ctr + 1, G);
+    k_zero<<<1, 1, 0, s>>>(cn, W.ctr + kExtendCursor, scnt);
+    auto shade = nee ? (W.nets ? k_shade<true, true> : k_shade<true, false>)
+                     : (W.nets ? k_shade<false, true> : k_shade<false, false>);
+    shade<<<grid, 128, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.Q, scnt, G);
     std::swap(cur, nxt);
     std::swap(cc, cn);
+  }
+  if (nee) {  // no path goes on; the last vertices' visibility rays
+    extend(cur, cc, nullptr);
+    k_zero<<<1, 1, 0, s>>>(cc, W.ctr + kExtendCursor, scnt);
   }
   if (W.recs) {
     k_record_weights<<<grid, 128, 0, s>>>(W.R, W.nr, W.L.off, W.ps, W.nets, W.nnet, W.recs, W.cnt + 2, W.rec_cap,
@@ -978,6 +1089,13 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
   if ((e = alloc_soa(W.A, c->ws, slots)) != cudaSuccess) return e;
   if ((e = alloc_soa(W.B, c->ws, slots)) != cudaSuccess) return e;
   if (!(W.hit = static_cast<int2*>(alloc(slots * sizeof(int2))))) return e;
+  bool any_nee = false;
+  for (int k = 0; k < nj; k++) any_nee = any_nee || recs[k].P.nee;
+  if (any_nee) {  // at most one visibility ray per live path
+    for (float4** q : {&W.Q.o, &W.Q.d, &W.Q.lit, &W.Q.dark})
+      if (!(*q = static_cast<float4*>(alloc((size_t)slots * sizeof(float4))))) return e;
+    if (!(W.Q.to = static_cast<int2*>(alloc((size_t)slots * sizeof(int2))))) return e;
+  }
   if (!(W.ctr = static_cast<unsigned long long*>(alloc(64 * sizeof(unsigned long long))))) return e;
   W.cnt = reinterpret_cast<unsigned*>(W.ctr + 8);
   cudaMemsetAsync(W.ctr, 0, 64 * sizeof(unsigned long long), s);

@@ -138,10 +138,26 @@ struct PHit {
   float t;
 };
 
+// d x e and d . q of the triangle tests. NEG: d is the negative of the direction that a
+// connection was built with (light to surface); the products are then rounded as the
+// compiler rounds them when it sees that negation (the other product of each pair is the
+// one rounded alone), so a visibility ray at the rim of a triangle gets the answer it gets
+// where the connection is traced in the kernel that builds it.
+template <bool NEG>
+__device__ __forceinline__ F3 ray_cross(F3 d, F3 e) {
+  if constexpr (!NEG) return cross(d, e);
+  return {fmaf(-d.z, e.y, __fmul_rn(d.y, e.z)), fmaf(-d.x, e.z, __fmul_rn(d.z, e.x)), fmaf(-d.y, e.x, __fmul_rn(d.x, e.y))};
+}
+template <bool NEG>
+__device__ __forceinline__ float ray_dot(F3 d, F3 q) {
+  if constexpr (!NEG) return dot(d, q);
+  return fmaf(d.z, q.z, fmaf(d.y, q.y, __fmul_rn(d.x, q.x)));
+}
+
 // Closest legal hit with t < tmax (ANY: stop at the first legal one). contact, inside:
 // object ids, -1 for none (-1/-1: no condition, as the camera ray's first query),
 // -2 for the camera as contact object.
-template <bool ANY, int STACK = kStackDepth>
+template <bool ANY, int STACK = kStackDepth, bool NEG = false>
 __device__ __forceinline__ PHit trace_cond(const DevScene& S, F3 o, F3 d, float tmax, int contact, int inside) {
   const DevAccel& A = S.accel;
   F3 inv = {fabsf(d.x) > 1e-30f ? 1.0f / d.x : copysignf(1e30f, d.x),
@@ -190,7 +206,7 @@ __device__ __forceinline__ PHit trace_cond(const DevScene& S, F3 o, F3 d, float 
         const float4* tp = A.tris + 3 * (size_t)(first + k);
         float4 w0 = __ldg(tp), w1 = __ldg(tp + 1), w2 = __ldg(tp + 2);
         F3 v0 = f3(w0), e1 = f3(w1) - v0, e2 = f3(w2) - v0;
-        F3 pv = cross(d, e2);
+        F3 pv = ray_cross<NEG>(d, e2);
         float det = dot(e1, pv);
         if (fabsf(det) < 1e-30f) continue;
         float idet = 1.0f / det;
@@ -198,7 +214,7 @@ __device__ __forceinline__ PHit trace_cond(const DevScene& S, F3 o, F3 d, float 
         float u = dot(sv, pv) * idet;
         if (u < -1e-7f || u > 1.0000001f) continue;
         F3 qv = cross(sv, e1);
-        float v = dot(d, qv) * idet;
+        float v = ray_dot<NEG>(d, qv) * idet;
         if (v < -1e-7f || u + v > 1.0000001f) continue;
         float t = dot(e2, qv) * idet;
         if (!(t >= 0.0f) || !(t < best.t)) continue;
@@ -207,7 +223,7 @@ __device__ __forceinline__ PHit trace_cond(const DevScene& S, F3 o, F3 d, float 
           float4 q0 = __ldg(nn), q1 = __ldg(nn + 1), q2 = __ldg(nn + 2);
           int obj = __float_as_int(q0.w);
           F3 n = normalize(f3(q0) * (1.0f - u - v) + f3(q1) * u + f3(q2) * v);
-          if (!legal_hit(contact, inside, obj, dot(d, n))) continue;
+          if (!legal_hit(contact, inside, obj, ray_dot<NEG>(d, n))) continue;
         }
         best = {__float_as_int(w0.w), t};
         if (ANY) return best;
@@ -237,7 +253,7 @@ constexpr int kShortStack = 16;
 // The cnt triangles of the 4-wide tree's leaf at slot `first` (Moller-Trumbore, the
 // NoSelfIntersectionCondition when cond): lowers best to the nearest legal hit; with ANY,
 // returns true at the first one.
-template <bool ANY>
+template <bool ANY, bool NEG = false>
 __device__ __forceinline__ bool leaf_test(const DevScene& S, int first, int cnt, F3 o, F3 d, bool cond, int contact,
                                           int inside, PHit& best) {
   const DevAccel& A = S.accel;
@@ -245,7 +261,7 @@ __device__ __forceinline__ bool leaf_test(const DevScene& S, int first, int cnt,
     const float4* tp = A.tris + 3 * (size_t)(first + k);
     float4 w0 = __ldg(tp), w1 = __ldg(tp + 1), w2 = __ldg(tp + 2);
     F3 v0 = f3(w0), e1 = f3(w1) - v0, e2 = f3(w2) - v0;
-    F3 pv = cross(d, e2);
+    F3 pv = ray_cross<NEG>(d, e2);
     float det = dot(e1, pv);
     if (fabsf(det) < 1e-30f) continue;
     float idet = 1.0f / det;
@@ -253,7 +269,7 @@ __device__ __forceinline__ bool leaf_test(const DevScene& S, int first, int cnt,
     float u = dot(sv, pv) * idet;
     if (u < -1e-7f || u > 1.0000001f) continue;
     F3 qv = cross(sv, e1);
-    float v = dot(d, qv) * idet;
+    float v = ray_dot<NEG>(d, qv) * idet;
     if (v < -1e-7f || u + v > 1.0000001f) continue;
     float t = dot(e2, qv) * idet;
     if (!(t >= 0.0f) || !(t < best.t)) continue;
@@ -262,7 +278,7 @@ __device__ __forceinline__ bool leaf_test(const DevScene& S, int first, int cnt,
       float4 q0 = __ldg(nn), q1 = __ldg(nn + 1), q2 = __ldg(nn + 2);
       int obj = __float_as_int(q0.w);
       F3 n = normalize(f3(q0) * (1.0f - u - v) + f3(q1) * u + f3(q2) * v);
-      if (!legal_hit(contact, inside, obj, dot(d, n))) continue;
+      if (!legal_hit(contact, inside, obj, ray_dot<NEG>(d, n))) continue;
     }
     best = {__float_as_int(w0.w), t};
     if (ANY) return true;
@@ -273,7 +289,7 @@ __device__ __forceinline__ bool leaf_test(const DevScene& S, int first, int cnt,
 // SH > 0: the first SH stack entries of each thread sit in shared memory, one column
 // per thread (callers are kernels of at most kShortCols threads per block).
 constexpr int kShortCols = 128;
-template <bool ANY, int SH = 0>
+template <bool ANY, int SH = 0, bool NEG = false>
 __device__ __forceinline__ PHit trace_cond4(const DevScene& S, F3 o, F3 d, float tmax, int contact, int inside) {
   const DevAccel& A = S.accel;
   constexpr int kSHN = SH > 0 ? SH : 1;
@@ -348,7 +364,7 @@ __device__ __forceinline__ PHit trace_cond4(const DevScene& S, F3 o, F3 d, float
         cur = r[0];
         continue;
       }
-    } else if (leaf_test<ANY>(S, leaf_first(cur), leaf_count(cur), o, d, cond, contact, inside, best)) {
+    } else if (leaf_test<ANY, NEG>(S, leaf_first(cur), leaf_count(cur), o, d, cond, contact, inside, best)) {
       return best;
     }
     bool found = false;
@@ -369,12 +385,12 @@ __device__ __forceinline__ PHit trace_cond4(const DevScene& S, F3 o, F3 d, float
 // Closest / any legal hit with the walk WALK selects: kWalk4 = the 4-wide BVH, kWalk4S =
 // the same with its first kShortStack stack entries in shared memory, else the binary
 // BVH with a stack of WALK entries.
-template <bool ANY, int WALK>
+template <bool ANY, int WALK, bool NEG = false>
 __device__ __forceinline__ PHit trace_walk(const DevScene& S, F3 o, F3 d, float tmax, int contact, int inside) {
-  if constexpr (WALK == kWalk4) return trace_cond4<ANY, 0>(S, o, d, tmax, contact, inside);
+  if constexpr (WALK == kWalk4) return trace_cond4<ANY, 0, NEG>(S, o, d, tmax, contact, inside);
   else if constexpr (WALK == kWalk4S || WALK == kWalk4P)
-    return trace_cond4<ANY, kShortStack>(S, o, d, tmax, contact, inside);
-  else return trace_cond<ANY, WALK>(S, o, d, tmax, contact, inside);
+    return trace_cond4<ANY, kShortStack, NEG>(S, o, d, tmax, contact, inside);
+  else return trace_cond<ANY, WALK, NEG>(S, o, d, tmax, contact, inside);
 }
 
 }  // namespace rx
