@@ -208,8 +208,11 @@ static __device__ __forceinline__ bool leaves_object(const float4* __restrict__ 
 // as long as the object list: 60 us of k_shade per bounce in a scene of 207 objects, however
 // few its paths; a 1024^2 x 16 frame of that scene 67.8 -> 57.4 ms). A point outside a medium's padded bounds is not inside it: a line meets a
 // box on one side of such a point only, so one of the two rays cannot hit. The walk ends
-// where the ray leaves the bounds.
+// where the ray leaves the bounds. MEDIA false: the scene is known to have no medium (here
+// and in the scattering functions: code and registers less).
+template <bool MEDIA = true>
 __device__ __forceinline__ int find_inside(const DevScene& S, F3 o, F3 d, int exclude) {
+  if constexpr (!MEDIA) return kNone;
   for (uint32_t m = 0; m < S.num_media; m++) {
     const float4 lo = __ldg(&S.media[2 * m]), hi = __ldg(&S.media[2 * m + 1]);
     const int i = __float_as_int(lo.w);
@@ -340,6 +343,7 @@ __device__ __forceinline__ float fresnel_er(float cur_n, float next_n, float ct,
   return (a * a + b * b) * 0.5f;
 }
 
+template <bool MEDIA = true>
 static __device__ PV scatter_material(const DevScene& S, const CamDev& cam, int obj, const PV& in, Hit3 h,
                                bool fix_is_light, bool russian, Rng& rng);
 
@@ -491,6 +495,7 @@ static __device__ PV scatter_vpm(const DevScene& S, const CamDev& cam, int self,
 // SceneObject::scatter with the object's material(s): Diffuse, Glossy, Phong (one lobe
 // picked uniformly, SceneObject.cpp:373-380), Refractive / Reflective, Emissive. A
 // medium object is not handled here (scatter_vpm).
+template <bool MEDIA>
 static __device__ PV scatter_material(const DevScene& S, const CamDev& cam, int obj, const PV& in, Hit3 h,
                                bool fix_is_light, bool russian, Rng& rng) {
   const DevObject& ob = S.objects[obj];
@@ -600,7 +605,7 @@ static __device__ PV scatter_material(const DevScene& S, const CamDev& cam, int 
   }
   float cd = fminf(fmaxf(dot(in.d, n), -1.0f), 1.0f);
   float theta = acosf(cd);
-  int outside = in.inside == obj ? find_inside(S, x, in.d, obj) : obj;
+  int outside = in.inside == obj ? find_inside<MEDIA>(S, x, in.d, obj) : obj;
   float cur_n = refr_coeff(S, in.inside), next_n = refr_coeff(S, outside);
   o.dprob = 1.0f;
   float sin_phi = cur_n / next_n * sinf(theta);
@@ -636,14 +641,15 @@ static __device__ PV scatter_material(const DevScene& S, const CamDev& cam, int 
 // The object's scatter: a medium's (SceneVPMObject::scatter); a dielectric the ray is
 // inside that hits another object hands the ray to that object
 // (RefractiveMaterial.cpp:183-187); else the object's material.
+template <bool MEDIA = true>
 static __device__ PV scatter_object(const DevScene& S, const CamDev& cam, int obj, const PV& in, Hit3 h, bool fix_is_light,
                              bool russian, Rng& rng) {
   const DevObject& ob = S.objects[obj];
-  if (ob.material == kVPM) return scatter_vpm(S, cam, obj, in, h, fix_is_light, russian, rng);
+  if (MEDIA && ob.material == kVPM) return scatter_vpm(S, cam, obj, in, h, fix_is_light, russian, rng);
   if (ob.material == kRefractive && h.obj != obj && in.inside == obj && h.obj >= 0 &&
       S.objects[h.obj].material != kVPM)
-    return scatter_material(S, cam, h.obj, in, h, fix_is_light, russian, rng);
-  return scatter_material(S, cam, obj, in, h, fix_is_light, russian, rng);
+    return scatter_material<MEDIA>(S, cam, h.obj, in, h, fix_is_light, russian, rng);
+  return scatter_material<MEDIA>(S, cam, obj, in, h, fix_is_light, russian, rng);
 }
 
 // One scatter of MCRenderer::samplePathIter (src/MCRenderer.cpp:169-217): the inside
@@ -661,10 +667,11 @@ __device__ __forceinline__ void leak_kill(const DevScene& S, const CamDev& cam, 
   }
 }
 
+template <bool MEDIA = true>
 static __device__ PV scatter_step(const DevScene& S, const CamDev& cam, const PV& in, Hit3 h, bool fix_is_light, bool russian,
                            Rng& rng) {
   int obj = in.inside != kNone ? in.inside : h.obj;
-  PV o = scatter_object(S, cam, obj, in, h, fix_is_light, russian, rng);
+  PV o = scatter_object<MEDIA>(S, cam, obj, in, h, fix_is_light, russian, rng);
   leak_kill(S, cam, in, o);
   return o;
 }

@@ -480,13 +480,62 @@ static __device__ PV scatter_guided(const DevScene& S, const PV& in, Hit3 h, boo
   return o;
 }
 
+// Which of the block's paths (index within the block) this thread shades: the block's paths
+// by the kind of scatter (diffuse; glossy and Phong; dielectric, mirror and anything inside
+// an object; emitters and misses), so that a warp runs one or two kinds instead of all.
+template <int kWarps>
+__device__ __forceinline__ uint32_t block_by_material(const SceneRec* R, const PathSoA& S, const int2* hit, uint32_t i,
+                                                      uint32_t n, uint32_t (&count)[kWarps][4],
+                                                      unsigned short (&perm)[32 * kWarps]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int key = 3;
+  if (i < n) {
+    const int tid = hit[i].x;
+    const int4 inf = S.info[i];
+    if (tid >= 0) {
+      const DevScene& SC = R[(uint32_t)inf.w >> 16].S;
+      const uint32_t m = SC.objects[__ldg(&SC.tri_obj[tid])].material;
+      key = inf.z >= 0 ? 2 : m == kDiffuse ? 0 : m == kGlossy || m == kPhong ? 1 : m == kEmissive ? 3 : 2;
+    }
+  }
+  uint32_t rank = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const unsigned b = __ballot_sync(0xffffffffu, key == k);
+    if (key == k) rank = __popc(b & ((1u << lane) - 1));
+    if (lane == k) count[warp][k] = __popc(b);
+  }
+  __syncthreads();
+  for (int k = 0; k < 4; k++)
+    for (int w = 0; w < kWarps; w++)
+      if (k < key || (k == key && w < warp)) rank += count[w][k];
+  perm[rank] = (unsigned short)threadIdx.x;
+  __syncthreads();
+  return perm[threadIdx.x];
+}
+
 // One bounce of MCRenderer::samplePathIter plus the estimator's bookkeeping. NEE: some scene
-// is a PathTracerTest (its visibility rays go to Q); GUIDE: some scene has a network.
-template <bool NEE, bool GUIDE>
-__global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassState* ps, PathSoA S,
+// is a PathTracerTest (its visibility rays go to Q); GUIDE: some scene has a network; MEDIA:
+// some scene has a medium.
+//
+// Bound by latency and instruction fetch, not by the 176 bytes a path moves (1 M paths over
+// the Cornell box: 77 us for 27 us of traffic): 64 registers and 1,024 resident threads per
+// SM, though the variants with media spill, beat 80 to 128 registers (1024^2 x 16 spp over
+// 1 M triangles 47.6 ms against 50.5-50.8, the Cornell frame 0.85 against 0.91). The paths of
+// a block are shaded by material: 12 of 32 lanes were busy in pixel order (47.6 against 48.5
+// ms; 16 scenes in one batch 5.55 against 6.65 ms). Blocks of 512 where media make the
+// branches longest (that batch 5.55 ms against 5.96 with 256 threads and 6.54 with 128),
+// else 256 (the Cornell frame 0.85 against 0.86 ms).
+template <bool MEDIA>
+constexpr int kShadeThreads = MEDIA ? 512 : 256;
+template <bool NEE, bool GUIDE, bool MEDIA>
+__global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MEDIA>) k_shade(const SceneRec* R, const PassState* ps, PathSoA S,
                                                const unsigned* count, const int2* hit, PathSoA N, unsigned* next_count,
                                                double* film_sum, double* film_sq, ShadowSoA Q, unsigned* scount,
-                                               GuideIO G) {
+                                               GuideIO G, bool sort) {
+  constexpr int kWarps = kShadeThreads<MEDIA> / 32;
+  __shared__ uint32_t s_count[kWarps][4];
+  __shared__ unsigned short s_perm[32 * kWarps];
   uint32_t n = *count;
   uint32_t stride = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
@@ -494,6 +543,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
   uint32_t nwarp_iter = (n + stride - 1) / stride;
   for (uint32_t it = 0; it < nwarp_iter; it++) {
     uint32_t i = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
+    if (sort) i += block_by_material(R, S, hit, i, n, s_count, s_perm) - threadIdx.x;
     bool cont = false;
     PV nx;
     F3 T{}, L{}, Tb{};
@@ -540,7 +590,7 @@ __global__ void __launch_bounds__(128) k_shade(const SceneRec* R, const PassStat
                               G.nets[net].frac);
           leak_kill(SC, P.cam, cur, nx);
         } else {
-          nx = scatter_step(SC, P.cam, cur, hh, false, russian, rng);
+          nx = scatter_step<MEDIA>(SC, P.cam, cur, hh, false, russian, rng);
         }
         float dist = length(nx.o - cur.o);
         bool killed = length(nx.d) < 0.5f;
@@ -882,6 +932,8 @@ struct Wave {
   uint32_t *keys, *order, *hist;  // ray binning of bounce rays (null: off)
   Layout L;                 // interleaved passes (L.off null: concatenated)
   int sms;
+  bool media;               // some scene has a medium
+  bool sort;                // shade each block's paths by material
   // guiding (nets null: off)
   const guide::NetDev* nets;
   int nnet;
@@ -924,6 +976,13 @@ cudaError_t enqueue_infer(const Wave& W, const PathSoA& cur, const unsigned* cc,
   return guide_infer_wave(W.nets, W.nnet, W.scenes, cur, cc, W.hit, W.lobes, W.rows, W.seg, pass, W.sms, s);
 }
 
+// The shading kernel for what the scenes hold (guided renders: the variant with media).
+auto shade_kernel(bool nee, bool guide, bool media) {
+  if (guide) return nee ? k_shade<true, true, true> : k_shade<false, true, true>;
+  if (media) return nee ? k_shade<true, false, true> : k_shade<false, false, true>;
+  return nee ? k_shade<true, false, false> : k_shade<false, false, false>;
+}
+
 // One pass: (layout), generate, `loops` x (extend, guiding inference, clear the next
 // queue, shade), (training), advance the cursor. Everything is a kernel on `s` with
 // device-resident counts and schedule, so the pass can be captured into a CUDA graph
@@ -937,6 +996,9 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   const GuideIO G{W.nets, W.lobes, W.recs, W.cnt + 2, W.rec_cap, W.lpath};
   const bool nee = W.Q.o != nullptr;
   unsigned* scnt = W.cnt + 3;
+  const bool media = W.media || W.nets;
+  auto shade = shade_kernel(nee, W.nets != nullptr, media);
+  const int threads = media ? kShadeThreads<true> : kShadeThreads<false>;
   PathSoA cur = W.A, nxt = W.B;
   unsigned *cc = W.cnt, *cn = W.cnt + 1;
   // the extension rays of a queue, and the visibility rays of the bounce before
@@ -954,9 +1016,8 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
     extend(cur, cc, order);
     if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, cc, grid, s);
     k_zero<<<1, 1, 0, s>>>(cn, W.ctr + kExtendCursor, scnt);
-    auto shade = nee ? (W.nets ? k_shade<true, true> : k_shade<true, false>)
-                     : (W.nets ? k_shade<false, true> : k_shade<false, false>);
-    shade<<<grid, 128, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.Q, scnt, G);
+    shade<<<grid * 128 / threads, threads, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.Q, scnt, G,
+                                                   W.sort);
     std::swap(cur, nxt);
     std::swap(cc, cn);
   }
@@ -1090,7 +1151,12 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
   if ((e = alloc_soa(W.B, c->ws, slots)) != cudaSuccess) return e;
   if (!(W.hit = static_cast<int2*>(alloc(slots * sizeof(int2))))) return e;
   bool any_nee = false;
-  for (int k = 0; k < nj; k++) any_nee = any_nee || recs[k].P.nee;
+  for (int k = 0; k < nj; k++) {
+    any_nee = any_nee || recs[k].P.nee;
+    W.media = W.media || recs[k].S.num_media > 0;
+    for (const rx_object& o : jobs[k].ctx->objects)
+      W.sort = W.sort || (o.material != RX_MAT_DIFFUSE && o.material != RX_MAT_EMISSIVE);
+  }
   if (any_nee) {  // at most one visibility ray per live path
     for (float4** q : {&W.Q.o, &W.Q.d, &W.Q.lit, &W.Q.dark})
       if (!(*q = static_cast<float4*>(alloc((size_t)slots * sizeof(float4))))) return e;
