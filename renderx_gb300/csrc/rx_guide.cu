@@ -216,20 +216,29 @@ __device__ void encode_row(const float (&q)[9], bool valid, const Box& box, unsi
   store_chunk(A0, tc::core_off(s, 72, kIn), f);
 }
 
-// Hidden-layer epilogue: the thread's accumulator row (64 columns) -> ReLU -> BF16 row s.
+// Hidden-layer epilogue: the thread's accumulator row (64 columns) -> BF16 -> ReLU -> row s.
+// (Rounding keeps the sign, so the packed maximum gives the rounded ReLU, NaN to 0 as
+// fmaxf does, in half the instructions.)
+__device__ __forceinline__ uint32_t pack_relu(float a, float b) {
+  uint32_t r = pack_bf16(a, b);
+  asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+  return r;
+}
 __device__ __forceinline__ void epi_relu(uint32_t tacc, unsigned char* out, int s) {
+  unsigned char* row = out + tc::core_off(s, 0, kHid);
 #pragma unroll
   for (int c0 = 0; c0 < kHid; c0 += 16) {
     float v[16];
     tc::tmem_ld16(tacc + c0, v);
-    float a[8], b[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      a[i] = fmaxf(v[i], 0.0f);
-      b[i] = fmaxf(v[8 + i], 0.0f);
+    for (int h = 0; h < 16; h += 8) {
+      uint4 u;
+      u.x = pack_relu(v[h], v[h + 1]);
+      u.y = pack_relu(v[h + 2], v[h + 3]);
+      u.z = pack_relu(v[h + 4], v[h + 5]);
+      u.w = pack_relu(v[h + 6], v[h + 7]);
+      *reinterpret_cast<uint4*>(row + (c0 + h) / 8 * 128) = u;
     }
-    store_chunk(out, tc::core_off(s, c0, kHid), a);
-    store_chunk(out, tc::core_off(s, c0 + 8, kHid), b);
   }
 }
 
@@ -308,36 +317,69 @@ __device__ float mix_loss_grad(const float (&raw)[48], const float (&wi)[3], flo
   return -scale * lq;
 }
 
-// Mixture for sampling / evaluation: per lobe weight, kappa, mean, weight x normaliser
-// (kLobes x kLobeFloats floats, written as 16-byte stores; `out` 16-byte aligned).
-__device__ void mix_store(const float (&raw)[48], float* out) {
-  Lobe L[kLobes];
-  decode(raw, L);
-  float o[kLobes * kLobeFloats];
+// The 40 raw outputs of the thread's accumulator row.
+__device__ __forceinline__ void load_outputs(uint32_t tacc, float (&v)[kOutUsed]) {
 #pragma unroll
-  for (int j = 0; j < kLobes; j++) {
-    o[j * kLobeFloats + 0] = expf(L[j].logpi);
-    o[j * kLobeFloats + 1] = L[j].kappa;
-    o[j * kLobeFloats + 2] = L[j].mu[0];
-    o[j * kLobeFloats + 3] = L[j].mu[1];
-    o[j * kLobeFloats + 4] = L[j].mu[2];
-    o[j * kLobeFloats + 5] = expf(L[j].logpi + L[j].lognorm);
+  for (int c0 = 0; c0 < kOutUsed; c0 += 8) {
+    float u[8];
+    tc::tmem_ld8(tacc + c0, u);
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[c0 + k] = u[k];
   }
-  float4* o4 = reinterpret_cast<float4*>(out);
-#pragma unroll
-  for (int k = 0; k < kLobes * kLobeFloats / 4; k++) o4[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
 }
 
-__device__ float mix_pdf_raw(const float (&raw)[48], const float (&wi)[3]) {
-  Lobe L[kLobes];
-  decode(raw, L);
-  float q = 0.0f;
+// Mixture for sampling / evaluation: per lobe weight, kappa, mean, weight x normaliser
+// (kLobes x kLobeFloats floats, written as 16-byte stores; `out` 16-byte aligned), with
+// decode's arithmetic, two lobes at a time (the inference kernel keeps 64 registers).
+__device__ __forceinline__ void mix_store(const float (&v)[kOutUsed], float* out) {
+  float amax = v[0];
+#pragma unroll
+  for (int j = 1; j < kLobes; j++) amax = fmaxf(amax, v[5 * j]);
+  float z = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kLobes; j++) z += expf(v[5 * j] - amax);
+  const float logz = amax + logf(z);
+#pragma unroll
+  for (int p = 0; p < kLobes / 2; p++) {
+    float o[2 * kLobeFloats];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float* r = v + 10 * p + 5 * h;
+      const float logpi = r[0] - logz;
+      const float kappa = expf(fminf(fmaxf(r[1], kLogKMin), kLogKMax));
+      const float len = fmaxf(sqrtf(r[2] * r[2] + r[3] * r[3] + r[4] * r[4]), 1e-6f);
+      const float lognorm = logf(kappa) - logf(2.0f * RX_PI) - logf(-expm1f(-2.0f * kappa));
+      o[h * kLobeFloats + 0] = expf(logpi);
+      o[h * kLobeFloats + 1] = kappa;
+      o[h * kLobeFloats + 2] = r[2] / len;
+      o[h * kLobeFloats + 3] = r[3] / len;
+      o[h * kLobeFloats + 4] = r[4] / len;
+      o[h * kLobeFloats + 5] = expf(logpi + lognorm);
+    }
+    float4* o4 = reinterpret_cast<float4*>(out) + 3 * p;
+#pragma unroll
+    for (int k = 0; k < 3; k++) o4[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+  }
+}
+
+// The mixture's density at wi: sum_j softmax_j x kappa_j / (2 pi (1 - e^{-2 kappa_j})) x
+// e^{kappa_j (mu_j . wi - 1)}, without the logarithms that the training loss needs.
+__device__ __forceinline__ float mix_pdf_raw(const float (&v)[kOutUsed], const float (&wi)[3]) {
+  float amax = v[0];
+#pragma unroll
+  for (int j = 1; j < kLobes; j++) amax = fmaxf(amax, v[5 * j]);
+  float z = 0.0f, q = 0.0f;
 #pragma unroll
   for (int j = 0; j < kLobes; j++) {
-    float t = L[j].mu[0] * wi[0] + L[j].mu[1] * wi[1] + L[j].mu[2] * wi[2];
-    q += expf(L[j].logpi + L[j].lognorm + L[j].kappa * (t - 1.0f));
+    const float w = expf(v[5 * j] - amax);
+    const float kappa = expf(fminf(fmaxf(v[5 * j + 1], kLogKMin), kLogKMax));
+    const float m0 = v[5 * j + 2], m1 = v[5 * j + 3], m2 = v[5 * j + 4];
+    const float len = fmaxf(sqrtf(m0 * m0 + m1 * m1 + m2 * m2), 1e-6f);
+    const float t = (m0 * wi[0] + m1 * wi[1] + m2 * wi[2]) / len;
+    z += w;
+    q += w * (kappa / -expm1f(-2.0f * kappa)) * expf(kappa * (t - 1.0f));
   }
-  return q;
+  return q / (z * (2.0f * RX_PI));
 }
 
 // Issues the forward MMAs of layer l (A: 128 x K K-major, W: 64 x K K-major) into `tacc`.
@@ -352,6 +394,17 @@ __device__ __forceinline__ void issue_fwd(uint32_t tacc, const unsigned char* A,
   }
 }
 
+// The same for layer L, with descriptors that are one constant apart: the issuing lane's
+// instructions are on every layer's critical path.
+template <int L>
+__device__ __forceinline__ void issue_layer(uint32_t tacc, uint32_t a0, uint32_t w0) {
+  constexpr int K = layer_k(L);
+  constexpr uint32_t id = tc::idesc_bf16(128, 64, false, false), sbo = (uint32_t)(K >> 3) * 128u;
+  const uint64_t ad = tc::sdesc(a0, 128u, sbo), wd = tc::sdesc(w0 + layer_img(L), 128u, sbo);
+#pragma unroll
+  for (int k = 0; k < K / 16; k++) tc::mma_bf16(tacc, ad + 16u * k, wd + 16u * k, id, k > 0);
+}
+
 // Block-wide barrier that also orders tensor-core work and generic shared-memory writes.
 __device__ __forceinline__ void tc_sync() {
   tc::fence_async_smem();
@@ -363,10 +416,10 @@ __device__ __forceinline__ void tc_sync() {
 // Shared-memory plan of the network kernels (bytes from the dynamic base).
 constexpr uint32_t kSmW = 0;                         // weight image, then the per-tile buffers
 constexpr uint32_t kActBytes = 128 * kHid * 2;       // one 128 x 64 BF16 activation tile
-constexpr int kInferTiles = 4;  // inference tiles in flight per CTA, one warpgroup each
-// per tile: the 128 x 80 input (its first 16 KB also hold the odd layers' outputs) and one
-// 128 x 64 activation buffer
-constexpr uint32_t kInferTileBytes = 128 * kIn * 2 + kActBytes;
+// per inference tile one buffer: the 128 x 80 input, then each hidden layer's 128 x 64
+// output in its place (a layer's MMAs have read their input when its output is written),
+// then the 128 x 40 raw outputs on their way out
+constexpr uint32_t kInferTileBytes = 128 * kIn * 2;
 constexpr uint32_t kSmInfer = kImgBytes + kInferTiles * kInferTileBytes;
 
 // Loads the weight image into shared memory with bulk copies (one per layer).
@@ -407,13 +460,31 @@ struct RecordIO {
     wi[0] = p.c.y; wi[1] = p.c.z; wi[2] = p.c.w;
     return valid;
   }
-  __device__ void store(uint32_t i, const float (&raw)[48], const float (&wi)[3]) const {
+  // Raw outputs leave by one bulk copy per warp: its 32 rows are contiguous, and 16-byte
+  // stores of a thread to its own row fill half a sector each. `stage`: the warp's 5,120
+  // bytes of the tile's buffer; `first`, `rows`: the warp's queries.
+  __device__ void store(uint32_t i, bool valid, uint32_t tacc, const float (&wi)[3], unsigned char* stage,
+                        uint32_t first, uint32_t rows) const {
+    const int lane = threadIdx.x & 31;
+    float v[kOutUsed];
+    load_outputs(tacc, v);
     if (raw_out) {
-      float4* o = reinterpret_cast<float4*>(raw_out + (size_t)i * kOutUsed);
+      float4* o = reinterpret_cast<float4*>(stage + (uint32_t)lane * kOutUsed * 4);
 #pragma unroll
-      for (int k = 0; k < kOutUsed / 4; k++) o[k] = make_float4(raw[4 * k], raw[4 * k + 1], raw[4 * k + 2], raw[4 * k + 3]);
+      for (int k = 0; k < kOutUsed / 4; k++) o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0 && rows) tc::bulk_s2g(raw_out + (size_t)first * kOutUsed, stage, rows * kOutUsed * 4);
     }
-    if (pdf_out) pdf_out[i] = mix_pdf_raw(raw, wi);
+    if (pdf_out) {
+      const float q = mix_pdf_raw(v, wi);
+      if (valid) pdf_out[i] = q;
+    }
+  }
+  // The stage is free again (by the lane that issued the copy).
+  __device__ void reuse_stage() const {
+    if ((threadIdx.x & 31) == 0) tc::bulk_read_done();
+    __syncwarp();
   }
 };
 
@@ -467,9 +538,13 @@ struct PathIO {
     q[6] = -p.d.x; q[7] = -p.d.y; q[8] = -p.d.z;
     return true;
   }
-  __device__ void store(uint32_t i, const float (&raw)[48], const float (&)[3]) const {
-    mix_store(raw, lobes + (size_t)i * kLobeStride);
+  __device__ void store(uint32_t i, bool valid, uint32_t tacc, const float (&)[3], unsigned char*, uint32_t,
+                        uint32_t) const {
+    float v[kOutUsed];
+    load_outputs(tacc, v);
+    if (valid) mix_store(v, lobes + (size_t)i * kLobeStride);
   }
+  __device__ void reuse_stage() const {}
 };
 
 // Barrier of warpgroup g (its 128 threads, named barrier g + 1) that also orders
@@ -504,20 +579,52 @@ __device__ __forceinline__ int seg_of(const uint32_t* seg, int nnet, uint32_t r)
   return lo;
 }
 
+// One layer of a warpgroup's tile: its MMAs, then (hidden layers) the output in the input's
+// place. Every thread takes part whatever `ok` says; a wait that gave up clears it.
+template <int L>
+__device__ __forceinline__ void layer(int g, int warp, int s, uint32_t tcol, uint32_t tacc, unsigned char* A, uint32_t a0,
+                                      uint32_t w_img, uint64_t* bar, uint32_t& ph, bool& ok) {
+  if ((warp & 3) == 0 && __all_sync(0xffffffffu, ok) && tc::elect_one()) {
+    issue_layer<L>(tcol, a0, w_img);
+    tc::mma_commit(bar);
+  }
+  __syncwarp();
+  if (ok) ok = tc::mbar_wait(bar, ph);
+  ph ^= 1;
+  __syncwarp();
+  tc::tc_fence_after();
+  if (L < 4) {
+    epi_relu(tacc, A, s);
+    wg_sync(g);
+  }
+}
+
 // Persistent inference: kInferTiles warpgroups per CTA share the weight image and each
-// runs its own 128-sample tiles through the five layers (its own input / activation
-// buffers, TMEM columns 64 g .. 64 g + 63, mbarrier, and MMA-issuing thread), so several
-// tiles' MMA -> epilogue chains interleave on the SM. The next tile's inputs are loaded
-// while the current one runs. A CTA's step covers kInferTiles consecutive tiles (tile
-// 4 st + g for warpgroup g).
+// runs its own 128-sample tiles through the five layers (its own buffer, TMEM columns
+// 64 g .. 64 g + 63, mbarrier, and MMA-issuing thread), so several tiles' MMA -> epilogue
+// chains interleave on the SM. The next tile's inputs are loaded while the current one
+// runs.
 //
-// GROUPED: rows[r] (or -1 for padding) name the queries, and network k owns rows
-// [seg[k], seg[k + 1]) (multiples of kGroupRows, so a step's four tiles share one
-// network). When a step's network differs from the staged one, the CTA waits until every
-// warpgroup is done with the old weights and stages the new ones (bulk copy, 43 KB).
-// Steps run in increasing row order per CTA, so a CTA stages each network at most once.
-// Every warpgroup runs the same number of steps; a failed wait skips the remaining work
-// instead of leaving the loop, so the CTA-wide barriers stay matched.
+// The chain of a tile is latency and instruction issue (five dependent MMA -> tensor-memory
+// load -> BF16 store steps; the tensor pipe is active 12% of the time), so the SM holds as
+// many tiles as tensor memory has room for accumulators: eight of 64 columns, with one
+// buffer each (the layers' outputs in place) and 64 registers a thread; and the lane that
+// issues the MMAs works from uniform registers and constants (600 cycles a layer as a loop
+// over addresses, with the tile's other warps waiting). 2^20 records, raw outputs and
+// densities: 156 us with four tiles (two buffers each, 128 registers, the outputs stored by
+// rows), 130 with eight, 90 with the short issue, 82 with the outputs loaded at once (35 us
+// of DRAM traffic). The mixtures of a 512^2 x 8 guided frame: 1,051 -> 781 us.
+//
+// Ungrouped: tile (k kInferTiles + g) gridDim + b for warpgroup g of CTA b, so few tiles
+// spread over the SMs first.
+// GROUPED: rows[r] (or -1 for padding) name the queries, a CTA's step covers kInferTiles
+// consecutive tiles, and network k owns rows [seg[k], seg[k + 1]) (multiples of kGroupRows,
+// so a step's tiles share one network). When a step's network differs from the staged one,
+// the CTA waits until every warpgroup is done with the old weights and stages the new ones
+// (bulk copy, 43 KB). Steps run in increasing row order per CTA, so a CTA stages each
+// network at most once. Every warpgroup runs the same number of steps.
+//
+// A failed wait (status) skips the MMAs and waits that remain, never a barrier.
 template <class IO, bool GROUPED>
 __global__ void __launch_bounds__(128 * kInferTiles, 1)
     k_guide_infer(IO io, const unsigned* count, uint32_t n_host, const NetDev* nets, int nnet, const int* rows,
@@ -525,16 +632,34 @@ __global__ void __launch_bounds__(128 * kInferTiles, 1)
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar_mma[kInferTiles], bar_w;
   __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, s = tid & 127;
-  uint32_t n = 0, nsteps;
+  // the warp's number made uniform, so that what the issuing lane needs stays in uniform registers
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), g = warp >> 2, s = tid & 127;
+  uint32_t n, ntiles;  // queries (GROUPED: rows), tiles
   if constexpr (GROUPED) {
-    nsteps = __ldg(&seg[nnet]) / kGroupRows;
+    n = __ldg(&seg[nnet]);
+    if (blockIdx.x * kGroupRows >= n) return;
   } else {
     if (pass && *pass < nets[0].warmup) return;
     n = count ? *count : n_host;
-    nsteps = (n + kGroupRows - 1) / kGroupRows;
+    if (blockIdx.x * (uint32_t)kTile >= n) return;
   }
-  if (blockIdx.x >= nsteps) return;
+  ntiles = (n + kTile - 1) / kTile;
+  // the query of row r: its index and whether it exists
+  auto query = [&](uint32_t r, uint32_t& i) -> bool {
+    i = r;
+    if (r >= n) return false;
+    if constexpr (GROUPED) {
+      const int q = __ldg(&rows[r]);
+      i = (uint32_t)q;
+      return q >= 0;
+    }
+    return true;
+  };
+  const uint32_t first = GROUPED ? blockIdx.x * kInferTiles + (uint32_t)g : (uint32_t)g * gridDim.x + blockIdx.x;
+  const uint32_t step = gridDim.x * kInferTiles;
+  uint32_t qi = 0;
+  bool qv = query(first * kTile + (uint32_t)s, qi);
+  typename IO::Pre pre = io.prefetch(qi, qv);
   if (tid == 0) {
     for (int k = 0; k < kInferTiles; k++) tc::mbar_init(&bar_mma[k], 1);
     tc::mbar_init(&bar_w, 1);
@@ -549,29 +674,13 @@ __global__ void __launch_bounds__(128 * kInferTiles, 1)
   const uint32_t tacc = tcol + ((uint32_t)((warp & 3) * 32) << 16);
   bool ok = __syncthreads_and(tc::mbar_wait(&bar_w, 0));
   uint32_t wph = 1;
-  Box box = nets[net].box;
   uint32_t ph = 0;
-  unsigned char* A0 = sm + kImgBytes + (uint32_t)g * kInferTileBytes;
-  unsigned char* A1 = A0 + 128 * kIn * 2;
-  // the query of row r: its index and whether it exists
-  auto query = [&](uint32_t r, uint32_t& i) -> bool {
+  unsigned char* A = sm + kImgBytes + (uint32_t)g * kInferTileBytes;
+  const uint32_t a0 = tc::smem_u32(A), w_img = tc::smem_u32(sm + kSmW);
+  unsigned char* stage = A + (uint32_t)(warp & 3) * (kInferTileBytes / 4);  // the warp's rows of the input
+  for (uint32_t tile = first; tile < ntiles; tile += step) {
     if constexpr (GROUPED) {
-      if (r >= nsteps * kGroupRows) return false;
-      int q = __ldg(&rows[r]);
-      i = (uint32_t)q;
-      return q >= 0;
-    } else {
-      i = r;
-      return r < n;
-    }
-  };
-  uint32_t st = blockIdx.x;
-  uint32_t qi = 0;
-  bool qv = query((st * kInferTiles + (uint32_t)g) * kTile + (uint32_t)s, qi);
-  typename IO::Pre pre = io.prefetch(qi, qv);
-  for (; st < nsteps; st += gridDim.x) {
-    if constexpr (GROUPED) {
-      const int j = seg_of(seg, nnet, st * kGroupRows);  // the same for the whole CTA
+      const int j = seg_of(seg, nnet, tile / kInferTiles * kGroupRows);  // the same for the whole CTA
       if (j != net) {
         tc::tc_fence_before();
         ok = __syncthreads_and(ok);  // every warpgroup's MMAs on the old weights are complete
@@ -580,40 +689,27 @@ __global__ void __launch_bounds__(128 * kInferTiles, 1)
         if (ok) ok = __syncthreads_and(tc::mbar_wait(&bar_w, wph));
         wph ^= 1;
         net = j;
-        box = nets[j].box;
       }
-    } else {
-      if (!ok) break;
     }
-    const uint32_t tile = st * kInferTiles + (uint32_t)g;
     const uint32_t i = qi;
     float q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, wi[3] = {0, 0, 0};
     const bool valid = io.finish(pre, i, qv, q, wi);
-    qv = query(((st + gridDim.x) * kInferTiles + (uint32_t)g) * kTile + (uint32_t)s, qi);
+    qv = query((tile + step) * kTile + (uint32_t)s, qi);
     pre = io.prefetch(qi, qv);
-    if (!GROUPED && tile * kTile >= n) continue;  // this warpgroup's tile is past the end
-    if (!ok) continue;
-    encode_row(q, valid, box, A0, s);
+    io.reuse_stage();
+    encode_row(q, valid, nets[net].box, A, s);
     wg_sync(g);
-    float raw[48];
-    for (int l = 0; l < 5; l++) {
-      // layer l reads A0 (l = 0, 2, 4) or A1 (l = 1, 3) and writes the other
-      const unsigned char* A = (l & 1) ? A1 : A0;
-      if (s == 0) {
-        issue_fwd(tcol, A, sm + kSmW + layer_img(l), layer_k(l));
-        tc::mma_commit(&bar_mma[g]);
-      }
-      ok = wg_and(g, tc::mbar_wait(&bar_mma[g], ph));
-      ph ^= 1;
-      tc::tc_fence_after();
-      if (!ok) break;
-      if (l < 4) epi_relu(tacc, (l & 1) ? A0 : A1, s);
-      else load_raw(tacc, raw);
-      wg_sync(g);
-    }
-    if (ok && valid) io.store(i, raw, wi);
+    layer<0>(g, warp, s, tcol, tacc, A, a0, w_img, &bar_mma[g], ph, ok);
+    layer<1>(g, warp, s, tcol, tacc, A, a0, w_img, &bar_mma[g], ph, ok);
+    layer<2>(g, warp, s, tcol, tacc, A, a0, w_img, &bar_mma[g], ph, ok);
+    layer<3>(g, warp, s, tcol, tacc, A, a0, w_img, &bar_mma[g], ph, ok);
+    layer<4>(g, warp, s, tcol, tacc, A, a0, w_img, &bar_mma[g], ph, ok);
+    const uint32_t w0 = tile * kTile + 32u * (uint32_t)(warp & 3);
+    io.store(i, valid && ok, tacc, wi, stage, w0, ok ? (w0 < n ? min(32u, n - w0) : 0u) : 0u);
+    tc::tc_fence_before();
   }
-  if (!ok && s == 0) atomicExch(nets[net].status, 1);
+  if ((tid & 31) == 0) tc::bulk_done();
+  if (!ok) atomicExch(nets[net].status, 1);
   tc::tc_fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem_base, 64 * kInferTiles);
@@ -1222,8 +1318,8 @@ extern "C" rx_status rx_guide_eval(rx_context* c, const float* recs, uint32_t n,
   cudaMemcpy(dr.p, recs, (size_t)n * rx::guide::kRec * 4, cudaMemcpyHostToDevice);
   rx::set_kernel_smem();
   rx::RecordIO io{dr.as<float>(), draw.as<float>(), dp.as<float>()};
-  uint32_t grid = std::min<uint32_t>((n + rx::guide::kGroupRows - 1) / rx::guide::kGroupRows, (uint32_t)g->sms);
-  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::kInferTiles, rx::kSmInfer, c->stream>>>(
+  uint32_t grid = std::min<uint32_t>((n + rx::guide::kTile - 1) / rx::guide::kTile, (uint32_t)g->sms);
+  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::guide::kInferTiles, rx::kSmInfer, c->stream>>>(
       io, nullptr, n, g->dnet.as<rx::guide::NetDev>(), 1, nullptr, nullptr, nullptr);
   if ((s = c->cuda(cudaStreamSynchronize(c->stream), "guide eval")) != RX_OK) return s;
   if ((s = guide_status(c)) != RX_OK) return s;
@@ -1245,7 +1341,7 @@ extern "C" rx_status rx_guide_eval_device(rx_context* c, const float* d_recs, ui
   rx::RecordIO io{d_recs, d_raw40, d_pdf};
   uint32_t grid = std::min<uint32_t>((n + rx::guide::kGroupRows - 1) / rx::guide::kGroupRows, (uint32_t)g->sms);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::kInferTiles, rx::kSmInfer, st>>>(
+  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::guide::kInferTiles, rx::kSmInfer, st>>>(
       io, nullptr, n, g->dnet.as<rx::guide::NetDev>(), 1, nullptr, nullptr, nullptr);
   return c->cuda(cudaGetLastError(), "guide eval");
 }

@@ -96,8 +96,9 @@ struct RecSeg {
 };
 
 // Rows of a grouped inference: each network's rows are a segment padded to a multiple of
-// kGroupRows (one inference CTA's four tiles), so a CTA's tiles share one network.
-constexpr uint32_t kGroupRows = 4 * kTile;
+// kGroupRows (one inference CTA's tiles), so a CTA's tiles share one network.
+constexpr int kInferTiles = 8;  // inference tiles in flight per CTA, one warpgroup each
+constexpr uint32_t kGroupRows = kInferTiles * kTile;
 
 }  // namespace guide
 
