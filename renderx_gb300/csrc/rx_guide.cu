@@ -189,9 +189,12 @@ __device__ __forceinline__ void store_chunk(unsigned char* base, uint32_t off, c
 // sincospif, each next one from the double-angle identities (sin 2a = 2 sin a cos a,
 // cos 2a = (cos a - sin a)(cos a + sin a)): the angle error doubles per step, about
 // 1e-4 at f = 11, far below the BF16 rounding of the features (4e-3).
-__device__ void encode_row(const float (&q)[9], bool valid, const Box& box, unsigned char* A0, int s) {
+// [c0, c1): the coordinates to encode; rest: also the features past the position's.
+__device__ __forceinline__ void encode_row(const float (&q)[9], bool valid, const Box& box, unsigned char* A0, int s,
+                                           int c0 = 0, int c1 = 3, bool rest = true) {
 #pragma unroll
   for (int c = 0; c < 3; c++) {
+    if (c < c0 || c >= c1) continue;
     float p = valid ? __fdiv_rn(__fsub_rn(q[c], box.mn[c]), box.ext[c]) : 0.0f;
     float sn = 0.0f, cs = 0.0f;
     if (valid) sincospif(p, &sn, &cs);
@@ -209,6 +212,7 @@ __device__ void encode_row(const float (&q)[9], bool valid, const Box& box, unsi
       store_chunk(A0, tc::core_off(s, c * 24 + part * 8, kIn), f);
     }
   }
+  if (!rest) return;
   float f[8] = {q[3], q[4], q[5], q[6], q[7], q[8], 1.0f, 0.0f};
   if (!valid)
 #pragma unroll
@@ -242,80 +246,7 @@ __device__ __forceinline__ void epi_relu(uint32_t tacc, unsigned char* out, int 
   }
 }
 
-__device__ __forceinline__ void load_raw(uint32_t tacc, float (&raw)[48]) {
-#pragma unroll
-  for (int c0 = 0; c0 < 48; c0 += 16) {
-    float v[16];
-    tc::tmem_ld16(tacc + c0, v);
-#pragma unroll
-    for (int i = 0; i < 16; i++) raw[c0 + i] = v[i];
-  }
-}
-
 constexpr float kLogKMin = -4.0f, kLogKMax = 8.0f;
-
-// Lobe j of the raw outputs: log weight (log-softmax), concentration, mean, and the log
-// of the vMF normaliser kappa / (2 pi (1 - e^{-2 kappa})).
-struct Lobe {
-  float logpi, kappa, mu[3], len, lognorm;
-  bool kin;  // log-concentration inside its clamp range (gradient flows)
-};
-__device__ __forceinline__ void decode(const float (&raw)[48], Lobe (&L)[kLobes]) {
-  float amax = raw[0];
-#pragma unroll
-  for (int j = 1; j < kLobes; j++) amax = fmaxf(amax, raw[5 * j]);
-  float z = 0.0f;
-#pragma unroll
-  for (int j = 0; j < kLobes; j++) z += expf(raw[5 * j] - amax);
-  float logz = amax + logf(z);
-#pragma unroll
-  for (int j = 0; j < kLobes; j++) {
-    Lobe& l = L[j];
-    l.logpi = raw[5 * j] - logz;
-    float b = raw[5 * j + 1];
-    l.kin = b > kLogKMin && b < kLogKMax;
-    l.kappa = expf(fminf(fmaxf(b, kLogKMin), kLogKMax));
-    float m0 = raw[5 * j + 2], m1 = raw[5 * j + 3], m2 = raw[5 * j + 4];
-    l.len = fmaxf(sqrtf(m0 * m0 + m1 * m1 + m2 * m2), 1e-6f);
-    l.mu[0] = m0 / l.len;
-    l.mu[1] = m1 / l.len;
-    l.mu[2] = m2 / l.len;
-    l.lognorm = logf(l.kappa) - logf(2.0f * RX_PI) - logf(-expm1f(-2.0f * l.kappa));
-  }
-}
-
-// -scale * log q(wi) and its gradient with respect to the 40 raw outputs (returns the former).
-__device__ float mix_loss_grad(const float (&raw)[48], const float (&wi)[3], float scale, float (&dz)[48]) {
-  Lobe L[kLobes];
-  decode(raw, L);
-  float lv[kLobes], t[kLobes];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int j = 0; j < kLobes; j++) {
-    t[j] = L[j].mu[0] * wi[0] + L[j].mu[1] * wi[1] + L[j].mu[2] * wi[2];
-    lv[j] = L[j].logpi + L[j].lognorm + L[j].kappa * (t[j] - 1.0f);
-    mx = fmaxf(mx, lv[j]);
-  }
-  float sum = 0.0f;
-#pragma unroll
-  for (int j = 0; j < kLobes; j++) sum += expf(lv[j] - mx);
-  float lq = mx + logf(sum);
-#pragma unroll
-  for (int j = 0; j < kLobes; j++) {
-    float g = expf(lv[j] - lq);  // responsibility
-    float pi = expf(L[j].logpi);
-    float k = L[j].kappa;
-    dz[5 * j] = scale * (pi - g);
-    float dk = 1.0f - 2.0f * k / expm1f(2.0f * k) + k * (t[j] - 1.0f);  // kappa * d log v / d kappa
-    dz[5 * j + 1] = L[j].kin ? -scale * g * dk : 0.0f;
-    float c = -scale * g * k / L[j].len;
-#pragma unroll
-    for (int a = 0; a < 3; a++) dz[5 * j + 2 + a] = c * (wi[a] - t[j] * L[j].mu[a]);
-  }
-#pragma unroll
-  for (int i = kOutUsed; i < 48; i++) dz[i] = 0.0f;
-  return -scale * lq;
-}
 
 // The 40 raw outputs of the thread's accumulator row.
 __device__ __forceinline__ void load_outputs(uint32_t tacc, float (&v)[kOutUsed]) {
@@ -382,20 +313,9 @@ __device__ __forceinline__ float mix_pdf_raw(const float (&v)[kOutUsed], const f
   return q / (z * (2.0f * RX_PI));
 }
 
-// Issues the forward MMAs of layer l (A: 128 x K K-major, W: 64 x K K-major) into `tacc`.
-__device__ __forceinline__ void issue_fwd(uint32_t tacc, const unsigned char* A, const unsigned char* W, int K) {
-  const uint32_t id = tc::idesc_bf16(128, 64, false, false);
-  const uint32_t a0 = tc::smem_u32(A), w0 = tc::smem_u32(W);
-  const uint32_t sbo = (uint32_t)(K >> 3) * 128u;
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    uint64_t ad = tc::sdesc(a0 + tc::core_off(0, k0, K), 128u, sbo);
-    uint64_t wd = tc::sdesc(w0 + tc::core_off(0, k0, K), 128u, sbo);
-    tc::mma_bf16(tacc, ad, wd, id, k0 > 0);
-  }
-}
-
-// The same for layer L, with descriptors that are one constant apart: the issuing lane's
-// instructions are on every layer's critical path.
+// Issues the forward MMAs of layer L (A: 128 x K K-major at a0, W: 64 x K K-major in the
+// weight image at w0) into `tacc`, with descriptors that are one constant apart: the issuing
+// lane's instructions are on every layer's critical path.
 template <int L>
 __device__ __forceinline__ void issue_layer(uint32_t tacc, uint32_t a0, uint32_t w0) {
   constexpr int K = layer_k(L);
@@ -548,26 +468,13 @@ struct PathIO {
 };
 
 // Barrier of warpgroup g (its 128 threads, named barrier g + 1) that also orders
-// tensor-core work and generic shared-memory writes; and its AND-reduction.
+// tensor-core work and generic shared-memory writes.
 __device__ __forceinline__ void wg_sync(int g) {
   tc::fence_async_smem();
   tc::tc_fence_before();
   asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory");
   tc::tc_fence_after();
 }
-__device__ __forceinline__ bool wg_and(int g, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(g + 1)
-      : "memory");
-  return r != 0;
-}
-
 // Network k of a grouped launch: the segment of seg[0..nnet] holding row r.
 __device__ __forceinline__ int seg_of(const uint32_t* seg, int nnet, uint32_t r) {
   int lo = 0, hi = nnet - 1;
@@ -737,14 +644,11 @@ __device__ __forceinline__ bool net_trains(const NetDev& N, const uint32_t* pass
   return !pass || (*pass < N.train && (uint32_t)step < N.steps_per_pass);
 }
 
-// Clears each training network's step scratch (weight sum, count, loss).
+// The step scratch {weight sum, count, loss, k_adam's ticket}: the sums are zero between
+// steps (k_adam's last block clears them, or this after a gradient without an update).
 __global__ void k_net_clear(const NetDev* nets, int nnet, const uint32_t* pass, int step) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nnet && net_trains(nets[j], pass, step)) {
-    nets[j].scratch[0] = 0.0f;
-    nets[j].scratch[1] = 0.0f;
-    nets[j].scratch[2] = 0.0f;
-  }
+  if (j < nnet && net_trains(nets[j], pass, step)) nets[j].scratch[0] = nets[j].scratch[1] = 0.0f;
 }
 
 // Sum of record weights and number of records per network (the loss normalisation);
@@ -753,6 +657,7 @@ __global__ void k_weight_sum(const NetDev* nets, const RecSeg* segs, int per, in
   const int j = blockIdx.x / per;
   if (!net_trains(nets[j], pass, step)) return;
   const RecSeg R = segs[j];
+  if (blockIdx.x % per == 0 && threadIdx.x == 0) nets[j].scratch[2] = 0.0f;  // the loss (k_guide_train adds to it)
   uint32_t lo, end;
   train_window(R, step, lo, end);
   float acc = 0.0f;
@@ -777,17 +682,25 @@ __global__ void k_weight_sum(const NetDev* nets, const RecSeg* segs, int per, in
 // scratch holds {sum w, count}; weights are clipped at 32 x their batch mean before
 // normalisation by the sum. CTAs [j * per, (j + 1) * per) train network j.
 //
-// A CTA carries kTrainTiles tiles of 128 samples at once, one warpgroup per tile (thread
-// s of warpgroup g owns sample s of tile g, TMEM lane s of that tile's accumulator). The
-// warpgroups run independently (own MMA-issuing thread, mbarrier and named barrier), so
-// one tile's epilogues overlap the other's MMAs; both add into the shared
-// weight-gradient accumulators, zeroed once, which the tensor core updates one MMA at a
-// time. The 128 x 80 input tile is not kept: it lives in the region of activations 3-4
-// during the forward pass and is encoded again from the records for the last weight
-// gradient.
+// A CTA carries kTrainTiles tiles of 128 samples at once, as many as shared memory holds the
+// activations of, with two warpgroups per tile: both hold sample s in thread s (TMEM lane s
+// of the tile's accumulator) and take half of its columns in every step, and half of its
+// lobes in the loss (the lobes' log densities meet in shared memory). The tiles run
+// independently (own MMA-issuing lane, mbarrier and named barrier), so one tile's epilogues
+// overlap the other's MMAs; both add into the shared weight-gradient accumulators, zeroed
+// once, which the tensor core updates one MMA at a time. The 128 x 80 input tile is not
+// kept: it lives in the region of activations 3-4 during the forward pass and is encoded
+// again from the records for the last weight gradient.
+//
+// Latency-bound (ten dependent MMA -> tensor-memory load -> store steps a tile, two tiles
+// an SM): one warpgroup per tile, descriptors formed per MMA by the issuing thread, two
+// barriers a layer and scalar atomics in the flush made a step 201 us at 2^18 records and 80 at 2^12;
+// now 97 and 29 us (104 and 37 before k_adam took the two bookkeeping launches).
 constexpr int kTrainTiles = 2;
+constexpr int kTrainThreads = 256 * kTrainTiles;
 constexpr uint32_t kTrainTileBytes = 5 * kActBytes;  // A1, A2, A3|A4 (A0 alias), dZ
-constexpr uint32_t kSmTrain2 = kImgBytes + kTrainTiles * kTrainTileBytes;
+constexpr uint32_t kLobeBytes = kLobes * kTile * 4;  // the lobes' log densities of a tile
+constexpr uint32_t kSmTrain2 = kImgBytes + kTrainTiles * (kTrainTileBytes + kLobeBytes);
 constexpr uint32_t kDwCols = 336;  // TMEM columns of the five weight-gradient accumulators
 
 __device__ __forceinline__ void load_record(const float* recs, uint32_t i, float (&q)[9], float (&wi)[3], float& w) {
@@ -798,13 +711,201 @@ __device__ __forceinline__ void load_record(const float* recs, uint32_t i, float
   w = e.x;
 }
 
-__global__ void __launch_bounds__(128 * kTrainTiles, 1)
+// Barrier of a tile's two warpgroups, ordering as wg_sync.
+__device__ __forceinline__ void tile_sync(int t) {
+  tc::fence_async_smem();
+  tc::tc_fence_before();
+  asm volatile("bar.sync %0, 256;" ::"r"(t + 1) : "memory");
+  tc::tc_fence_after();
+}
+
+// What a thread of the training kernel works on: tile t of the CTA, columns half h of it.
+struct TrainLane {
+  int t, h, warp, s;            // warp: of the CTA, uniform
+  uint32_t tcol, tacc;          // the tile's accumulator; with the warp's lanes
+  unsigned char *act[5], *dz;   // activations A0..A4 (A0 over A3), dZ
+  uint32_t w_img;
+  uint64_t* bar;
+  uint32_t ph;
+  bool ok;
+  // whether this warp issues the tile's MMAs, and its elected lane
+  __device__ __forceinline__ bool issues() const {
+    return (warp & 7) == 0 && __all_sync(0xffffffffu, ok) && tc::elect_one();
+  }
+  __device__ __forceinline__ void wait() {
+    __syncwarp();
+    if (ok) ok = tc::mbar_wait(bar, ph);
+    ph ^= 1;
+    __syncwarp();
+    tc::tc_fence_after();
+  }
+};
+
+template <int L>
+__device__ __forceinline__ void train_forward(TrainLane& T) {
+  if (T.issues()) {
+    issue_layer<L>(T.tcol, tc::smem_u32(T.act[L]), T.w_img);
+    tc::mma_commit(T.bar);
+  }
+  T.wait();
+  if (L < 4) {
+    unsigned char* row = T.act[L + 1] + tc::core_off(T.s, 32 * T.h, kHid);
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += 16) {
+      float v[16];
+      tc::tmem_ld16(T.tacc + 32 * T.h + c0, v);
+#pragma unroll
+      for (int k = 0; k < 16; k += 8) {
+        uint4 u;
+        u.x = pack_relu(v[k], v[k + 1]);
+        u.y = pack_relu(v[k + 2], v[k + 3]);
+        u.z = pack_relu(v[k + 4], v[k + 5]);
+        u.w = pack_relu(v[k + 6], v[k + 7]);
+        *reinterpret_cast<uint4*>(row + (c0 + k) / 8 * 128) = u;
+      }
+    }
+    tile_sync(T.t);
+  }
+}
+
+// dZ_{L+1} -> dW_L += dZ^T A_L and dA_L = dZ W_L -> dZ_L (masked by A_L).
+template <int L>
+__device__ __forceinline__ void train_backward(TrainLane& T, uint32_t t_dw) {
+  constexpr int K = layer_k(L);
+  if (T.issues()) {
+    constexpr uint32_t id_w = tc::idesc_bf16(64, (uint32_t)K, true, true);
+    constexpr uint32_t id_a = tc::idesc_bf16(128, (uint32_t)K, false, true);
+    const uint32_t dz0 = tc::smem_u32(T.dz), a0 = tc::smem_u32(T.act[L]), w0 = T.w_img + layer_img(L);
+    {  // 16 samples per MMA: the next two rows of core matrices of both operands
+      const uint64_t ad = tc::sdesc(dz0, (kOut >> 3) * 128u, 128u), bd = tc::sdesc(a0, (uint32_t)(K >> 3) * 128u, 128u);
+#pragma unroll
+      for (int k = 0; k < kTile / 16; k++)
+        tc::mma_bf16(t_dw, ad + (uint64_t)(tc::core_off(16 * k, 0, kOut) >> 4), bd + (uint64_t)(tc::core_off(16 * k, 0, K) >> 4), id_w, 1u);
+    }
+    if (L > 0) {
+      const uint64_t ad = tc::sdesc(dz0, 128u, (kOut >> 3) * 128u), bd = tc::sdesc(w0, (uint32_t)(K >> 3) * 128u, 128u);
+#pragma unroll
+      for (int k = 0; k < kOut / 16; k++)
+        tc::mma_bf16(T.tcol, ad + (uint64_t)(tc::core_off(0, 16 * k, kOut) >> 4), bd + (uint64_t)(tc::core_off(16 * k, 0, K) >> 4), id_a, k > 0);
+    }
+    tc::mma_commit(T.bar);
+  }
+  T.wait();
+  if (L > 0) {
+    const uint32_t off = tc::core_off(T.s, 32 * T.h, kHid);
+#pragma unroll
+    for (int c0 = 0; c0 < 32; c0 += 16) {
+      float v[16];
+      tc::tmem_ld16(T.tacc + 32 * T.h + c0, v);
+#pragma unroll
+      for (int k = 0; k < 16; k += 8) {
+        const uint32_t o = off + (c0 + k) / 8 * 128;
+        const uint4 m = *reinterpret_cast<const uint4*>(T.act[L] + o);
+        const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+        float a[8];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          a[2 * i] = bf16_lo(mw[i]) > 0.0f ? v[k + 2 * i] : 0.0f;
+          a[2 * i + 1] = bf16_hi(mw[i]) > 0.0f ? v[k + 2 * i + 1] : 0.0f;
+        }
+        store_chunk(T.dz, o, a);
+      }
+    }
+  }
+  tile_sync(T.t);
+}
+
+// The loss of sample s, -scale log q(wi), and its gradient with respect to the raw outputs as
+// dZ_5: this thread forms lobes 4 h .. 4 h + 3; `lv` (kLobes x 128) holds every lobe's log
+// density log(pi_j v_j(wi)) once the tile's threads have met. Returns the loss (one of the
+// two threads of a sample; `live` false: no contribution, zero gradient).
+__device__ __forceinline__ float train_loss(TrainLane& T, float* lv, const float (&wi)[3], float scale, bool live) {
+  float logit[kLobes], raw[20];  // every lobe's weight logit; this thread's four lobes
+  {
+    float v[kOutUsed];
+#pragma unroll
+    for (int c0 = 0; c0 < kOutUsed; c0 += 8) {
+      float u[8];
+      tc::tmem_ld8(T.tacc + c0, u);
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[c0 + k] = u[k];
+    }
+#pragma unroll
+    for (int j = 0; j < kLobes; j++) logit[j] = v[5 * j];
+#pragma unroll
+    for (int k = 0; k < 20; k++) raw[k] = T.h ? v[20 + k] : v[k];
+  }
+  float amax = logit[0], z = 0.0f;
+#pragma unroll
+  for (int j = 1; j < kLobes; j++) amax = fmaxf(amax, logit[j]);
+#pragma unroll
+  for (int j = 0; j < kLobes; j++) z += expf(logit[j] - amax);
+  const float logz = amax + logf(z);
+  float t[4], kap[4], len[4], lown[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float* r = raw + 5 * j;
+    kap[j] = expf(fminf(fmaxf(r[1], kLogKMin), kLogKMax));
+    len[j] = fmaxf(sqrtf(r[2] * r[2] + r[3] * r[3] + r[4] * r[4]), 1e-6f);
+    const float lognorm = logf(kap[j]) - logf(2.0f * RX_PI) - logf(-expm1f(-2.0f * kap[j]));
+    t[j] = (r[2] / len[j]) * wi[0] + (r[3] / len[j]) * wi[1] + (r[4] / len[j]) * wi[2];
+    lown[j] = (r[0] - logz) + lognorm + kap[j] * (t[j] - 1.0f);
+    lv[(4 * T.h + j) * kTile + T.s] = lown[j];
+  }
+  asm volatile("bar.sync %0, 256;" ::"r"(T.t + 1) : "memory");
+  float l[kLobes], mx = -INFINITY, sum = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kLobes; j++) {
+    l[j] = lv[j * kTile + T.s];
+    mx = fmaxf(mx, l[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < kLobes; j++) sum += expf(l[j] - mx);
+  const float lq = mx + logf(sum);
+  float d[20];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float* r = raw + 5 * j;
+    const float g = expf(lown[j] - lq);  // responsibility
+    const float k = kap[j];
+    d[5 * j] = scale * (expf(r[0] - logz) - g);
+    const float dk = 1.0f - 2.0f * k / expm1f(2.0f * k) + k * (t[j] - 1.0f);  // kappa * d log v / d kappa
+    d[5 * j + 1] = r[1] > kLogKMin && r[1] < kLogKMax ? -scale * g * dk : 0.0f;
+    const float c = -scale * g * k / len[j];
+#pragma unroll
+    for (int a = 0; a < 3; a++) d[5 * j + 2 + a] = c * (wi[a] - t[j] * (r[2 + a] / len[j]));
+  }
+#pragma unroll
+  for (int k = 0; k < 20; k++) d[k] = live ? d[k] : 0.0f;
+  // columns 0..19 (h = 0: two chunks and half of the third) or 20..63 (the third's other
+  // half, two chunks, then zeros)
+  unsigned char* row = T.dz + tc::core_off(T.s, 0, kOut);
+  const float (&c)[20] = d;
+  if (T.h == 0) {
+    const float f0[8] = {c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7]};
+    const float f1[8] = {c[8], c[9], c[10], c[11], c[12], c[13], c[14], c[15]};
+    store_chunk(row, 0, f0);
+    store_chunk(row, 128, f1);
+    *reinterpret_cast<uint2*>(row + 256) = make_uint2(pack_bf16(c[16], c[17]), pack_bf16(c[18], c[19]));
+  } else {
+    const float f0[8] = {c[4], c[5], c[6], c[7], c[8], c[9], c[10], c[11]};
+    const float f1[8] = {c[12], c[13], c[14], c[15], c[16], c[17], c[18], c[19]};
+    *reinterpret_cast<uint2*>(row + 264) = make_uint2(pack_bf16(c[0], c[1]), pack_bf16(c[2], c[3]));
+    store_chunk(row, 3 * 128, f0);
+    store_chunk(row, 4 * 128, f1);
+#pragma unroll
+    for (int k = 5; k < 8; k++) *reinterpret_cast<uint4*>(row + k * 128) = make_uint4(0, 0, 0, 0);
+  }
+  return live && T.h == 0 ? -scale * lq : 0.0f;
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
     k_guide_train(const NetDev* nets, const RecSeg* segs, int per, int step, const uint32_t* pass) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar_mma[kTrainTiles], bar_w;
   __shared__ uint32_t tmem_base;
-  __shared__ float red[4 * kTrainTiles];
-  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, s = tid & 127;
+  __shared__ float red[kTrainThreads / 32];
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int j = blockIdx.x / per, part = blockIdx.x % per;
   const NetDev& N = nets[j];
   if (!net_trains(N, pass, step)) return;
@@ -817,6 +918,11 @@ __global__ void __launch_bounds__(128 * kTrainTiles, 1)
   const uint32_t n = end - first;
   const uint32_t ntiles = (n + kTile - 1) / kTile;
   if ((uint32_t)part * kTrainTiles >= ntiles) return;
+  TrainLane T;
+  T.warp = warp;
+  T.t = warp >> 3;
+  T.h = (warp >> 2) & 1;
+  T.s = tid & 127;
   if (tid == 0) {
     for (int k = 0; k < kTrainTiles; k++) tc::mbar_init(&bar_mma[k], 1);
     tc::mbar_init(&bar_w, 1);
@@ -830,134 +936,78 @@ __global__ void __launch_bounds__(128 * kTrainTiles, 1)
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
   // TMEM columns: per tile one 64-column accumulator (forward, then dA); the shared dW
   const uint32_t t_dw[5] = {T0 + 128, T0 + 208, T0 + 272, T0 + 336, T0 + 400};
-  if (g == 0) {  // zero the weight-gradient accumulators (every MMA into them accumulates)
+  if (warp < 4) {  // zero the weight-gradient accumulators (every MMA into them accumulates)
     const float z[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (uint32_t c0 = 0; c0 < kDwCols; c0 += 16) tc::tmem_st16(T0 + 128 + lane_off + c0, z);
   }
-  unsigned char* A1 = sm + kImgBytes + (uint32_t)g * kTrainTileBytes;  // this warpgroup's buffers
-  unsigned char* A2 = A1 + kActBytes;
-  unsigned char* A34 = A1 + 2 * kActBytes;  // A3, A4; A0 (20 KB) aliases it
-  unsigned char* dZ = A1 + 4 * kActBytes;
-  unsigned char* Al[5] = {A34, A1, A2, A34, A34 + kActBytes};
-  const uint32_t tacc_col = T0 + 64u * (uint32_t)g;
-  const uint32_t t_acc = tacc_col + lane_off;
+  unsigned char* A1 = sm + kImgBytes + (uint32_t)T.t * kTrainTileBytes;  // this tile's buffers
+  unsigned char* A34 = A1 + 2 * kActBytes;                               // A3, A4; A0 (20 KB) aliases it
+  T.act[0] = A34;
+  T.act[1] = A1;
+  T.act[2] = A1 + kActBytes;
+  T.act[3] = A34;
+  T.act[4] = A34 + kActBytes;
+  T.dz = A1 + 4 * kActBytes;
+  float* lv = reinterpret_cast<float*>(sm + kImgBytes + kTrainTiles * kTrainTileBytes + (uint32_t)T.t * kLobeBytes);
+  T.tcol = T0 + 64u * (uint32_t)T.t;
+  T.tacc = T.tcol + lane_off;
+  T.w_img = tc::smem_u32(sm + kSmW);
+  T.bar = &bar_mma[T.t];
+  T.ph = 0;
   const float total = N.scratch[0], cnt = fmaxf(N.scratch[1], 1.0f);
   const float wclip = 32.0f * total / cnt;
   const float inv_total = total > 0.0f ? 1.0f / total : 0.0f;
   tc::tc_fence_before();
-  bool ok = __syncthreads_and(tc::mbar_wait(&bar_w, 0));
+  T.ok = __syncthreads_and(tc::mbar_wait(&bar_w, 0));
   tc::tc_fence_after();
-  uint32_t ph = 0;
   float loss = 0.0f;
-  for (uint32_t tile = (uint32_t)part * kTrainTiles + (uint32_t)g; ok && tile < ntiles;
-       tile += (uint32_t)per * kTrainTiles) {
-    const uint32_t i = first + tile * kTile + s;
+  for (uint32_t tile = (uint32_t)part * kTrainTiles + (uint32_t)T.t; tile < ntiles; tile += (uint32_t)per * kTrainTiles) {
+    const uint32_t i = first + tile * kTile + T.s;
     const bool valid = i < end;
     float q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, wi[3] = {0, 0, 0}, w = 0.0f;
     if (valid) {
       load_record(recs, i, q, wi, w);
       w = fminf(w, wclip) * inv_total;
     }
-    encode_row(q, valid, box, Al[0], s);
-    wg_sync(g);
-    // forward
-    for (int l = 0; l < 5 && ok; l++) {
-      if (s == 0) {
-        issue_fwd(tacc_col, Al[l], sm + kSmW + layer_img(l), layer_k(l));
-        tc::mma_commit(&bar_mma[g]);
-      }
-      ok = wg_and(g, tc::mbar_wait(&bar_mma[g], ph));
-      ph ^= 1;
-      tc::tc_fence_after();
-      if (!ok) break;
-      if (l < 4) {
-        epi_relu(t_acc, Al[l + 1], s);
-      } else {
-        float raw[48], dz[48];
-        load_raw(t_acc, raw);
-        if (valid && w > 0.0f) {
-          loss += mix_loss_grad(raw, wi, w, dz);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 48; k++) dz[k] = 0.0f;
-        }
-#pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 8) {
-          float f[8];
-#pragma unroll
-          for (int k = 0; k < 8; k++) f[k] = c0 + k < 48 ? dz[c0 + k] : 0.0f;
-          store_chunk(dZ, tc::core_off(s, c0, kOut), f);
-        }
-      }
-      wg_sync(g);
-    }
-    // backward: dZ holds dZ_{l+1}; dW_l += dZ^T A_l; dA_l = dZ W_l
-    for (int l = 4; l >= 0 && ok; l--) {
-      const int K = layer_k(l);
-      if (l == 0) {  // the input tile again, into the (now free) activation 3-4 region
-        encode_row(q, valid, box, Al[0], s);
-        wg_sync(g);
-      }
-      if (s == 0) {
-        const uint32_t w0 = tc::smem_u32(sm + kSmW + layer_img(l));
-        const uint32_t id_w = tc::idesc_bf16(64, (uint32_t)K, true, true);
-        const uint32_t id_a = tc::idesc_bf16(128, (uint32_t)K, false, true);
-        const uint32_t dz0 = tc::smem_u32(dZ), a0 = tc::smem_u32(Al[l]);
-        for (int s0 = 0; s0 < kTile; s0 += 16) {
-          uint64_t ad = tc::sdesc(dz0 + tc::core_off(s0, 0, kOut), (kOut >> 3) * 128u, 128u);
-          uint64_t bd = tc::sdesc(a0 + tc::core_off(s0, 0, K), (uint32_t)(K >> 3) * 128u, 128u);
-          tc::mma_bf16(t_dw[l], ad, bd, id_w, 1u);
-        }
-        if (l > 0) {
-          for (int n0 = 0; n0 < kOut; n0 += 16) {
-            uint64_t ad = tc::sdesc(dz0 + tc::core_off(0, n0, kOut), 128u, (kOut >> 3) * 128u);
-            uint64_t bd = tc::sdesc(w0 + tc::core_off(n0, 0, K), (uint32_t)(K >> 3) * 128u, 128u);
-            tc::mma_bf16(tacc_col, ad, bd, id_a, n0 > 0);
-          }
-        }
-        tc::mma_commit(&bar_mma[g]);
-      }
-      ok = wg_and(g, tc::mbar_wait(&bar_mma[g], ph));
-      ph ^= 1;
-      tc::tc_fence_after();
-      if (!ok) break;
-      if (l > 0) {
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 16) {
-          float v[16];
-          tc::tmem_ld16(t_acc + c0, v);
-          uint4 m0 = *reinterpret_cast<const uint4*>(Al[l] + tc::core_off(s, c0, kHid));
-          uint4 m1 = *reinterpret_cast<const uint4*>(Al[l] + tc::core_off(s, c0 + 8, kHid));
-          uint32_t mw[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-          float a[8], b[8];
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            a[2 * k] = bf16_lo(mw[k]) > 0.0f ? v[2 * k] : 0.0f;
-            a[2 * k + 1] = bf16_hi(mw[k]) > 0.0f ? v[2 * k + 1] : 0.0f;
-            b[2 * k] = bf16_lo(mw[4 + k]) > 0.0f ? v[8 + 2 * k] : 0.0f;
-            b[2 * k + 1] = bf16_hi(mw[4 + k]) > 0.0f ? v[8 + 2 * k + 1] : 0.0f;
-          }
-          store_chunk(dZ, tc::core_off(s, c0, kHid), a);
-          store_chunk(dZ, tc::core_off(s, c0 + 8, kHid), b);
-        }
-      }
-      wg_sync(g);
-    }
+    // half 0 encodes two coordinates, half 1 the third and the other features
+    encode_row(q, valid, box, T.act[0], T.s, T.h ? 2 : 0, T.h ? 3 : 2, T.h != 0);
+    tile_sync(T.t);
+    train_forward<0>(T);
+    train_forward<1>(T);
+    train_forward<2>(T);
+    train_forward<3>(T);
+    train_forward<4>(T);
+    loss += train_loss(T, lv, wi, w, valid && w > 0.0f);
+    tile_sync(T.t);
+    train_backward<4>(T, t_dw[4]);
+    train_backward<3>(T, t_dw[3]);
+    train_backward<2>(T, t_dw[2]);
+    train_backward<1>(T, t_dw[1]);
+    // the input tile again, into the (now free) activation 3-4 region
+    encode_row(q, valid, box, T.act[0], T.s, T.h ? 2 : 0, T.h ? 3 : 2, T.h != 0);
+    tile_sync(T.t);
+    train_backward<0>(T, t_dw[0]);
   }
   tc::tc_fence_before();
-  ok = __syncthreads_and(ok);
+  const bool ok = __syncthreads_and(T.ok);
   tc::tc_fence_after();
-  // flush the weight-gradient accumulators (warpgroup 0 reads them)
-  if (ok && g == 0) {
-    const int row = m64_row(s);
+  // flush the weight-gradient accumulators: 21 pieces of 16 columns over the warpgroups
+  if (ok) {
+    const int row = m64_row(T.s);
+    int piece = 0;
+#pragma unroll
     for (int l = 0; l < 5; l++) {
       const int K = layer_k(l);
-      for (int c0 = 0; c0 < K; c0 += 16) {
+      for (int c0 = 0; c0 < K; c0 += 16, piece++) {
+        if (piece % (kTrainThreads / 128) != warp >> 2) continue;
         float v[16];
         tc::tmem_ld16(t_dw[l] + lane_off + c0, v);
         if (row >= 0)
 #pragma unroll
-          for (int k = 0; k < 16; k++) atomicAdd(&grad[layer_w(l) + row * K + c0 + k], v[k]);
+          for (int k = 0; k < 16; k += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(&grad[layer_w(l) + row * K + c0 + k]),
+                         "f"(v[k]), "f"(v[k + 1]), "f"(v[k + 2]), "f"(v[k + 3])
+                         : "memory");
       }
     }
   }
@@ -968,7 +1018,7 @@ __global__ void __launch_bounds__(128 * kTrainTiles, 1)
   __syncthreads();
   if (tid == 0) {
     float t = 0.0f;
-    for (int k = 0; k < 4 * kTrainTiles; k++) t += red[k];
+    for (int k = 0; k < kTrainThreads / 32; k++) t += red[k];
     atomicAdd(N.scratch + 2, t);
   }
   if (warp == 0) tc::tmem_dealloc(T0, 512);
@@ -988,29 +1038,35 @@ __global__ void k_make_image(const float* w, unsigned char* img) {
 }
 
 // Adam (bias-corrected with the network's step count), then the BF16 image; clears the
-// gradient. blockIdx.y = network.
+// gradient, and the last block of a network counts the step and clears the step's sums (two
+// launches of a few threads each otherwise). blockIdx.y = network.
 __global__ void k_adam(const NetDev* nets, const uint32_t* pass, int step, float b1, float b2, float eps) {
   const NetDev& N = nets[blockIdx.y];
   if (!net_trains(N, pass, step)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
-  const float t = (float)(*N.step + 1u);
-  const float c1 = 1.0f / (1.0f - powf(b1, t)), c2 = 1.0f / (1.0f - powf(b2, t));
-  float gi = N.grad[i];
-  N.grad[i] = 0.0f;
-  float mi = b1 * N.m[i] + (1.0f - b1) * gi;
-  float vi = b2 * N.v[i] + (1.0f - b2) * gi * gi;
-  N.m[i] = mi;
-  N.v[i] = vi;
-  float wi = N.params[i] - N.lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  N.params[i] = wi;
-  image_store(const_cast<unsigned char*>(N.img), i, wi);
-}
-
-// Counts the Adam step of every training network (after k_adam read the old count).
-__global__ void k_net_step(const NetDev* nets, int nnet, const uint32_t* pass, int step) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nnet && net_trains(nets[j], pass, step)) *nets[j].step += 1u;
+  if (i < kParams) {
+    const float t = (float)(*N.step + 1u);
+    const float c1 = 1.0f / (1.0f - powf(b1, t)), c2 = 1.0f / (1.0f - powf(b2, t));
+    float gi = N.grad[i];
+    N.grad[i] = 0.0f;
+    float mi = b1 * N.m[i] + (1.0f - b1) * gi;
+    float vi = b2 * N.v[i] + (1.0f - b2) * gi * gi;
+    N.m[i] = mi;
+    N.v[i] = vi;
+    float wi = N.params[i] - N.lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    N.params[i] = wi;
+    image_store(const_cast<unsigned char*>(N.img), i, wi);
+  }
+  __syncthreads();  // the block has read the step count
+  if (threadIdx.x == 0) {
+    unsigned* ticket = reinterpret_cast<unsigned*>(N.scratch + 3);
+    __threadfence();
+    if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+      *N.step += 1u;
+      N.scratch[0] = N.scratch[1] = 0.0f;
+      *ticket = 0u;
+    }
+  }
 }
 
 }  // namespace rx
@@ -1079,7 +1135,7 @@ namespace rx {
 struct GuideState {
   rx_guide_options opt{};
   guide::Box box{};
-  // params, Adam moments, gradient, BF16 image; scratch {sum w, count, loss}; status;
+  // params, Adam moments, gradient, BF16 image; scratch {sum w, count, loss, ticket}; status;
   // step count; device copies of this network's NetDev and of the record segment the
   // single-network entry points train on
   DevBuf params, m, v, grad, img, scratch, status, step, dnet, dseg;
@@ -1151,14 +1207,11 @@ static int train_ctas_per_net(uint32_t batch, int nnet, int sms) {
 static cudaError_t train_nets_step(const NetDev* nets, const RecSeg* segs, int nnet, int per, int step,
                                    const uint32_t* pass, bool update, int sms, cudaStream_t s) {
   set_kernel_smem();
-  k_net_clear<<<(nnet + 127) / 128, 128, 0, s>>>(nets, nnet, pass, step);
   const int wper = std::max(1, std::min(4 * sms / nnet, 64));
   k_weight_sum<<<nnet * wper, 256, 0, s>>>(nets, segs, wper, step, pass);
-  k_guide_train<<<nnet * per, 128 * kTrainTiles, kSmTrain2, s>>>(nets, segs, per, step, pass);
-  if (update) {
-    k_adam<<<dim3((kParams + 255) / 256, nnet), 256, 0, s>>>(nets, pass, step, 0.9f, 0.999f, 1e-8f);
-    k_net_step<<<(nnet + 127) / 128, 128, 0, s>>>(nets, nnet, pass, step);
-  }
+  k_guide_train<<<nnet * per, kTrainThreads, kSmTrain2, s>>>(nets, segs, per, step, pass);
+  if (update) k_adam<<<dim3((kParams + 255) / 256, nnet), 256, 0, s>>>(nets, pass, step, 0.9f, 0.999f, 1e-8f);
+  else k_net_clear<<<(nnet + 127) / 128, 128, 0, s>>>(nets, nnet, pass, step);
   return cudaGetLastError();
 }
 
@@ -1253,6 +1306,7 @@ extern "C" rx_status rx_guide_init(rx_context* c, const rx_guide_options* opt, c
   cudaMemset(g->img.p, 0, rx::guide::kImgBytes);
   cudaMemset(g->status.p, 0, 16);
   cudaMemset(g->step.p, 0, 16);
+  cudaMemset(g->scratch.p, 0, 64);
   const rx::guide::NetDev view = rx::guide_net(g);
   cudaMemcpy(g->dnet.p, &view, sizeof view, cudaMemcpyHostToDevice);
   rx::k_make_image<<<(rx::guide::kParams + 255) / 256, 256, 0, c->stream>>>(g->params.as<float>(),

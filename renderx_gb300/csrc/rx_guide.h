@@ -75,7 +75,7 @@ __device__ __forceinline__ F3 mix_sample(const float* L, float u0, float u1, flo
 struct NetDev {
   const unsigned char* img;  // BF16 weight image (core-matrix layout)
   float *params, *m, *v, *grad;
-  float* scratch;            // {sum of record weights, record count, loss} of the current step
+  float* scratch;            // {sum of record weights, record count, loss} of the current step, a ticket
   int* status;               // set when a bounded tensor-core wait gave up
   uint32_t* step;            // Adam steps taken
   guide::Box box;            // position-encoding box

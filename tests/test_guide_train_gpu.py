@@ -1,0 +1,52 @@
+"""The training kernel at the edges of its tiles (128 records, two tiles a CTA), and the sums
+it keeps between steps: gradients and Adam steps in any order start from clear ones.
+
+The gradient is a mean over the records, so with equal weights the gradient of 2 m records is
+the mean of those of its halves. Halving the count doubles every back-propagated value
+exactly, BF16 roundings included, so the two differ by the order of FP32 sums alone (a record
+lost or counted twice moves them by about 1 / m)."""
+import numpy as np
+import pytest
+import torch
+
+import renderx_gb300 as rx
+from oracle import guide_mlp as gm
+
+pytestmark = pytest.mark.gpu
+BOX = ((0.0, 0.0, 0.0), (5.56, 5.56, 5.56))
+
+
+def _records(n, seed):
+    rng = np.random.default_rng(seed)
+    r = np.zeros((n, 16), np.float32)
+    r[:, 0:3] = rng.random((n, 3)) * 5.56
+    for k in (3, 6, 9):
+        v = rng.normal(size=(n, 3))
+        r[:, k:k + 3] = v / np.linalg.norm(v, axis=1, keepdims=True)
+    r[:, 12] = 1.0
+    return r
+
+
+@pytest.mark.parametrize("m", [1, 31, 63, 64, 65, 127, 128, 129, 257, 152 * 128 + 1])
+def test_gradient_of_two_halves(m):
+    recs = _records(2 * m, m)
+    rng = np.random.default_rng(2)
+    p = gm.init_params(9)
+    p = (p + rng.normal(scale=0.03, size=p.shape).astype(np.float32) * (p != 0)).astype(np.float32)
+    with rx.Context(0) as ctx:
+        ctx.guide_init(seed=9, box=BOX)
+        ctx.guide_set_params(p)
+        loss, g = ctx.guide_gradient(recs)
+        la, ga = ctx.guide_gradient(recs[:m])
+        lb, gb = ctx.guide_gradient(recs[m:])
+        stepped = ctx.guide_train_step(torch.from_numpy(recs).cuda(), 2 * m)
+        after = ctx.guide_params()
+        ctx.guide_set_params(p)
+        loss2, g2 = ctx.guide_gradient(recs)
+    scale = max(1.0, abs(loss))
+    assert np.linalg.norm(g) > 0
+    assert np.linalg.norm(g - 0.5 * (ga + gb)) <= 5e-5 * np.linalg.norm(g)
+    assert abs(loss - 0.5 * (la + lb)) <= 1e-5 * scale
+    assert np.linalg.norm(g2 - g) <= 5e-5 * np.linalg.norm(g)
+    assert abs(loss2 - loss) <= 1e-5 * scale and abs(stepped - loss) <= 1e-5 * scale
+    assert np.abs(after - p).max() <= 5.1e-3  # Adam's first step: at most its step size
