@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(128, 8) k_extend_p(const SceneRec* R, PathSoA 
                                                      unsigned long long* rays, unsigned long long* cursor) {
   const uint32_t n = *count, m = SHADOW ? *scount : 0u;
   ExtendLane<SHADOW> L{R, S, n, m, order, hit, Q, film, sq};
-  walk_persistent<4, kShortStack, 64>(L, cursor);
+  walk_persistent<4, kShortStack, 64>(L, cursor, kNoRay, walk_lanes(n + m));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     atomicAdd(rays, (unsigned long long)n);
     if (SHADOW && m) atomicAdd(rays + 1, (unsigned long long)m);

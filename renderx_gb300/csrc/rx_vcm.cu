@@ -1037,7 +1037,7 @@ struct ShadowLane {
 __global__ void __launch_bounds__(128, 8) k_shadow_wide(DevScene S, const ShadowQ* q, const unsigned* qn, float* img,
                                                         unsigned long long* cursor) {
   ShadowLane L{S, q, *qn, img};
-  walk_persistent<4, kShortStack, 64>(L, cursor);
+  walk_persistent<4, kShortStack, 64>(L, cursor, kNoRay, walk_lanes(L.n));
 }
 // The same, one thread per queued ray over the binary BVH (when the 4-wide tree is too
 // deep for the persistent walk's stack).

@@ -13,11 +13,11 @@
 // returning a limit below every entry distance.
 //
 // Traversal steps are warp-uniform: a lane without a leaf to test walks until it finds
-// one; meanwhile a lane that already holds one keeps walking inner nodes (its leaf
-// postponed, as in Aila and Laine's speculative traversal), so fewer lanes idle. A lane
-// stops when it reaches a second leaf. Pruning uses the limit before the postponed
-// leaf, which only visits more candidates, never fewer; leaves are tested in the order
-// they are reached, as a walk without postponing tests them.
+// one or its warp leaves the node loop (kWalkLeave); meanwhile a lane that already holds one
+// keeps walking inner nodes (its leaf postponed, as in Aila and Laine's speculative
+// traversal), so fewer lanes idle. A lane stops when it reaches a second leaf. Pruning uses
+// the limit before the postponed leaf, which only visits more candidates, never fewer;
+// leaves are tested in the order they are reached, as a walk without postponing tests them.
 //
 // kShort > 0: the first kShort entries of each thread's stack sit in shared memory (one
 // column per thread of a 128-thread block, conflict-free), deeper ones in local memory.
@@ -41,15 +41,35 @@ namespace rx {
 
 // kOnce: one ray per lane, `once` (kNoRay: none); no refills and no cursor.
 constexpr uint32_t kNoRay = 0xffffffffu;
+// A warp leaves the node loop for its leaves when at most kWalkLeave lanes still look for one
+// (and some lane waits with a leaf or a finished ray, so that every round makes progress),
+// and refills its idle lanes when there are kWalkRefill of them (or none works): with every
+// lane waited for and each idle lane refilled at once, 10 to 13 of 32 lanes were busy. Walk
+// of 2^24 rays over 4.1 M triangles 7.42 -> 6.4 ms (7.09, 6.88, 6.70, 6.69, 6.84 with 2, 4,
+// 8, 12, 16 lanes left behind and refills at once; 6.66, 6.62, 6.49, 6.39, 6.33 with 8 and
+// refills from 2, 4, 8, 12, 16 on), a 1024^2 x 16 frame over 1 M triangles 47.7 -> 43.3 ms,
+// the Cornell frame 0.868 -> 0.85 ms. A warp that walks one ray per lane has nothing to
+// refill and gains nothing by leaving early (100,003 rays over 25 K triangles 59.1 us, 62.5
+// with 4).
+constexpr int kWalkLeave = 6, kWalkRefill = 12;
+// Lanes of each warp that a launch of resident 128-thread blocks uses for n rays: as few as
+// let every ray start at once, since the lanes of a warp wait for one another. (A frame's
+// late bounces: 1024^2 x 16 over 1 M triangles 43.1 -> 41.6 ms, 128^2 x 4 over 77 K 1.34 ->
+// 1.08 ms; with half of the warps 41.9 and 1.11, a quarter 42.1 and 1.13.)
+__device__ __forceinline__ int walk_lanes(uint32_t n) {
+  const uint32_t warps = gridDim.x * 4;
+  return (int)min(32u, max(1u, (n + warps - 1) / warps));
+}
 template <int W, int kShort, int kStack, bool kOnce = false, class Lane>
-__device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cursor, uint32_t once = kNoRay) {
+__device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cursor, uint32_t once = kNoRay,
+                                                int lanes = 32) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int DONE = INT_MIN;
   constexpr int kShortN = kShort > 0 ? kShort : 1;
   __shared__ int s_ref[kShortN][128];
   __shared__ float s_tn[kShortN][128];
   const int lane = threadIdx.x & 31, tx = threadIdx.x;
-  bool active = false, exhausted = false;
+  bool active = false, exhausted = lane >= lanes;
   F3 o{}, d{}, inv{}, ood{};
   int near_bits = 0;  // bit k: the near plane of axis k is the upper bound
   int stack_ref[kStack - kShort];
@@ -68,7 +88,7 @@ __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cur
 
   while (true) {
     const unsigned want = __ballot_sync(FULL, !active && !exhausted);
-    if (want) {
+    if (want && (__popc(want) >= kWalkRefill || !__any_sync(FULL, active))) {
       const int leader = __ffs(want) - 1;
       unsigned long long base = 0;
       if (!kOnce && lane == leader) base = atomicAdd(cursor, (unsigned long long)__popc(want));
@@ -94,7 +114,10 @@ __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cur
     int pl = DONE;  // the next leaf to test (packed)
     while (true) {
       const bool need = active && pl == DONE && cur != DONE;
-      if (!__any_sync(FULL, need)) break;
+      // lanes to go on for, and lanes that wait with a leaf or a finished ray (leaving makes
+      // progress only when there are some)
+      const unsigned go = __ballot_sync(FULL, need), wait = kOnce ? 0u : __ballot_sync(FULL, active && !need);
+      if (go == 0 || (wait != 0 && __popc(go) <= kWalkLeave)) break;
       if (!(need || (active && cur >= 0))) continue;
       if (cur < 0) {  // a leaf (only lanes that need one get here)
         pl = cur;
