@@ -96,7 +96,8 @@ typedef struct rx_pt_options {
   uint32_t nee;            /* 0: PathTracer (BSDF sampling only); 1: PathTracerTest
                               (light sampling + balance-heuristic MIS) */
   uint64_t seed;
-  uint32_t paths_per_pass; /* wavefront size, 0 = 2^22 */
+  uint32_t paths_per_pass; /* wavefront size, 0 = 2^22 (rx_render_pt without guiding, time
+                              budget or snapshots: even passes of up to 2^24) */
   uint32_t flags;          /* RX_PT_GUIDED or 0 */
   float time_budget_s;     /* > 0: stop after the pass during which this much wall time
                               has passed (whole passes, spp the cap); paths run in
