@@ -119,12 +119,17 @@ struct DevBuf {
 // Device memory that a context's renders take their buffers from and that stays with the
 // context between calls: cudaMalloc and cudaFree of a render's buffers cost more than many
 // renders do (1.3 of 2.1 ms for a 256^2 x 16 frame, 9 of 65 ms for VCM at 512^2). A stack
-// of blocks: a Frame (one per render call) takes buffers from the top and gives all of them
-// back when it ends, so a call made from a snapshot callback nests. Buffers are used on the
+// of blocks: a Frame (one per render call) gives back when it ends what was taken since it
+// began, so a call made from a snapshot callback nests. Buffers are used on the
 // context's stream only, which orders one frame's work before the next one's. At most kKeep
 // bytes stay after the outermost frame; a context's memory goes with it. Not thread-safe, as
 // calls on one context are not.
 class Workspace {
+  struct Block {
+    void* p;
+    size_t size, used;
+  };
+
  public:
   static constexpr size_t kKeep = (size_t)8 << 30;
   Workspace() = default;
@@ -133,40 +138,41 @@ class Workspace {
   ~Workspace() { trim(0); }
   class Frame {
    public:
-    explicit Frame(Workspace& ws) : w(ws), top(ws.top_), used(ws.blocks_.empty() ? 0 : ws.blocks_[ws.top_].used) {
+    explicit Frame(Workspace& ws) : w(ws) {
+      for (const Block& b : w.blocks_) used.push_back(b.used);
       w.depth_++;
     }
     Frame(const Frame&) = delete;
     Frame& operator=(const Frame&) = delete;
-    ~Frame() {
-      for (size_t k = top + 1; k < w.blocks_.size(); k++) w.blocks_[k].used = 0;
-      if (!w.blocks_.empty()) w.blocks_[top].used = used;
-      w.top_ = top;
+    ~Frame() {  // what earlier frames hold stays
+      for (size_t k = 0; k < w.blocks_.size(); k++) w.blocks_[k].used = k < used.size() ? used[k] : 0;
       if (--w.depth_ == 0) w.trim(kKeep);
     }
 
    private:
     Workspace& w;
-    size_t top, used;
+    std::vector<size_t> used;
   };
-  // `bytes` of device memory, 256-byte aligned, until the innermost frame ends.
+  // `bytes` of device memory, 256-byte aligned, until the innermost frame ends: from the
+  // first block with room.
   cudaError_t alloc(size_t bytes, void** out) {
     bytes = (bytes + 255) & ~(size_t)255;
-    for (size_t k = top_; k < blocks_.size(); k++)
-      if (blocks_[k].size - blocks_[k].used >= bytes) return take(k, bytes, out);
     size_t all = 0;
-    for (const Block& b : blocks_) all += b.size;
+    for (Block& b : blocks_) {
+      if (b.size - b.used >= bytes) return take(b, bytes, out);
+      all += b.size;
+    }
     Block b{nullptr, std::max({bytes, std::min(all / 2, (size_t)512 << 20), (size_t)32 << 20}), 0};
     cudaError_t e = cudaMalloc(&b.p, b.size);
-    if (e == cudaErrorMemoryAllocation) {  // give back the unused blocks, take no more than asked
+    if (e == cudaErrorMemoryAllocation) {  // give back the unused blocks at the top, take no more than asked
       cudaGetLastError();
-      while (blocks_.size() > top_ + 1) pop();
+      while (!blocks_.empty() && blocks_.back().used == 0) pop();
       b.size = bytes;
       e = cudaMalloc(&b.p, b.size);
     }
     if (e != cudaSuccess) return e;
     blocks_.push_back(b);
-    return take(blocks_.size() - 1, bytes, out);
+    return take(blocks_.back(), bytes, out);
   }
   // Frees blocks from the top until at most `keep` bytes stay (no frame open).
   void trim(size_t keep) {
@@ -176,18 +182,12 @@ class Workspace {
       all -= blocks_.back().size;
       pop();
     }
-    top_ = 0;
   }
 
  private:
-  struct Block {
-    void* p;
-    size_t size, used;
-  };
-  cudaError_t take(size_t k, size_t bytes, void** out) {
-    *out = static_cast<char*>(blocks_[k].p) + blocks_[k].used;
-    blocks_[k].used += bytes;
-    top_ = k;
+  static cudaError_t take(Block& b, size_t bytes, void** out) {
+    *out = static_cast<char*>(b.p) + b.used;
+    b.used += bytes;
     return cudaSuccess;
   }
   void pop() {
@@ -195,7 +195,6 @@ class Workspace {
     blocks_.pop_back();
   }
   std::vector<Block> blocks_;
-  size_t top_ = 0;
   int depth_ = 0;
 };
 

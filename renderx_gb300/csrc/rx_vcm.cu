@@ -339,8 +339,12 @@ struct SubSink {
 // Light subpaths from emit_start (k_vcm_light's stream) or eye subpaths from
 // camera_start (k_vcm_eye_full's), each subpath's vertices in the store; `light`: the
 // isLightPath argument of the scattering. cursor: subpaths handed out (zero at launch).
-template <bool LIGHT>
-__global__ void __launch_bounds__(128) k_sub_run(DevScene S, VcmParams P, SubSink out, bool light_scatter,
+// kBlocks: 5 blocks per SM (96 registers), or 8 with spills where there are subpaths enough
+// to fill them: 2^20 light subpaths 2.88 ms against 3.34, but two iterations of 84 K subpaths
+// each way 3.11 ms against 2.91.
+constexpr uint32_t kSubManyPaths = 1u << 18;
+template <bool LIGHT, int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) k_sub_run(DevScene S, VcmParams P, SubSink out, bool light_scatter,
                                                  unsigned* cursor, unsigned long long* rays) {
   constexpr unsigned FULL = 0xffffffffu;
   const uint32_t n = LIGHT ? P.n_light : P.n_pixels;
@@ -1263,6 +1267,9 @@ __global__ void __launch_bounds__(128) k_merge_queries(DevScene S, VcmParams P, 
 
 // The eye side of a merge query, formed once per query in spatial order (k_merge_eye):
 // what a pair needs of the eye vertex E, its predecessor pe and E's record.
+// kEyeBehind: pe's direction leaves E's surface, so a pair on that side looks up its inside
+// object (find_inside); a vertex reached from the front never does.
+constexpr uint32_t kEyeRandom = 1u, kEyeBehind = 2u;
 struct alignas(16) EyeSide {
   F3 o;         // E's origin
   float oprob;
@@ -1275,13 +1282,13 @@ struct alignas(16) EyeSide {
   F3 thr;
   float prob;
   float pbr, sea;
-  uint32_t prand;  // pe sampled at random
+  uint32_t flags;  // kEyeRandom: pe sampled at random; kEyeBehind
   uint32_t pixel;
 };
 __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, const float4* ev, const MisE* emis,
-                                                   const uint32_t* qlist, const uint32_t* order, const unsigned* count,
+                                                   const uint32_t* qlist, const uint32_t* order, unsigned* count,
                                                    EyeSide* out) {
-  const uint32_t n = *count;
+  const uint32_t n = count[0];  // count[1]: queries with kEyeBehind
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const uint32_t q = __ldg(&qlist[__ldg(&order[j])]);  // vertex q % maxv >= 1 of pixel q / maxv
     const PV E = load_pv(ev + 4 * (size_t)q), pe = load_pv(ev + 4 * ((size_t)q - 1));
@@ -1299,8 +1306,9 @@ __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, cons
     e.prob = me.prob;
     e.pbr = me.pbr;
     e.sea = me.sea;
-    e.prand = rnd(pe) ? 1u : 0u;
+    e.flags = (rnd(pe) ? kEyeRandom : 0u) | (E.contact != kNone && !(dot(e.n, pe.d) <= 0.0f) ? kEyeBehind : 0u);
     e.pixel = q / P.maxv;
+    if (e.flags & kEyeBehind) atomicAdd(&count[1], 1u);
     out[j] = e;
   }
 }
@@ -1310,6 +1318,7 @@ __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, cons
 // does for a merge, then colour, probability and MIS weight from the records (join and
 // join_eval with merged set, on the parts formed per photon and per query; zero where the
 // reference drops the path). r: the merge radius.
+template <bool BEHIND>
 __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, const EyeSide& e, float r, float norm) {
   const float4 j0 = __ldg(jd), j1 = __ldg(jd + 1), j2 = __ldg(jd + 2), j5 = __ldg(jd + 5);
   const int lcontact = __float_as_int(j5.x), linside = __float_as_int(j5.y);
@@ -1322,8 +1331,7 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
   int einside = e.inside;
   if (!evol) {
     if (dot(e.n, ed) <= 0.0f) einside = e.contact;
-    else if (dot(e.n, e.pd) <= 0.0f) einside = e.pin;
-    else einside = find_inside(S, e.o, ed, e.contact);
+    else einside = BEHIND ? find_inside(S, e.o, ed, e.contact) : e.pin;
   }
   const int eobj = evol ? einside : e.contact;
   const bool lmed = is_vpm(S, linside), emed = is_vpm(S, einside);
@@ -1362,7 +1370,7 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
     sum += pb0 * (back * j2.w + j3.w);
   }
   const float pf1 = cosE * g * (rl ? dpf * opf : 1.0f);  // pf[ci+1] / pf[ci]
-  if (e.prand) sum += pf1 * e.pbr;
+  if (e.flags & kEyeRandom) sum += pf1 * e.pbr;
   sum += pf1 * merge_pdf(S, evol ? e.pin : e.contact, evol, e.n, ld, e.rd) * e.sea;
   const float wt = M / sum;
   return col * ((wt >= 0.0f ? wt : 0.0f) / prob) * (1.0f / norm);
@@ -1382,12 +1390,15 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
 // back, one counter that every walking warp waited on, the list's size read by the host
 // and the walk repeated when it had grown), and the evaluation formed both vertices'
 // normals and reversed directions per pair: 14.1 + 3.75 ms (7.5 when the walk repeated)
-// against 6.76 ms here, with 128 registers (bounds of 5 or 6 blocks per SM spill: 7.25,
-// 8.59 ms).
+// against 5.06 ms here. BEHIND: the queries whose pairs may look up an inside object, hardly
+// any; apart from them the kernel fits in 80 registers and six blocks per SM (7, 5 and 4
+// blocks: 5.64, 5.54 and 6.34 ms; with the look-up in the one kernel 6.76 at 128 registers).
 constexpr int kMergeList = 32 + 128;
-__global__ void __launch_bounds__(128) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
+template <bool BEHIND>
+__global__ void __launch_bounds__(128, 6) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
                                                const unsigned* count, float* img, unsigned long long* merges) {
   __shared__ uint2 s_list[4][kMergeList];
+  if (BEHIND && count[1] == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint2* list = s_list[warp];
   const unsigned lt = (1u << lane) - 1u;
@@ -1404,9 +1415,10 @@ __global__ void __launch_bounds__(128) k_merge(DevScene S, VcmParams P, Grid G, 
       acc = F3{0, 0, 0};
       cur = e.pixel;
     }
-    acc = acc + merge_pair(S, G.join + (size_t)kJoin * pair.x, e, r, P.norm);
+    acc = acc + merge_pair<BEHIND>(S, G.join + (size_t)kJoin * pair.x, e, r, P.norm);
   };
   for (uint32_t j = blockIdx.x * 4 + warp; j < nq; j += nw) {
+    if (((eye[j].flags & kEyeBehind) != 0) != BEHIND) continue;
     const F3 x = eye[j].o;
     // the cells the sphere touches (as merge_buckets), one per lane; equal buckets are
     // walked once, by the lowest lane that holds them
@@ -1857,7 +1869,9 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   P.norm = (float)P.n_light;
   const unsigned cap = P.bpt ? 1u : P.n_light * P.maxv;  // photon capacity (none without merging)
   unsigned buckets = 1u << 16;
-  while (buckets < cap && buckets < (1u << 26)) buckets <<= 1;
+  // a bucket per two photons and more (about two a path are stored); one for each that could
+  // be stored costs 0.4 ms of scans an iteration at 2^20 paths
+  while (buckets < std::min<uint64_t>(cap, 4ull * P.n_light) && buckets < (1u << 26)) buckets <<= 1;
   Workspace::Frame frame(c->ws);
   std::vector<WsBuf> bufs(33);
   cudaError_t e;
@@ -1907,14 +1921,15 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   int grid = c->trace_cfg.sms * 4;
   // shadow rays on the persistent 4-wide walk when the tree fits its stack
   const bool wide_shadow = c->d_bvh4.p && 3 * c->bvh4.max_depth + 1 <= 64;
-  int sub_grid[2] = {0, 0}, merge_grid = 0, rec_grid[2] = {0, 0};  // resident blocks: k_sub_run<false>, <true>; k_merge; k_records
+  auto sub_light = P.n_light >= kSubManyPaths ? k_sub_run<true, 8> : k_sub_run<true, 5>;
+  int sub_grid[2] = {0, 0}, merge_grid = 0, rec_grid[2] = {0, 0};  // resident blocks: k_sub_run (eye, light); k_merge; k_records
   {
     int per = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<false>, 128, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<false, 5>, 128, 0)) != cudaSuccess) return e;
     sub_grid[0] = c->trace_cfg.sms * std::max(per, 1);
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sub_run<true>, 128, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sub_light, 128, 0)) != cudaSuccess) return e;
     sub_grid[1] = c->trace_cfg.sms * std::max(per, 1);
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_merge, 128, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_merge<false>, 128, 0)) != cudaSuccess) return e;
     merge_grid = c->trace_cfg.sms * std::max(per, 1);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_records<false>, 128, 0)) != cudaSuccess) return e;
     rec_grid[0] = c->trace_cfg.sms * std::max(per, 1);
@@ -1949,8 +1964,8 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       unsigned* cursor = bufs[26].as<unsigned>() + (light_side ? 0 : 1);
       unsigned long long* rc = ctr + (light_side ? 0 : 1);
       const bool light_scatter = light_side || !P.bpt;  // VCM samples eye paths with light-path scattering
-      if (light_side) k_sub_run<true><<<sub_grid[1], 128, 0, s>>>(S, P, out, light_scatter, cursor, rc);
-      else k_sub_run<false><<<sub_grid[0], 128, 0, s>>>(S, P, out, light_scatter, cursor, rc);
+      if (light_side) sub_light<<<sub_grid[1], 128, 0, s>>>(S, P, out, light_scatter, cursor, rc);
+      else k_sub_run<false, 5><<<sub_grid[0], 128, 0, s>>>(S, P, out, light_scatter, cursor, rc);
     };
     if (full_mis)
       k_vcm_light<<<grid * 4, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[2].as<float4>(),
@@ -2049,14 +2064,15 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       uint32_t* qorder = bufs[29].as<uint32_t>();
       uint32_t* qhist = bufs[30].as<uint32_t>();
       unsigned* qcount = bufs[31].as<unsigned>();
-      cudaMemsetAsync(qcount, 0, sizeof(unsigned), s);
+      cudaMemsetAsync(qcount, 0, 2 * sizeof(unsigned), s);
       cudaMemsetAsync(qhist, 0, (size_t)kRayBins * sizeof(uint32_t), s);
       k_merge_queries<<<grid, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[13].as<int>(), qlist, qkey, qhist, qcount);
       scan_bins(qhist, qhist + kRayBins, s);
       k_ray_scatter<<<grid * 2, 256, 0, s>>>(qkey, 0, qcount, qhist, qorder);
       k_merge_eye<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), qlist, qorder, qcount,
                                            bufs[24].as<EyeSide>());
-      k_merge<<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
+      k_merge<false><<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
+      k_merge<true><<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
       k_count_photons<<<1, 1, 0, s>>>(qcount, nq, ctr + 5);
       if (m1) {  // device time of this iteration's merge gather (walk + pair evaluation)
         cudaEventRecord(m1, s);
