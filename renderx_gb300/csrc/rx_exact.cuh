@@ -139,19 +139,24 @@ __device__ __forceinline__ int box_clear_pass(F3 mn, F3 mx, F3 o, F3 d, F3 inv, 
   const float nx = fminf(t0x, t1x), ny = fminf(t0y, t1y), nz = fminf(t0z, t1z);
   const float fx = fmaxf(t0x, t1x), fy = fmaxf(t0y, t1y), fz = fmaxf(t0z, t1z);
   const float te = max3f(nx, ny, nz), tx = min3f(fx, fy, fz);  // entry and exit faces
-#pragma unroll
-  for (int f = 0; f < 2; f++) {
-    const float t = f == 0 ? te : tx;
-    if (!(t >= 0.0f)) continue;
-    // the face's axis (any axis that attains t: each is a face the ray meets at t), then
-    // the point on it inside the other two slabs with the margin, all three axes at once
-    const int a = f == 0 ? (nx == t ? 0 : (ny == t ? 1 : 2)) : (fx == t ? 0 : (fy == t ? 1 : 2));
+  // the face at distance t whose axis is the first of (sx, sy, sz) that attains it (any axis
+  // that does: each is a face the ray meets at t): its point inside the other two slabs with
+  // the margin, all three axes at once
+  auto inside = [&](float t, float sx, float sy) {
     const float px = o.x + t * d.x, py = o.y + t * d.y, pz = o.z + t * d.z;
     const float dx = fmaf(t, m.md.x, m.mo.x), dy = fmaf(t, m.md.y, m.mo.y), dz = fmaf(t, m.md.z, m.mo.z);
     const bool inx = (px >= mn.x + dx) && (px <= mx.x - dx), iny = (py >= mn.y + dy) && (py <= mx.y - dy);
     const bool inz = (pz >= mn.z + dz) && (pz <= mx.z - dz);
-    if ((inx || a == 0) && (iny || a == 1) && (inz || a == 2)) return 1;
-  }
+    const bool ax = sx == t, ay = !ax && sy == t, az = !ax && !ay;
+    return (inx || ax) && (iny || ay) && (inz || az);
+  };
+  // the entry face, or for an origin inside the box the exit face: one evaluation for the
+  // lanes of both kinds (2^24 checks of 13 boxes 1.34 ms against 1.52 with a face after the
+  // other); the exit face of a box entered near its rim is tried apart
+  const bool in_front = te >= 0.0f;
+  const float t = in_front ? te : tx;
+  if (t >= 0.0f && inside(t, in_front ? nx : fx, in_front ? ny : fy)) return 1;
+  if (in_front && tx >= 0.0f && inside(tx, fx, fy)) return 1;
   return 0;
 }
 
