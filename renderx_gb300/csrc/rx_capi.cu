@@ -81,6 +81,7 @@ void rx_destroy(rx_context* c) {
     c->guide = nullptr;
     c->ws.trim(0);
     if (c->stream) cudaStreamDestroy(c->stream);
+    if (c->side_stream) cudaStreamDestroy(c->side_stream);
     for (auto s : c->copy_stream)
       if (s) cudaStreamDestroy(s);
   }

@@ -227,6 +227,38 @@ struct Event {
   operator cudaEvent_t() const { return e; }
 };
 
+// A render's second stream: `begin` lets it start after the work queued on `s` so far, `join`
+// makes `s` wait for what it holds. The render's buffers are used on it, so however the
+// render ends it waits for the side stream before they are given back.
+struct SideStream {
+  cudaStream_t side = nullptr;
+  Event ev[2];
+  bool busy = false;
+  SideStream() = default;
+  SideStream(const SideStream&) = delete;
+  SideStream& operator=(const SideStream&) = delete;
+  ~SideStream() {
+    if (busy) cudaStreamSynchronize(side);
+  }
+  cudaError_t open(cudaStream_t& kept) {
+    cudaError_t e = kept ? cudaSuccess : cudaStreamCreateWithFlags(&kept, cudaStreamNonBlocking);
+    side = kept;
+    for (Event& v : ev)
+      if (e == cudaSuccess) e = v.create(cudaEventDisableTiming);
+    return e;
+  }
+  cudaError_t begin(cudaStream_t s) {
+    cudaError_t e = cudaEventRecord(ev[0], s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side, ev[0], 0);
+    busy = true;
+    return e;
+  }
+  cudaError_t join(cudaStream_t s) {
+    cudaError_t e = cudaEventRecord(ev[1], side);
+    return e == cudaSuccess ? cudaStreamWaitEvent(s, ev[1], 0) : e;
+  }
+};
+
 // A captured CUDA graph and its executable, destroyed with their owner.
 struct Graph {
   cudaGraph_t g = nullptr;
@@ -245,6 +277,7 @@ struct Graph {
 struct rx_context {
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side_stream = nullptr;  // work of a render beside its stream's (made when first used)
   cudaStream_t copy_stream[2] = {nullptr, nullptr};
   std::string err;
 

@@ -1936,6 +1936,8 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_records<true>, 128, 0)) != cudaSuccess) return e;
     rec_grid[1] = c->trace_cfg.sms * std::max(per, 1);
   }
+  SideStream side;
+  if ((e = side.open(c->side_stream)) != cudaSuccess) return e;
   Event e0, e1, m0, m1;  // render; merge gather of an iteration (with stats)
   if ((e = e0.create()) != cudaSuccess || (e = e1.create()) != cudaSuccess) return e;
   if (stats && ((e = m0.create()) != cudaSuccess || (e = m1.create()) != cudaSuccess)) return e;
@@ -1956,7 +1958,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     cudaMemsetAsync(bufs[26].p, 0, bufs[26].bytes, s);  // subpath cursors
     // the subpaths on persistent warps (the whole-path check mode keeps one thread per
     // subpath): one launch per side, as many blocks as stay resident
-    auto subpaths = [&](bool light_side) {
+    auto subpaths = [&](bool light_side, cudaStream_t s) {
       const SubSink out = light_side ? SubSink{bufs[0].as<float4>(), bufs[1].as<int>(), !P.bpt, bufs[2].as<float4>(),
                                                bufs[3].as<int>(), nph, cap}
                                      : SubSink{bufs[12].as<float4>(), bufs[13].as<int>(), false, nullptr, nullptr,
@@ -1970,8 +1972,12 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     if (full_mis)
       k_vcm_light<<<grid * 4, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[2].as<float4>(),
                                        bufs[3].as<int>(), nph, cap, ctr);
-    else
-      subpaths(true);
+    else {
+      // the eye subpaths beside the light subpaths: neither fills the GPU to its end
+      if ((e = side.begin(s)) != cudaSuccess) return e;
+      subpaths(false, side.side);
+      subpaths(true, s);
+    }
     k_records<false><<<rec_grid[0], 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[19].as<MisL>(),
                                                  nullptr, bufs[25].as<uint32_t>(), nullptr, nullptr, nullptr);
     const float cell = 2.0f * radius;
@@ -2016,7 +2022,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       k_vcm_eye_full<<<grid, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[12].as<float4>(),
                                           bufs[13].as<int>(), bufs[10].as<float>(), ctr + 1);
     } else {
-      subpaths(false);
+      if ((e = side.join(s)) != cudaSuccess) return e;
       k_records<true><<<rec_grid[1], 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[13].as<int>(), nullptr,
                                                   bufs[20].as<MisE>(), bufs[25].as<uint32_t>(), bufs[21].as<uint2>(), qc,
                                                   bufs[10].as<float>());
