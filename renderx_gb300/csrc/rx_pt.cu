@@ -138,15 +138,7 @@ __device__ __forceinline__ int scene_at(const uint32_t* off, int nr, uint32_t i)
   return lo;
 }
 
-// The counts a bounce reads, adds to and clears for the next one (a kernel of its own that
-// cleared them cost 3 us a bounce: 25 of the 860 us of a 512x512x1 frame).
-struct Counts {
-  unsigned *count, *next, *clear;  // queue lengths: this bounce's, the next one's, the one after
-  unsigned *vis, *vis_done;        // visibility rays: this bounce's, the last one's
-  unsigned long long* cursor;      // of the persistent extension walk
-};
-
-__global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, PathSoA S, Counts C) {
+__global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, PathSoA S, unsigned* count) {
   uint32_t np;
   const bool inter = ps->interleaved != 0;
   if (inter) {
@@ -190,9 +182,7 @@ __global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, P
     S.id[i] = pid | ((uint64_t)i << kLocalShift);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *C.count = np;
-    *C.next = *C.vis = *C.vis_done = 0;  // C.clear is the first bounce's to clear
-    *C.cursor = 0ull;
+    *count = np;
     ps->npaths = np;
   }
 }
@@ -540,16 +530,13 @@ template <bool MEDIA>
 constexpr int kShadeThreads = MEDIA ? 512 : 256;
 template <bool NEE, bool GUIDE, bool MEDIA>
 __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MEDIA>) k_shade(const SceneRec* R, const PassState* ps, PathSoA S,
-                                               Counts C, const int2* hit, PathSoA N, double* film_sum,
-                                               double* film_sq, ShadowSoA Q, GuideIO G, bool sort) {
+                                               const unsigned* count, const int2* hit, PathSoA N, unsigned* next_count,
+                                               double* film_sum, double* film_sq, ShadowSoA Q, unsigned* scount,
+                                               GuideIO G, bool sort) {
   constexpr int kWarps = kShadeThreads<MEDIA> / 32;
   __shared__ uint32_t s_count[kWarps][4];
   __shared__ unsigned short s_perm[32 * kWarps];
-  uint32_t n = *C.count;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {  // nothing reads these during this kernel
-    *C.clear = *C.vis_done = 0;
-    *C.cursor = 0ull;
-  }
+  uint32_t n = *count;
   uint32_t stride = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   // every lane of a warp walks the same number of iterations (ballots need all 32)
@@ -678,7 +665,7 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
     if (m) {
       unsigned base = 0;
       int leader = __ffs(m) - 1;
-      if (lane == leader) base = atomicAdd(C.next, (unsigned)__popc(m));
+      if (lane == leader) base = atomicAdd(next_count, (unsigned)__popc(m));
       base = __shfl_sync(0xffffffffu, base, leader);
       if (cont) {
         uint32_t j = base + __popc(m & ((1u << lane) - 1));
@@ -697,7 +684,7 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
       if (sm) {
         unsigned base = 0;
         const int leader = __ffs(sm) - 1;
-        if (lane == leader) base = atomicAdd(C.vis, (unsigned)__popc(sm));
+        if (lane == leader) base = atomicAdd(scount, (unsigned)__popc(sm));
         base = __shfl_sync(0xffffffffu, base, leader);
         if (pend) {
           const uint32_t j = base + __popc(sm & ((1u << lane) - 1));
@@ -715,6 +702,11 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
 // The next queue's length, the extension walk's refill cursor for the next bounce
 // (kWalk4P: every k_extend_p launch of a pass is followed by this one, so the cursor is
 // zero when the next starts) and the number of visibility rays.
+__global__ void k_zero(unsigned* p, unsigned long long* cursor, unsigned* scount) {
+  *p = 0;
+  *cursor = 0ull;
+  *scount = 0;
+}
 __global__ void k_advance(PassState* ps) {
   ps->base += ps->per_pass;
   ps->pass += 1;
@@ -922,7 +914,7 @@ PtParams make_pt_params(const rx_context* c, const rx_camera& cam, const rx_pt_o
 namespace {
 
 // W.ctr slot of the persistent extension walk's refill cursor (slots 0 and 1 count rays,
-// 8 onwards hold the unsigned counts).
+// 8 onwards hold the unsigned queue counts).
 constexpr int kExtendCursor = 40;
 
 // Device buffers of one wavefront render.
@@ -934,7 +926,7 @@ struct Wave {
   int2* hit;
   ShadowSoA Q;              // visibility rays of a bounce (null without next-event estimation)
   unsigned long long* ctr;  // [0] extension rays, [1] shadow rays
-  unsigned* cnt;            // [0..2] queue lengths, [3] raw training records, [4..5] visibility rays
+  unsigned* cnt;            // [0], [1] queue lengths, [2] raw training records, [3] visibility rays
   double *film, *sq;
   uint32_t loops;           // bounce stages per pass (max depth cap + 1)
   uint32_t *keys, *order, *hist;  // ray binning of bounce rays (null: off)
@@ -960,13 +952,6 @@ struct Wave {
   uint32_t* seg;
   int* rows;
 };
-
-// Bounce d's counts. Queue lengths rotate through three slots and visibility rays through
-// two, so that the shading kernel of a bounce clears what the next one adds to.
-Counts bounce_counts(const Wave& W, uint32_t d) {
-  return {W.cnt + d % 3, W.cnt + (d + 1) % 3, W.cnt + (d + 2) % 3, W.cnt + 4 + (d & 1), W.cnt + 4 + (~d & 1),
-          W.ctr + kExtendCursor};
-}
 
 // Bins the queue's rays (bounces after the camera rays) and returns the visiting order.
 const uint32_t* enqueue_binning(const Wave& W, PathSoA cur, const unsigned* cc, int grid, cudaStream_t s) {
@@ -998,44 +983,50 @@ auto shade_kernel(bool nee, bool guide, bool media) {
   return nee ? k_shade<true, false, false> : k_shade<false, false, false>;
 }
 
-// One pass: (layout), generate, `loops` x (extend, guiding inference, shade), (training),
-// advance the cursor. Everything is a kernel on `s` with
+// One pass: (layout), generate, `loops` x (extend, guiding inference, clear the next
+// queue, shade), (training), advance the cursor. Everything is a kernel on `s` with
 // device-resident counts and schedule, so the pass can be captured into a CUDA graph
 // once and replayed.
 template <int STACK>
 cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   if (W.L.off) k_layout<<<1, 256, 0, s>>>(W.R, W.nr, W.L);
-  if (W.recs) k_records_begin<<<1, 256, 0, s>>>(W.nets, W.nnet, W.ps, W.cnt + 3, W.net_count);
-  k_generate<<<grid, 256, 0, s>>>(W.R, W.nr, W.ps, W.L, W.A, bounce_counts(W, 0));
-  const GuideIO G{W.nets, W.lobes, W.recs, W.cnt + 3, W.rec_cap, W.lpath};
+  if (W.recs) k_records_begin<<<1, 256, 0, s>>>(W.nets, W.nnet, W.ps, W.cnt + 2, W.net_count);
+  k_generate<<<grid, 256, 0, s>>>(W.R, W.nr, W.ps, W.L, W.A, W.cnt);
+  const GuideIO G{W.nets, W.lobes, W.recs, W.cnt + 2, W.rec_cap, W.lpath};
   const bool nee = W.Q.o != nullptr;
+  unsigned* scnt = W.cnt + 3;
   const bool media = W.media || W.nets;
   auto shade = shade_kernel(nee, W.nets != nullptr, media);
   const int threads = media ? kShadeThreads<true> : kShadeThreads<false>;
   PathSoA cur = W.A, nxt = W.B;
+  unsigned *cc = W.cnt, *cn = W.cnt + 1;
   // the extension rays of a queue, and the visibility rays of the bounce before
-  auto extend = [&](const PathSoA& q, const Counts& C, const uint32_t* order) {
+  auto extend = [&](const PathSoA& q, const unsigned* count, const uint32_t* order) {
     if constexpr (STACK == kWalk4P) {  // persistent: the blocks that stay resident (8 per SM)
       auto k = nee ? k_extend_p<true> : k_extend_p<false>;
-      k<<<W.sms * 8, 128, 0, s>>>(W.R, q, C.count, order, W.hit, W.Q, C.vis_done, W.film, W.sq, W.ctr, C.cursor);
+      k<<<W.sms * 8, 128, 0, s>>>(W.R, q, count, order, W.hit, W.Q, scnt, W.film, W.sq, W.ctr, W.ctr + kExtendCursor);
     } else {
-      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, C.count, order, W.hit, W.ctr);
-      if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, C.vis_done, W.film, W.sq, W.ctr);
+      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, count, order, W.hit, W.ctr);
+      if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, scnt, W.film, W.sq, W.ctr);
     }
   };
   for (uint32_t d = 0; d < W.loops; d++) {
-    const Counts C = bounce_counts(W, d);
-    const uint32_t* order = d > 0 ? enqueue_binning(W, cur, C.count, grid, s) : nullptr;
-    extend(cur, C, order);
-    if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, C.count, grid, s);
-    shade<<<grid * 128 / threads, threads, 0, s>>>(W.R, W.ps, cur, C, W.hit, nxt, W.film, W.sq, W.Q, G, W.sort);
+    const uint32_t* order = d > 0 ? enqueue_binning(W, cur, cc, grid, s) : nullptr;
+    extend(cur, cc, order);
+    if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, cc, grid, s);
+    k_zero<<<1, 1, 0, s>>>(cn, W.ctr + kExtendCursor, scnt);
+    shade<<<grid * 128 / threads, threads, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.Q, scnt, G,
+                                                   W.sort);
     std::swap(cur, nxt);
+    std::swap(cc, cn);
   }
-  // no path goes on; the last vertices' visibility rays
-  if (nee) extend(cur, bounce_counts(W, W.loops), nullptr);
+  if (nee) {  // no path goes on; the last vertices' visibility rays
+    extend(cur, cc, nullptr);
+    k_zero<<<1, 1, 0, s>>>(cc, W.ctr + kExtendCursor, scnt);
+  }
   if (W.recs) {
-    k_record_weights<<<grid, 128, 0, s>>>(W.R, W.nr, W.L.off, W.ps, W.nets, W.nnet, W.recs, W.cnt + 3, W.rec_cap,
+    k_record_weights<<<grid, 128, 0, s>>>(W.R, W.nr, W.L.off, W.ps, W.nets, W.nnet, W.recs, W.cnt + 2, W.rec_cap,
                                           W.lpath, W.train, W.net_count, W.rbase, W.rcap);
     if (e == cudaSuccess) e = guide_train_nets(W.nets, W.segs, W.nnet, W.steps, W.batch_max, &W.ps->pass, W.sms, s);
   }
