@@ -138,7 +138,21 @@ __device__ __forceinline__ int scene_at(const uint32_t* off, int nr, uint32_t i)
   return lo;
 }
 
-__global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, PathSoA S, unsigned* count) {
+// The counts of a bounce. The extension kernel reads the first three and clears the others
+// for the kernels behind it (a kernel of its own that cleared them took 3 us of every
+// bounce: 25 of the 870 us of a 512x512x1 frame).
+struct Counts {
+  unsigned *count, *vis_done;      // queue length; visibility rays of the bounce before
+  unsigned long long* cursor;      // of the persistent extension walk
+  unsigned *next, *vis;            // next queue's length; visibility rays of this bounce
+  unsigned long long* cursor_next;
+  __device__ void clear() const {
+    *next = *vis = 0;
+    *cursor_next = 0ull;
+  }
+};
+
+__global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, PathSoA S, Counts C) {
   uint32_t np;
   const bool inter = ps->interleaved != 0;
   if (inter) {
@@ -182,7 +196,9 @@ __global__ void k_generate(const SceneRec* R, int nr, PassState* ps, Layout L, P
     S.id[i] = pid | ((uint64_t)i << kLocalShift);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *count = np;
+    *C.count = np;
+    *C.vis_done = 0;
+    *C.cursor = 0ull;
     ps->npaths = np;
   }
 }
@@ -297,14 +313,14 @@ struct ExtendLane {
 // instead of each thread walking its share of the queue to the end. SHADOW: and the
 // visibility rays of the bounce before. rays[0], rays[1] count both.
 template <bool SHADOW>
-__global__ void __launch_bounds__(128, 8) k_extend_p(const SceneRec* R, PathSoA S, const unsigned* count,
+__global__ void __launch_bounds__(128, 8) k_extend_p(const SceneRec* R, PathSoA S, Counts C,
                                                      const uint32_t* __restrict__ order, int2* hit, ShadowSoA Q,
-                                                     const unsigned* scount, double* film, double* sq,
-                                                     unsigned long long* rays, unsigned long long* cursor) {
-  const uint32_t n = *count, m = SHADOW ? *scount : 0u;
+                                                     double* film, double* sq, unsigned long long* rays) {
+  const uint32_t n = *C.count, m = SHADOW ? *C.vis_done : 0u;
   ExtendLane<SHADOW> L{R, S, n, m, order, hit, Q, film, sq};
-  walk_persistent<4, kShortStack, 64>(L, cursor, kNoRay, walk_lanes(n + m));
+  walk_persistent<4, kShortStack, 64>(L, C.cursor, kNoRay, walk_lanes(n + m));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    C.clear();
     atomicAdd(rays, (unsigned long long)n);
     if (SHADOW && m) atomicAdd(rays + 1, (unsigned long long)m);
   }
@@ -336,10 +352,10 @@ __global__ void k_path_keys(const SceneRec* R, PathSoA S, const unsigned* count,
 // Closest legal hit of each live path's ray; `order` (optional) visits the paths in
 // binned order.
 template <int STACK>
-__global__ void __launch_bounds__(128) k_extend(const SceneRec* R, PathSoA S, const unsigned* count,
+__global__ void __launch_bounds__(128) k_extend(const SceneRec* R, PathSoA S, Counts C,
                                                 const uint32_t* __restrict__ order, int2* hit,
                                                 unsigned long long* rays) {
-  uint32_t n = *count;
+  uint32_t n = *C.count;
   uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
     uint32_t i = order ? __ldg(&order[j]) : j;
@@ -350,7 +366,10 @@ __global__ void __launch_bounds__(128) k_extend(const SceneRec* R, PathSoA S, co
     PHit h = trace_walk<false, STACK>(SC, f3(o), f3(d), INFINITY, camera ? kNone : inf.y, camera ? kNone : inf.z);
     hit[i] = make_int2(h.tid, __float_as_int(h.t));
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(rays, (unsigned long long)n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    C.clear();
+    atomicAdd(rays, (unsigned long long)n);
+  }
 }
 
 // PathTracerTest::colorByConnectingLights (src/PathTracerTest.cpp:88-136) at vertex `v`
@@ -702,11 +721,6 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
 // The next queue's length, the extension walk's refill cursor for the next bounce
 // (kWalk4P: every k_extend_p launch of a pass is followed by this one, so the cursor is
 // zero when the next starts) and the number of visibility rays.
-__global__ void k_zero(unsigned* p, unsigned long long* cursor, unsigned* scount) {
-  *p = 0;
-  *cursor = 0ull;
-  *scount = 0;
-}
 __global__ void k_advance(PassState* ps) {
   ps->base += ps->per_pass;
   ps->pass += 1;
@@ -913,9 +927,9 @@ PtParams make_pt_params(const rx_context* c, const rx_camera& cam, const rx_pt_o
 
 namespace {
 
-// W.ctr slot of the persistent extension walk's refill cursor (slots 0 and 1 count rays,
-// 8 onwards hold the unsigned queue counts).
-constexpr int kExtendCursor = 40;
+// W.ctr slots of the persistent extension walk's refill cursors (slots 0 and 1 count rays,
+// 8 onwards hold the unsigned counts).
+constexpr int kExtendCursor = 40;  // and 41, by turns
 
 // Device buffers of one wavefront render.
 struct Wave {
@@ -926,7 +940,7 @@ struct Wave {
   int2* hit;
   ShadowSoA Q;              // visibility rays of a bounce (null without next-event estimation)
   unsigned long long* ctr;  // [0] extension rays, [1] shadow rays
-  unsigned* cnt;            // [0], [1] queue lengths, [2] raw training records, [3] visibility rays
+  unsigned* cnt;            // [0], [1] queue lengths, [2] raw training records, [4], [5] visibility rays
   double *film, *sq;
   uint32_t loops;           // bounce stages per pass (max depth cap + 1)
   uint32_t *keys, *order, *hist;  // ray binning of bounce rays (null: off)
@@ -952,6 +966,12 @@ struct Wave {
   uint32_t* seg;
   int* rows;
 };
+
+// Bounce d's counts: two slots each by turns, those of a bounce's end cleared at its start.
+Counts bounce_counts(const Wave& W, uint32_t d) {
+  const uint32_t a = d & 1, b = 1 - a;
+  return {W.cnt + a, W.cnt + 4 + b, W.ctr + kExtendCursor + a, W.cnt + b, W.cnt + 4 + a, W.ctr + kExtendCursor + b};
+}
 
 // Bins the queue's rays (bounces after the camera rays) and returns the visiting order.
 const uint32_t* enqueue_binning(const Wave& W, PathSoA cur, const unsigned* cc, int grid, cudaStream_t s) {
@@ -983,8 +1003,8 @@ auto shade_kernel(bool nee, bool guide, bool media) {
   return nee ? k_shade<true, false, false> : k_shade<false, false, false>;
 }
 
-// One pass: (layout), generate, `loops` x (extend, guiding inference, clear the next
-// queue, shade), (training), advance the cursor. Everything is a kernel on `s` with
+// One pass: (layout), generate, `loops` x (extend, guiding inference, shade), (training),
+// advance the cursor. Everything is a kernel on `s` with
 // device-resident counts and schedule, so the pass can be captured into a CUDA graph
 // once and replayed.
 template <int STACK>
@@ -992,39 +1012,34 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   if (W.L.off) k_layout<<<1, 256, 0, s>>>(W.R, W.nr, W.L);
   if (W.recs) k_records_begin<<<1, 256, 0, s>>>(W.nets, W.nnet, W.ps, W.cnt + 2, W.net_count);
-  k_generate<<<grid, 256, 0, s>>>(W.R, W.nr, W.ps, W.L, W.A, W.cnt);
+  k_generate<<<grid, 256, 0, s>>>(W.R, W.nr, W.ps, W.L, W.A, bounce_counts(W, 0));
   const GuideIO G{W.nets, W.lobes, W.recs, W.cnt + 2, W.rec_cap, W.lpath};
   const bool nee = W.Q.o != nullptr;
-  unsigned* scnt = W.cnt + 3;
   const bool media = W.media || W.nets;
   auto shade = shade_kernel(nee, W.nets != nullptr, media);
   const int threads = media ? kShadeThreads<true> : kShadeThreads<false>;
   PathSoA cur = W.A, nxt = W.B;
-  unsigned *cc = W.cnt, *cn = W.cnt + 1;
   // the extension rays of a queue, and the visibility rays of the bounce before
-  auto extend = [&](const PathSoA& q, const unsigned* count, const uint32_t* order) {
+  auto extend = [&](const PathSoA& q, const Counts& C, const uint32_t* order) {
     if constexpr (STACK == kWalk4P) {  // persistent: the blocks that stay resident (8 per SM)
       auto k = nee ? k_extend_p<true> : k_extend_p<false>;
-      k<<<W.sms * 8, 128, 0, s>>>(W.R, q, count, order, W.hit, W.Q, scnt, W.film, W.sq, W.ctr, W.ctr + kExtendCursor);
+      k<<<W.sms * 8, 128, 0, s>>>(W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
     } else {
-      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, count, order, W.hit, W.ctr);
-      if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, scnt, W.film, W.sq, W.ctr);
+      k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, C, order, W.hit, W.ctr);
+      if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, C.vis_done, W.film, W.sq, W.ctr);
     }
   };
   for (uint32_t d = 0; d < W.loops; d++) {
-    const uint32_t* order = d > 0 ? enqueue_binning(W, cur, cc, grid, s) : nullptr;
-    extend(cur, cc, order);
-    if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, cc, grid, s);
-    k_zero<<<1, 1, 0, s>>>(cn, W.ctr + kExtendCursor, scnt);
-    shade<<<grid * 128 / threads, threads, 0, s>>>(W.R, W.ps, cur, cc, W.hit, nxt, cn, W.film, W.sq, W.Q, scnt, G,
-                                                   W.sort);
+    const Counts C = bounce_counts(W, d);
+    const uint32_t* order = d > 0 ? enqueue_binning(W, cur, C.count, grid, s) : nullptr;
+    extend(cur, C, order);
+    if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, C.count, grid, s);
+    shade<<<grid * 128 / threads, threads, 0, s>>>(W.R, W.ps, cur, C.count, W.hit, nxt, C.next, W.film, W.sq, W.Q,
+                                                   C.vis, G, W.sort);
     std::swap(cur, nxt);
-    std::swap(cc, cn);
   }
-  if (nee) {  // no path goes on; the last vertices' visibility rays
-    extend(cur, cc, nullptr);
-    k_zero<<<1, 1, 0, s>>>(cc, W.ctr + kExtendCursor, scnt);
-  }
+  // no path goes on; the last vertices' visibility rays
+  if (nee) extend(cur, bounce_counts(W, W.loops), nullptr);
   if (W.recs) {
     k_record_weights<<<grid, 128, 0, s>>>(W.R, W.nr, W.L.off, W.ps, W.nets, W.nnet, W.recs, W.cnt + 2, W.rec_cap,
                                           W.lpath, W.train, W.net_count, W.rbase, W.rcap);
