@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(128 * kInferTiles, 1)
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar_mma[kInferTiles], bar_w;
   __shared__ uint32_t tmem_base;
+  cudaGridDependencySynchronize();
   // the warp's number made uniform, so that what the issuing lane needs stays in uniform registers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), g = warp >> 2, s = tid & 127;
   uint32_t n, ntiles;  // queries (GROUPED: rows), tiles
@@ -654,6 +655,7 @@ __global__ void k_net_clear(const NetDev* nets, int nnet, const uint32_t* pass, 
 // Sum of record weights and number of records per network (the loss normalisation);
 // blocks [j * per, (j + 1) * per) serve network j.
 __global__ void k_weight_sum(const NetDev* nets, const RecSeg* segs, int per, int step, const uint32_t* pass) {
+  cudaGridDependencySynchronize();
   const int j = blockIdx.x / per;
   if (!net_trains(nets[j], pass, step)) return;
   const RecSeg R = segs[j];
@@ -905,6 +907,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   __shared__ __align__(8) uint64_t bar_mma[kTrainTiles], bar_w;
   __shared__ uint32_t tmem_base;
   __shared__ float red[kTrainThreads / 32];
+  cudaGridDependencySynchronize();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int j = blockIdx.x / per, part = blockIdx.x % per;
   const NetDev& N = nets[j];
@@ -1041,6 +1044,7 @@ __global__ void k_make_image(const float* w, unsigned char* img) {
 // gradient, and the last block of a network counts the step and clears the step's sums (two
 // launches of a few threads each otherwise). blockIdx.y = network.
 __global__ void k_adam(const NetDev* nets, const uint32_t* pass, int step, float b1, float b2, float eps) {
+  cudaGridDependencySynchronize();
   const NetDev& N = nets[blockIdx.y];
   if (!net_trains(N, pass, step)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1190,8 +1194,8 @@ cudaError_t guide_infer_wave(const NetDev* nets, int nnet, const DevScene* scene
   if (rows)
     k_guide_infer<PathIO, true><<<sms, 128 * kInferTiles, kSmInfer, s>>>(io, nullptr, 0, nets, nnet, rows, seg, pass);
   else
-    k_guide_infer<PathIO, false><<<sms, 128 * kInferTiles, kSmInfer, s>>>(io, count, 0, nets, 1, nullptr, nullptr,
-                                                                           pass);
+    launch_early(k_guide_infer<PathIO, false>, sms, 128 * kInferTiles, kSmInfer, s, io, count, 0, nets, 1, nullptr,
+                 nullptr, pass);
   return cudaGetLastError();
 }
 
@@ -1208,9 +1212,9 @@ static cudaError_t train_nets_step(const NetDev* nets, const RecSeg* segs, int n
                                    const uint32_t* pass, bool update, int sms, cudaStream_t s) {
   set_kernel_smem();
   const int wper = std::max(1, std::min(4 * sms / nnet, 64));
-  k_weight_sum<<<nnet * wper, 256, 0, s>>>(nets, segs, wper, step, pass);
-  k_guide_train<<<nnet * per, kTrainThreads, kSmTrain2, s>>>(nets, segs, per, step, pass);
-  if (update) k_adam<<<dim3((kParams + 255) / 256, nnet), 256, 0, s>>>(nets, pass, step, 0.9f, 0.999f, 1e-8f);
+  launch_early(k_weight_sum, nnet * wper, 256, 0, s, nets, segs, wper, step, pass);
+  launch_early(k_guide_train, nnet * per, kTrainThreads, kSmTrain2, s, nets, segs, per, step, pass);
+  if (update) launch_early(k_adam, dim3((kParams + 255) / 256, nnet), 256, 0, s, nets, pass, step, 0.9f, 0.999f, 1e-8f);
   else k_net_clear<<<(nnet + 127) / 128, 128, 0, s>>>(nets, nnet, pass, step);
   return cudaGetLastError();
 }

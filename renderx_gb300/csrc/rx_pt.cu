@@ -1005,27 +1005,6 @@ auto shade_kernel(bool nee, bool guide, bool media) {
   return nee ? k_shade<true, false, false> : k_shade<false, false, false>;
 }
 
-// Launches `k` so that its blocks come up while the kernel before it drains (`k` waits for
-// that one's results in cudaGridDependencySynchronize, its first statement; behind
-// anything but a kernel it just follows). Between an extension and a shading kernel 2-3 us
-// of launch and drain are hidden: 512x512x1 845 -> 800 us, a batch of 16 scenes 5.33 ->
-// 5.26 ms, a guided frame 4.45 -> 4.39. Letting the next kernel's blocks in before a block's end was slower on large
-// frames (35.4 against 35.0 ms): they take the places that the running kernel's own blocks
-// leave one by one.
-template <class... P, class... A>
-void launch_early(void (*k)(P...), int grid, int threads, cudaStream_t s, A... a) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
-}
-
 // One pass: (layout), generate, `loops` x (extend, guiding inference, shade), (training),
 // advance the cursor. Everything is a kernel on `s` with
 // device-resident counts and schedule, so the pass can be captured into a CUDA graph
@@ -1046,7 +1025,7 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   auto extend = [&](const PathSoA& q, const Counts& C, const uint32_t* order) {
     if constexpr (STACK == kWalk4P) {  // persistent: the blocks that stay resident (8 per SM)
       auto k = nee ? k_extend_p<true> : k_extend_p<false>;
-      launch_early(k, W.sms * 8, 128, s, W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
+      launch_early(k, W.sms * 8, 128, 0, s, W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
     } else {
       k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, C, order, W.hit, W.ctr);
       if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, C.vis_done, W.film, W.sq, W.ctr);
@@ -1057,7 +1036,7 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
     const uint32_t* order = d > 0 ? enqueue_binning(W, cur, C.count, grid, s) : nullptr;
     extend(cur, C, order);
     if (W.nets && e == cudaSuccess) e = enqueue_infer(W, cur, C.count, grid, s);
-    launch_early(shade, grid * 128 / threads, threads, s, W.R, W.ps, cur, C.count, W.hit, nxt, C.next, W.film, W.sq, W.Q,
+    launch_early(shade, grid * 128 / threads, threads, 0, s, W.R, W.ps, cur, C.count, W.hit, nxt, C.next, W.film, W.sq, W.Q,
                  C.vis, G, W.sort);
     std::swap(cur, nxt);
   }

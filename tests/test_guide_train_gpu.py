@@ -50,3 +50,37 @@ def test_gradient_of_two_halves(m):
     assert np.linalg.norm(g2 - g) <= 5e-5 * np.linalg.norm(g)
     assert abs(loss2 - loss) <= 1e-5 * scale and abs(stepped - loss) <= 1e-5 * scale
     assert np.abs(after - p).max() <= 5.1e-3  # Adam's first step: at most its step size
+
+
+@pytest.mark.parametrize("n", [128, 5000])
+def test_captured_steps(n):
+    """Steps in a replayed CUDA graph do what steps launched one by one do: the same loss after
+    twelve. Float atomics move single weights of undecided gradient sign by up to a step, which
+    the loss does not see to first order (5e-3 of it allowed)."""
+    recs = _records(n, n)
+    dev = torch.from_numpy(recs).cuda()
+    p = gm.init_params(9)
+    with rx.Context(0) as ctx:
+        ctx.guide_init(seed=9, box=BOX)
+        losses = []
+        for captured in (False, True):
+            s = torch.cuda.Stream()
+            # not captured: the batch's descriptor goes to the device with its first step
+            ctx.guide_train_step(dev, n, stream=s.cuda_stream)
+            ctx.guide_set_params(p)
+            torch.cuda.synchronize()
+            if captured:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=s):
+                    for _ in range(4):
+                        ctx.guide_train_step(dev, n, stream=s.cuda_stream, want_loss=False)
+                for _ in range(3):
+                    graph.replay()
+            else:
+                for _ in range(12):
+                    ctx.guide_train_step(dev, n, stream=s.cuda_stream, want_loss=False)
+            torch.cuda.synchronize()
+            moved = np.abs(ctx.guide_params() - p)
+            assert moved.max() > 0.02  # a weight whose gradient keeps its sign: 12 steps of 5e-3
+            losses.append(ctx.guide_gradient(recs)[0])
+    assert abs(losses[1] - losses[0]) <= 5e-3 * max(1.0, abs(losses[0]))
