@@ -279,9 +279,9 @@ struct Graph {
 // a load of the read-only path need not stay behind the wait. Between an extension and a
 // shading kernel 2-3 us of launch and drain are hidden: 512x512x1 845 -> 800 us, a batch of
 // 16 scenes 5.33 -> 5.26 ms, a guided frame 4.45 -> 4.33; a training step of 2^12 records
-// 28.8 -> 22.7 us, of 2^18 96.4 -> 90.3. Letting the next kernel's blocks
-// in before a block's end was slower on large frames (35.4 against 35.0 ms): they take the
-// places that the running kernel's own blocks leave one by one.
+// 28.8 -> 22.7 us, of 2^18 96.4 -> 90.3. Letting the next kernel's blocks in before a
+// block's end was slower on large frames (35.4 against 35.0 ms): they take the places that
+// the running kernel's own blocks leave one by one.
 template <class... P, class... A>
 void launch_early(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... a) {
   cudaLaunchAttribute at{};

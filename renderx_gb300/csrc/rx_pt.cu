@@ -314,7 +314,7 @@ struct ExtendLane {
 // visibility rays of the bounce before. rays[0], rays[1] count both.
 template <bool SHADOW>
 __global__ void __launch_bounds__(128, 8) k_extend_p(const SceneRec* R, PathSoA S, Counts C,
-                                                     const uint32_t* __restrict__ order, int2* hit, ShadowSoA Q,
+                                                     const uint32_t* order, int2* hit, ShadowSoA Q,
                                                      double* film, double* sq, unsigned long long* rays) {
   cudaGridDependencySynchronize();
   const uint32_t n = *C.count, m = SHADOW ? *C.vis_done : 0u;
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
         Hit3 hh{(int)__ldg(&SC.tri_obj[h.x]), h.x, __int_as_float(h.y)};
         bool russian = P.rr_mode == 0 || depth >= 3;
         bool guided = net >= 0 && G.lobes && !P.nee && ps->pass >= G.nets[net].warmup &&
-                      __ldg(&G.lobes[(size_t)i * guide::kLobeStride]) >= 0.0f;
+                      G.lobes[(size_t)i * guide::kLobeStride] >= 0.0f;
         if (guided) {
           nx = scatter_guided(SC, cur, hh, russian, rng, G.lobes + (size_t)i * guide::kLobeStride,
                               G.nets[net].frac);
@@ -1025,7 +1025,10 @@ cudaError_t enqueue_pass(const Wave& W, int grid, cudaStream_t s) {
   auto extend = [&](const PathSoA& q, const Counts& C, const uint32_t* order) {
     if constexpr (STACK == kWalk4P) {  // persistent: the blocks that stay resident (8 per SM)
       auto k = nee ? k_extend_p<true> : k_extend_p<false>;
-      launch_early(k, W.sms * 8, 128, 0, s, W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
+      if (order)  // the kernel before wrote it; read through the read-only path
+        k<<<W.sms * 8, 128, 0, s>>>(W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
+      else
+        launch_early(k, W.sms * 8, 128, 0, s, W.R, q, C, order, W.hit, W.Q, W.film, W.sq, W.ctr);
     } else {
       k_extend<STACK><<<grid, 128, 0, s>>>(W.R, q, C, order, W.hit, W.ctr);
       if (nee) k_shadow<STACK><<<grid, 128, 0, s>>>(W.R, q, W.Q, C.vis_done, W.film, W.sq, W.ctr);
