@@ -444,7 +444,7 @@ def section_vcm(peak, iters: int = 32, res: int = 512, light_paths: int = 1 << 2
             "photons_per_iteration": st["photons"] // iters, "merge_gather_ms_per_iteration": st["merge_ms"] / iters,
             "roofline": None if gbs is None else {
                 "bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
-                "kernel": "k_merge_walk + k_merge_eval (merge gather)",
+                "kernel": "k_merge_eye + k_merge (merge gather)",
                 "algorithmic_bytes_per_iteration": alg // iters},
             "cpu_baseline": vcm_cpu_reference(),
             "image_mean": [float(x) for x in img.mean(axis=(0, 1))]}

@@ -411,8 +411,8 @@ rx_status rx_trace_set_staging(rx_context* ctx, uint32_t chunk_rays);
 rx_status rx_trace_set_binning(rx_context* ctx, int32_t cell_bits, int32_t dir_bits, int32_t dir_map);
 /* Per-kernel device timing of rx_trace_closest_device calls: the next max_calls calls
  * record CUDA events around their three kernels (walk, reference-visibility check,
- * re-walk of rejected winners); 0 turns timing off. No reference counterpart
- * (measurement). */
+ * re-walk of rejected winners); a batch small enough for the one-launch walk reports that
+ * launch as its walk. 0 turns timing off. No reference counterpart (measurement). */
 rx_status rx_trace_set_timing(rx_context* ctx, int32_t max_calls);
 /* ms3[3*i + j]: device milliseconds of kernel j in recorded call i (waits for the
  * events); *calls = number of recorded calls. ms3 may be NULL to query the count. */

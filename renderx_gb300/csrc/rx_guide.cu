@@ -696,8 +696,9 @@ __global__ void k_weight_sum(const NetDev* nets, const RecSeg* segs, int per, in
 //
 // Latency-bound (ten dependent MMA -> tensor-memory load -> store steps a tile, two tiles
 // an SM): one warpgroup per tile, descriptors formed per MMA by the issuing thread, two
-// barriers a layer and scalar atomics in the flush made a step 201 us at 2^18 records and 80 at 2^12;
-// now 97 and 29 us (104 and 37 before k_adam took the two bookkeeping launches).
+// barriers a layer and scalar atomics in the flush made a step 201 us at 2^18 records and 80 at
+// 2^12; now 90 and 23 us (104 and 37 before k_adam took the two bookkeeping launches, 97 and
+// 29 before the step's kernels were launched early).
 constexpr int kTrainTiles = 2;
 constexpr int kTrainThreads = 256 * kTrainTiles;
 constexpr uint32_t kTrainTileBytes = 5 * kActBytes;  // A1, A2, A3|A4 (A0 alias), dZ

@@ -121,9 +121,9 @@ struct DevBuf {
 // renders do (1.3 of 2.1 ms for a 256^2 x 16 frame, 9 of 65 ms for VCM at 512^2). A stack
 // of blocks: a Frame (one per render call) gives back when it ends what was taken since it
 // began, so a call made from a snapshot callback nests. Buffers are used on the
-// context's stream only, which orders one frame's work before the next one's. At most kKeep
-// bytes stay after the outermost frame; a context's memory goes with it. Not thread-safe, as
-// calls on one context are not.
+// context's stream (and on a side stream that the render waits for), which orders one frame's
+// work before the next one's. At most kKeep bytes stay after the outermost frame; a context's
+// memory goes with it. Not thread-safe, as calls on one context are not.
 class Workspace {
   struct Block {
     void* p;

@@ -124,8 +124,8 @@ __device__ __forceinline__ F3 decay_of(const DevScene& S, int inside, float dist
 
 // One side of findInsideObject: whether the ray from o along d meets object `obj` (its
 // nearest triangle below tmax, no condition: the reference's per-object tree) at a positive
-// distance and leaves it there. (Out of line it cost k_merge_eval 14.2 -> 20.3 ms: the
-// registers saved around the call.)
+// distance and leaves it there. (Out of line it cost VCM's pair evaluation 14.2 -> 20.3
+// ms: the registers saved around the call.)
 static __device__ __forceinline__ bool leaves_object(const float4* __restrict__ bvh, const float4* __restrict__ tris,
                                                   const float4* __restrict__ slot_n, const float4* __restrict__ tri_v,
                                                   const float4* __restrict__ tri_n, const DevObject* objects, int obj,

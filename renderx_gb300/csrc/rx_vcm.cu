@@ -12,10 +12,11 @@
 //     per-iteration PointKDTree (include/PointKDTree.h), queried with the same strict
 //     |p-x| < r test over the (up to) 8 cells the sphere touches.
 //  3. Per pixel, the eye subpath (the same kernel, with light-path scattering, as
-//     VCMTracer.cpp:107 does), then colorByMergingPaths (:566-636) and
-//     colorByConnectingPaths (:430-562) with the full-path MIS of connectMergeWeight
-//     (:321-428, double precision) and light-tracing splats through
-//     Camera::transToPixel.
+//     VCMTracer.cpp:107 does, on a second stream beside the light subpaths), then the
+//     MIS records of both sides' vertices (k_records), colorByConnectingPaths (:430-562,
+//     k_conn_eval and its queued shadow rays) and colorByMergingPaths (:566-636, k_merge)
+//     with the full-path MIS of connectMergeWeight (:321-428) formed from the records,
+//     and light-tracing splats through Camera::transToPixel.
 //  4. Vignetting correction of the iteration image and the running mean (FP64 film).
 //
 // The same pipeline without photons and merging is the reference's
@@ -1973,7 +1974,10 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       k_vcm_light<<<grid * 4, 128, 0, s>>>(S, P, bufs[0].as<float4>(), bufs[1].as<int>(), bufs[2].as<float4>(),
                                        bufs[3].as<int>(), nph, cap, ctr);
     else {
-      // the eye subpaths beside the light subpaths: neither fills the GPU to its end
+      // the eye subpaths beside the light subpaths: neither fills the GPU to its end (BPT
+      // at 333x251 x 2 2.91 -> 2.73 ms, VCM at 200x150 with 2^15 light paths 2.61 -> 2.13;
+      // at 512^2 with 2^20 the same either way). All subpaths at 64 registers, or on smaller
+      // grids side by side, gained nothing on top (BPT 2.94, 3.07).
       if ((e = side.begin(s)) != cudaSuccess) return e;
       subpaths(false, side.side);
       subpaths(true, s);
