@@ -1,5 +1,8 @@
 // The C ABI (include/renderx.h): context, scene upload, accelerator build and the
 // closest-hit entry points.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -19,11 +22,22 @@ rx_status upload(rx_context* c, DevBuf& b, const void* src, size_t bytes, const 
   return c->cuda(cudaMemcpy(b.p, src, bytes, cudaMemcpyHostToDevice), what);
 }
 
+// Faults in a film's pages ahead of the copy to it (their bytes stay): a copy that meets pages
+// of the heap which have never been written takes 1 GB/s (a new film of 1024^2 now and then 22
+// ms instead of 1.7). Where the kernel does not know the request, the copy faults them in.
+void populate(void* out, size_t bytes) {
+  constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, which older C libraries do not name
+  const uintptr_t at = reinterpret_cast<uintptr_t>(out), lo = at & ~((uintptr_t)sysconf(_SC_PAGESIZE) - 1);
+  madvise(reinterpret_cast<void*>(lo), at + bytes - lo, kPopulateWrite);
+}
+
 // The mean of a device film of sums (`n` samples over all pixels) to the caller's buffer.
 rx_status mean_to_host(rx_context* c, double* film, size_t pixels, uint64_t n, double* out) {
   rx_status s = c->cuda(rx::film_mean(film, pixels, n, c->stream), "film mean");
   if (s != RX_OK) return s;
-  s = c->cuda(cudaMemcpyAsync(out, film, pixels * 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "film copy");
+  const size_t bytes = pixels * 3 * sizeof(double);
+  populate(out, bytes);
+  s = c->cuda(cudaMemcpyAsync(out, film, bytes, cudaMemcpyDeviceToHost, c->stream), "film copy");
   return s != RX_OK ? s : c->cuda(cudaStreamSynchronize(c->stream), "film copy");
 }
 
@@ -494,6 +508,7 @@ rx_status rx_render_pt_batch(rx_context* c, const rx_batch_item* items, uint32_t
     }
     for (uint32_t k = 0; k < n; k++) {
       const size_t bytes = (size_t)items[k].camera.width * items[k].camera.height * 3 * sizeof(double);
+      populate(items[k].film_rgb, bytes);
       if ((s = c->cuda(cudaMemcpyAsync(items[k].film_rgb, film.as<double>() + jobs[k].film_base * 3, bytes,
                                        cudaMemcpyDeviceToHost, c->stream),
                        "film copy")) != RX_OK)
