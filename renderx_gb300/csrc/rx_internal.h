@@ -277,7 +277,7 @@ struct Graph {
 // that one's results in cudaGridDependencySynchronize, its first statement; behind
 // anything but a kernel it just follows). `k` reads what that kernel wrote by plain loads:
 // a load of the read-only path need not stay behind the wait. Between an extension and a
-// shading kernel 2-3 us of launch and drain are hidden: 512x512x1 845 -> 800 us, a batch of
+// shading kernel 2-3 us of launch and drain are hidden: 256x256x16 845 -> 800 us, a batch of
 // 16 scenes 5.33 -> 5.26 ms, a guided frame 4.45 -> 4.33; a training step of 2^12 records
 // 28.8 -> 22.7 us, of 2^18 96.4 -> 90.3. Letting the next kernel's blocks in before a
 // block's end was slower on large frames (35.4 against 35.0 ms): they take the places that

@@ -140,7 +140,7 @@ __device__ __forceinline__ int scene_at(const uint32_t* off, int nr, uint32_t i)
 
 // The counts of a bounce. The extension kernel reads the first three and clears the others
 // for the kernels behind it (a kernel of its own that cleared them took 3 us of every
-// bounce: 25 of the 870 us of a 512x512x1 frame).
+// bounce: 25 of the 870 us of a 256x256x16 frame).
 struct Counts {
   unsigned *count, *vis_done;      // queue length; visibility rays of the bounce before
   unsigned long long* cursor;      // of the persistent extension walk
