@@ -43,23 +43,36 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Waits for the phase with parity `phase` to complete, at most `limit` tries, each of which
-// the hardware suspends for a while (a poll that returns at once takes issue slots from the
-// epilogues beside it: 2^20 inference queries 91.9 us against 89.8).
-// Returns false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint32_t limit = 1u << 22) {
-  uint32_t a = smem_u32(bar);
-  for (uint32_t it = 0; it < limit; it++) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(a), "r"(phase)
-        : "memory");
-    if (done) return true;
-  }
+// Nanoseconds of the GPU's clock, for limits on waits.
+__device__ __forceinline__ uint64_t now_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t phase) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(phase)
+      : "memory");
+  return done != 0;
+}
+// Waits for the phase with parity `phase` to complete; false when `limit_ns` have passed
+// first. A try that fails is one that the hardware suspended for a time of its own choosing
+// (a poll that returns at once takes issue slots from the epilogues beside it: 2^20
+// inference queries 91.9 us against 89.8), so a number of tries bounds no time and the
+// clock does.
+constexpr uint64_t kWaitNs = 1000000000ull;
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint64_t limit_ns = kWaitNs) {
+  const uint32_t a = smem_u32(bar);
+  if (mbar_try(a, phase)) return true;
+  const uint64_t t0 = now_ns();
+  do {
+    if (mbar_try(a, phase)) return true;
+  } while (now_ns() - t0 < limit_ns);
   return false;
 }
 
