@@ -436,8 +436,8 @@ rx_status rx_guide_set_params(rx_context* ctx, const float* params);
  * network outputs; pdf (n, optional) = the mixture density of each record's incident
  * direction. */
 rx_status rx_guide_eval(rx_context* ctx, const float* recs, uint32_t n, float* raw40, float* pdf);
-/* The same on device buffers (16-byte aligned records), enqueued on `stream` (NULL: the
- * context's stream); d_raw40 / d_pdf may each be NULL. */
+/* The same on device buffers, enqueued on `stream` (NULL: the context's stream); d_recs and
+ * d_raw40 must be 16-byte aligned; d_raw40 / d_pdf may each be NULL. */
 rx_status rx_guide_eval_device(rx_context* ctx, const float* d_recs, uint32_t n, float* d_raw40, float* d_pdf,
                                void* stream);
 /* Gradient (training kernel, no update) of the batch loss

@@ -1394,6 +1394,7 @@ extern "C" rx_status rx_guide_eval_device(rx_context* c, const float* d_recs, ui
   if (n == 0) return RX_OK;
   if (!d_recs || (!d_raw40 && !d_pdf)) return c->fail(RX_ERR_INVALID, "null buffer");
   if (reinterpret_cast<uintptr_t>(d_recs) % 16) return c->fail(RX_ERR_INVALID, "records must be 16-byte aligned");
+  if (reinterpret_cast<uintptr_t>(d_raw40) % 16) return c->fail(RX_ERR_INVALID, "raw outputs must be 16-byte aligned");
   DeviceGuard dg(c->device);
   rx::GuideState* g = c->guide;
   rx::set_kernel_smem();
