@@ -1377,8 +1377,7 @@ extern "C" rx_status rx_guide_eval(rx_context* c, const float* recs, uint32_t n,
   cudaMemcpy(dr.p, recs, (size_t)n * rx::guide::kRec * 4, cudaMemcpyHostToDevice);
   rx::set_kernel_smem();
   rx::RecordIO io{dr.as<float>(), draw.as<float>(), dp.as<float>()};
-  uint32_t grid = std::min<uint32_t>((n + rx::guide::kTile - 1) / rx::guide::kTile, (uint32_t)g->sms);
-  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::guide::kInferTiles, rx::kSmInfer, c->stream>>>(
+  rx::k_guide_infer<rx::RecordIO, false><<<rx::guide::infer_ctas(n, g->sms), 128 * rx::guide::kInferTiles, rx::kSmInfer, c->stream>>>(
       io, nullptr, n, g->dnet.as<rx::guide::NetDev>(), 1, nullptr, nullptr, nullptr);
   if ((s = c->cuda(cudaStreamSynchronize(c->stream), "guide eval")) != RX_OK) return s;
   if ((s = guide_status(c)) != RX_OK) return s;
@@ -1399,9 +1398,8 @@ extern "C" rx_status rx_guide_eval_device(rx_context* c, const float* d_recs, ui
   rx::GuideState* g = c->guide;
   rx::set_kernel_smem();
   rx::RecordIO io{d_recs, d_raw40, d_pdf};
-  uint32_t grid = std::min<uint32_t>((n + rx::guide::kGroupRows - 1) / rx::guide::kGroupRows, (uint32_t)g->sms);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
-  rx::k_guide_infer<rx::RecordIO, false><<<grid, 128 * rx::guide::kInferTiles, rx::kSmInfer, st>>>(
+  rx::k_guide_infer<rx::RecordIO, false><<<rx::guide::infer_ctas(n, g->sms), 128 * rx::guide::kInferTiles, rx::kSmInfer, st>>>(
       io, nullptr, n, g->dnet.as<rx::guide::NetDev>(), 1, nullptr, nullptr, nullptr);
   return c->cuda(cudaGetLastError(), "guide eval");
 }

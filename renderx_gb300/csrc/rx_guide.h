@@ -1,6 +1,7 @@
 // Path-guiding network: sizes, parameter layout, the mixture of von Mises-Fisher lobes
 // the network outputs, and the host-side state a context keeps for it.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -99,6 +100,12 @@ struct RecSeg {
 // kGroupRows (one inference CTA's tiles), so a CTA's tiles share one network.
 constexpr int kInferTiles = 8;  // inference tiles in flight per CTA, one warpgroup each
 constexpr uint32_t kGroupRows = kInferTiles * kTile;
+// CTAs of an ungrouped inference over n rows: one per tile until every SM has one, since a
+// CTA's tiles are dealt out over the grid (20,000 rows 16.4 us in CTAs of eight tiles, on 20
+// of 152 SMs; 10.2 us in one of a tile or two each).
+inline uint32_t infer_ctas(uint32_t n, int sms) {
+  return (uint32_t)std::min<uint64_t>(((uint64_t)n + kTile - 1) / kTile, (uint64_t)sms);
+}
 
 }  // namespace guide
 
