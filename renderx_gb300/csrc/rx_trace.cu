@@ -113,21 +113,33 @@ struct HitLane {
   }
 };
 
-template <int W, int kShort, int kStack>
+// Whether a warp of the 4-wide walk goes on in the node loop until each of its lanes has a
+// leaf (no early leaving, kWalkLeave): lanes that get hardly more than one ray each have
+// nothing to be refilled with, so leaving early pays there only in deep trees, whose walks
+// are long and unequal; in the smallest trees it never does. A batch in us, waiting / leaving:
+//             36 triangles (2 levels)   25 K (9)      256 K (11)      4.1 M (14)
+//   156,000   38.4 / 41.4               78.4 / 85.8   113.6 / 114.6   256.9 / 248.5
+//   240,000   45.5 / 48.2               91.8 / 93.8   141.7 / 136.8
+//   258,000   47.4 / 49.6               94.7 / 96.3   148.1 / 142.7
+static bool walk_waits(uint32_t depth, uint32_t n, uint64_t lanes) {
+  return depth <= (n > lanes + lanes / 8 ? 4 : 10);
+}
+
+template <int W, int kShort, int kStack, int kLeave>
 __device__ __forceinline__ void walk_wide(const DevAccel& A, const float4* __restrict__ nodes,
                                           const rx_ray* __restrict__ rays, uint32_t n,
                                           const uint32_t* __restrict__ order, int32_t* __restrict__ out_tid,
                                           float* __restrict__ out_dist, uint32_t* __restrict__ hit_leaf,
                                           int4* __restrict__ slot_rec, unsigned long long* __restrict__ counters) {
   HitLane L{A, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, nodes};
-  walk_persistent<W, kShort, kStack>(L, counters + 4);
+  walk_persistent<W, kShort, kStack, false, kLeave>(L, counters + 4);
 }
 
 // 4-wide walk: 128-byte nodes; at most 3 stack entries per level of a tree shallower
 // than 22 levels. At most 64 registers, so that eight blocks (32 warps) stay resident per
 // SM: 2% faster than the 68 registers the compiler picks unbounded (seven blocks), on
 // the 2^24-ray batch over 4.1 M triangles; tighter bounds spill the stack and lose.
-template <int kShort>
+template <int kShort, int kLeave>
 __global__ void __launch_bounds__(128, 8) k_trace_persistent4(DevAccel A, const rx_ray* __restrict__ rays, uint32_t n,
                                                            const uint32_t* __restrict__ order,
                                                            int32_t* __restrict__ out_tid,
@@ -135,7 +147,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_persistent4(DevAccel A, const 
                                                            uint32_t* __restrict__ hit_leaf,
                                                            int4* __restrict__ slot_rec,
                                                            unsigned long long* __restrict__ counters) {
-  walk_wide<4, kShort, 64>(A, A.bvh4, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, counters);
+  walk_wide<4, kShort, 64, kLeave>(A, A.bvh4, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, counters);
 }
 
 // A batch that the GPU holds at once: one launch, a ray per lane, the winner's visibility
@@ -189,7 +201,7 @@ __global__ void __launch_bounds__(128) k_trace_persistent8(DevAccel A, const rx_
                                                            uint32_t* __restrict__ hit_leaf,
                                                            int4* __restrict__ slot_rec,
                                                            unsigned long long* __restrict__ counters) {
-  walk_wide<8, kShort, 80>(A, A.bvh8, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, counters);
+  walk_wide<8, kShort, 80, kWalkLeave>(A, A.bvh8, rays, n, order, out_tid, out_dist, hit_leaf, slot_rec, counters);
 }
 
 // The same check with one thread per ray: each thread walks its winner's ancestor list
@@ -570,10 +582,12 @@ cudaError_t launch_trace_closest(const DevAccel& A, const rx_ray* rays, uint32_t
     const bool walk8 = A.bvh8 && 7 * A.bvh8_depth + 1 <= 80;  // the 8-wide walk's
     if ((cfg.variant == 5 && walk8) || (cfg.variant == 4 && !walk4 && walk8))
       k_trace_persistent8<16><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
+    else if ((cfg.variant == 4 || cfg.variant == 5) && walk4 && walk_waits(A.bvh4_depth, n, (uint64_t)blocks * 128))
+      k_trace_persistent4<16, 0><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
     else if ((cfg.variant == 4 || cfg.variant == 5) && walk4)
-      k_trace_persistent4<16><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
+      k_trace_persistent4<16, kWalkLeave><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
     else if (cfg.variant == 3 && walk4)
-      k_trace_persistent4<0><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
+      k_trace_persistent4<0, kWalkLeave><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
     else if (cfg.variant == 1 && shallow)
       k_trace_persistent<false, 32><<<blocks, 128, 0, s>>>(A, rays, n, order, tid, dist, hit_leaf, slot_rec, counters);
     else if (cfg.variant == 1)

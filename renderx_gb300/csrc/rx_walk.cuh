@@ -60,7 +60,7 @@ __device__ __forceinline__ int walk_lanes(uint32_t n) {
   const uint32_t warps = gridDim.x * 4;
   return (int)min(32u, max(1u, (n + warps - 1) / warps));
 }
-template <int W, int kShort, int kStack, bool kOnce = false, class Lane>
+template <int W, int kShort, int kStack, bool kOnce = false, int kLeave = kWalkLeave, class Lane>
 __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cursor, uint32_t once = kNoRay,
                                                 int lanes = 32) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -116,8 +116,8 @@ __device__ __forceinline__ void walk_persistent(Lane& L, unsigned long long* cur
       const bool need = active && pl == DONE && cur != DONE;
       // lanes to go on for, and lanes that wait with a leaf or a finished ray (leaving makes
       // progress only when there are some)
-      const unsigned go = __ballot_sync(FULL, need), wait = kOnce ? 0u : __ballot_sync(FULL, active && !need);
-      if (go == 0 || (wait != 0 && __popc(go) <= kWalkLeave)) break;
+      const unsigned go = __ballot_sync(FULL, need), wait = kOnce || kLeave == 0 ? 0u : __ballot_sync(FULL, active && !need);
+      if (go == 0 || (wait != 0 && __popc(go) <= kLeave)) break;
       if (!(need || (active && cur >= 0))) continue;
       if (cur < 0) {  // a leaf (only lanes that need one get here)
         pl = cur;
