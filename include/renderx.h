@@ -218,9 +218,12 @@ typedef struct rx_render_stats {
 /* Replaces the process-global GPU state of IntersectionGPU::init
  * (reference src/IntersectionGPU.cpp:16-44). */
 rx_status rx_create(rx_context** out, int device);
-/* A context keeps the device buffers of its renders between calls, at most 8 GiB; they go
- * with it. */
 void rx_destroy(rx_context* ctx);
+/* The contexts of a device share the device buffers of their renders and keep them between
+ * calls, at most 8 GiB in all. This gives back what no running render holds, for others that
+ * allocate on the device (allocations of this library have it given back by themselves
+ * before they fail); so does the rx_destroy of the device's last context. */
+rx_status rx_release_memory(rx_context* ctx);
 const char* rx_last_error(const rx_context* ctx);
 /* Build identification string (kernels, architecture). */
 const char* rx_version(void);

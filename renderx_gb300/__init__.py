@@ -125,6 +125,11 @@ class Context:
     def __exit__(self, *a):
         self.close()
 
+    def release_memory(self):
+        """Gives back the device memory that the renders of this device's contexts keep between
+        calls (at most 8 GiB), for other allocators of the process."""
+        self._ck(self._L.rx_release_memory(self.h))
+
     def _ck(self, st):
         _capi.check(self.h, st)
 

@@ -104,6 +104,7 @@ SNAPSHOT_FN = ctypes.CFUNCTYPE(None, P, ctypes.c_double, ctypes.c_double, ctypes
 SIGNATURES = [
     ("rx_create", S, [ctypes.POINTER(P), S]),
     ("rx_destroy", None, [P]),
+    ("rx_release_memory", S, [P]),
     ("rx_last_error", ctypes.c_char_p, [P]),
     ("rx_version", ctypes.c_char_p, []),
     ("rx_scene_set_geometry", S, [P, P, U32, P, U32, P, P, P]),

@@ -69,6 +69,9 @@ rx_status rx_create(rx_context** out, int device) {
   }
   cudaMemset(c->d_counters.p, 0, c->d_counters.bytes);
   cudaDeviceGetAttribute(&c->trace_cfg.sms, cudaDevAttrMultiProcessorCount, device);
+  c->ws.device = device;
+  c->ws.stream = c->stream;
+  rx::WorkspacePool::of(device).add_context();
   *out = c;
   return RX_OK;
 }
@@ -93,13 +96,20 @@ void rx_destroy(rx_context* c) {
     for (cudaEvent_t e : c->timing_ev) cudaEventDestroy(e);
     rx::guide_free(c->guide);
     c->guide = nullptr;
-    c->ws.trim(0);
+    rx::WorkspacePool::of(c->device).drop_context();
     if (c->stream) cudaStreamDestroy(c->stream);
     if (c->side_stream) cudaStreamDestroy(c->side_stream);
     for (auto s : c->copy_stream)
       if (s) cudaStreamDestroy(s);
   }
   delete c;
+}
+
+rx_status rx_release_memory(rx_context* c) {
+  if (!c) return RX_ERR_INVALID;
+  DeviceGuard g(c->device);
+  rx::WorkspacePool::of(c->device).drain();
+  return RX_OK;
 }
 
 const char* rx_last_error(const rx_context* c) { return c ? c->err.c_str() : "null context"; }
@@ -438,7 +448,7 @@ rx_status rx_render_pt(rx_context* c, const rx_camera* cam, const rx_pt_options*
   }
   DeviceGuard g(c->device);
   const size_t np = (size_t)cam->width * cam->height, film_bytes = np * 3 * sizeof(double);
-  rx::Workspace::Frame frame(c->ws);
+  rx::WorkspaceHold::Frame frame(c->ws);
   rx::WsBuf sum, sq;
   rx_status s;
   if ((s = c->cuda(sum.alloc(c->ws, film_bytes), "film")) != RX_OK) return s;
@@ -486,7 +496,7 @@ rx_status rx_render_pt_batch(rx_context* c, const rx_batch_item* items, uint32_t
     pixels += (uint64_t)cam.width * cam.height;
   }
   DeviceGuard g(c->device);
-  rx::Workspace::Frame frame(c->ws);
+  rx::WorkspaceHold::Frame frame(c->ws);
   rx::WsBuf film;
   rx_status s;
   if ((s = c->cuda(film.alloc(c->ws, pixels * 3 * sizeof(double)), "film")) != RX_OK) return s;
@@ -546,7 +556,7 @@ static rx_status render_bidirectional(rx_context* c, const rx_camera* cam, const
   if (c->scene.num_lights == 0) return c->fail(RX_ERR_INVALID, "vertex connection and merging needs an emitter");
   DeviceGuard g(c->device);
   size_t np = (size_t)cam->width * cam->height;
-  rx::Workspace::Frame frame(c->ws);
+  rx::WorkspaceHold::Frame frame(c->ws);
   rx::WsBuf film;
   rx_status s;
   if ((s = c->cuda(film.alloc(c->ws, np * 3 * sizeof(double)), "film")) != RX_OK) return s;
@@ -591,7 +601,7 @@ rx_status rx_render_pm(rx_context* c, const rx_camera* cam, const rx_pm_options*
   if (c->scene.num_lights == 0) return c->fail(RX_ERR_INVALID, "photon mapping needs an emitter");
   DeviceGuard g(c->device);
   size_t np = (size_t)cam->width * cam->height;
-  rx::Workspace::Frame frame(c->ws);
+  rx::WorkspaceHold::Frame frame(c->ws);
   rx::WsBuf film;
   rx_status s;
   if ((s = c->cuda(film.alloc(c->ws, np * 3 * sizeof(double)), "film")) != RX_OK) return s;

@@ -10,6 +10,7 @@
 #include "../../include/renderx.h"
 #include "rx_accel.h"
 #include "rx_device.h"
+#include "rx_memory.h"
 #include "rx_scene.h"
 
 namespace rx {
@@ -75,143 +76,6 @@ struct DeviceGuard {
     cudaGetDevice(&cur);
     if (prev >= 0 && cur != prev) cudaSetDevice(prev);
   }
-};
-
-// A device allocation, released when its owner goes away (move-only).
-struct DevBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  DevBuf() = default;
-  DevBuf(const DevBuf&) = delete;
-  DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes) {
-    o.p = nullptr;
-    o.bytes = 0;
-  }
-  DevBuf& operator=(DevBuf&& o) noexcept {
-    if (this != &o) {
-      release();
-      p = o.p;
-      bytes = o.bytes;
-      o.p = nullptr;
-      o.bytes = 0;
-    }
-    return *this;
-  }
-  ~DevBuf() { release(); }
-  cudaError_t alloc(size_t b) {
-    release();
-    if (b == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc(&p, b);
-    if (e == cudaSuccess) bytes = b;
-    else p = nullptr;
-    return e;
-  }
-  void release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
-  }
-  template <class T>
-  T* as() const { return static_cast<T*>(p); }
-};
-
-// Device memory that a context's renders take their buffers from and that stays with the
-// context between calls: cudaMalloc and cudaFree of a render's buffers cost more than many
-// renders do (1.3 of 2.1 ms for a 256^2 x 16 frame, 9 of 65 ms for VCM at 512^2). A stack
-// of blocks: a Frame (one per render call) gives back when it ends what was taken since it
-// began, so a call made from a snapshot callback nests. Buffers are used on the
-// context's stream (and on a side stream that the render waits for), which orders one frame's
-// work before the next one's. At most kKeep bytes stay after the outermost frame; a context's
-// memory goes with it. Not thread-safe, as calls on one context are not.
-class Workspace {
-  struct Block {
-    void* p;
-    size_t size, used;
-  };
-
- public:
-  static constexpr size_t kKeep = (size_t)8 << 30;
-  Workspace() = default;
-  Workspace(const Workspace&) = delete;
-  Workspace& operator=(const Workspace&) = delete;
-  ~Workspace() { trim(0); }
-  class Frame {
-   public:
-    explicit Frame(Workspace& ws) : w(ws) {
-      for (const Block& b : w.blocks_) used.push_back(b.used);
-      w.depth_++;
-    }
-    Frame(const Frame&) = delete;
-    Frame& operator=(const Frame&) = delete;
-    ~Frame() {  // what earlier frames hold stays
-      for (size_t k = 0; k < w.blocks_.size(); k++) w.blocks_[k].used = k < used.size() ? used[k] : 0;
-      if (--w.depth_ == 0) w.trim(kKeep);
-    }
-
-   private:
-    Workspace& w;
-    std::vector<size_t> used;
-  };
-  // `bytes` of device memory, 256-byte aligned, until the innermost frame ends: from the
-  // first block with room.
-  cudaError_t alloc(size_t bytes, void** out) {
-    bytes = (bytes + 255) & ~(size_t)255;
-    size_t all = 0;
-    for (Block& b : blocks_) {
-      if (b.size - b.used >= bytes) return take(b, bytes, out);
-      all += b.size;
-    }
-    Block b{nullptr, std::max({bytes, std::min(all / 2, (size_t)512 << 20), (size_t)32 << 20}), 0};
-    cudaError_t e = cudaMalloc(&b.p, b.size);
-    if (e == cudaErrorMemoryAllocation) {  // give back the unused blocks at the top, take no more than asked
-      cudaGetLastError();
-      while (!blocks_.empty() && blocks_.back().used == 0) pop();
-      b.size = bytes;
-      e = cudaMalloc(&b.p, b.size);
-    }
-    if (e != cudaSuccess) return e;
-    blocks_.push_back(b);
-    return take(blocks_.back(), bytes, out);
-  }
-  // Frees blocks from the top until at most `keep` bytes stay (no frame open).
-  void trim(size_t keep) {
-    size_t all = 0;
-    for (const Block& b : blocks_) all += b.size;
-    while (!blocks_.empty() && all > keep) {
-      all -= blocks_.back().size;
-      pop();
-    }
-  }
-
- private:
-  static cudaError_t take(Block& b, size_t bytes, void** out) {
-    *out = static_cast<char*>(b.p) + b.used;
-    b.used += bytes;
-    return cudaSuccess;
-  }
-  void pop() {
-    cudaFree(blocks_.back().p);
-    blocks_.pop_back();
-  }
-  std::vector<Block> blocks_;
-  int depth_ = 0;
-};
-
-// A buffer of a render, from its frame's workspace.
-struct WsBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  cudaError_t alloc(Workspace& w, size_t b) {
-    p = nullptr;
-    bytes = 0;
-    if (b == 0) return cudaSuccess;
-    cudaError_t e = w.alloc(b, &p);
-    if (e == cudaSuccess) bytes = b;
-    return e;
-  }
-  template <class T>
-  T* as() const { return static_cast<T*>(p); }
 };
 
 // A CUDA event, destroyed with its owner (null until created).
@@ -328,7 +192,7 @@ struct rx_context {
   rx::DevBuf d_slot_n, d_tri_v, d_tri_n, d_tri_obj, d_objects, d_light_cdf, d_light_tri, d_media;
   rx::DevBuf d_counters;     // 4 x u64 diagnostics + per-slot queue lengths
   rx::DevBuf d_queue;        // closest-hit scratch (winner leaves + eager queue)
-  rx::Workspace ws;          // the renders' buffers
+  rx::WorkspaceHold ws;      // the renders' buffers
   // staging ring for host-buffer calls
   static constexpr int kRing = 3;  // staging slots of the host-buffer trace
   rx::DevBuf ring_rays[kRing], ring_tid[kRing], ring_dist[kRing], ring_queue[kRing], ring_counters[kRing];

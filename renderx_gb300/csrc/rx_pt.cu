@@ -878,7 +878,7 @@ __global__ void k_net_pad(int nnet, unsigned* ncount, const uint32_t* seg, int* 
 // -------------------------------------------------------------------------------------
 // Host driver
 // -------------------------------------------------------------------------------------
-static cudaError_t alloc_soa(PathSoA& s, Workspace& ws, size_t n) {
+static cudaError_t alloc_soa(PathSoA& s, WorkspaceHold& ws, size_t n) {
   size_t sizes[6] = {16, 16, 16, 16, 16, 8};
   void** ptrs[6] = {(void**)&s.o, (void**)&s.d, (void**)&s.T, (void**)&s.L, (void**)&s.info, (void**)&s.id};
   for (int k = 0; k < 6; k++) {
@@ -1139,7 +1139,7 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
   const uint32_t slots = (uint32_t)slots64;
   const int sms = c->trace_cfg.sms;
 
-  Workspace::Frame frame(c->ws);
+  WorkspaceHold::Frame frame(c->ws);
   cudaError_t e;
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;

@@ -1903,7 +1903,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   // a bucket per two photons and more (about two a path are stored); one for each that could
   // be stored costs 0.4 ms of scans an iteration at 2^20 paths
   while (buckets < std::min<uint64_t>(cap, 4ull * P.n_light) && buckets < (1u << 26)) buckets <<= 1;
-  Workspace::Frame frame(c->ws);
+  WorkspaceHold::Frame frame(c->ws);
   std::vector<WsBuf> bufs(33);
   cudaError_t e;
   auto al = [&](int k, size_t bytes) { return bufs[k].alloc(c->ws, bytes); };
@@ -2172,7 +2172,7 @@ cudaError_t render_pm(rx_context* c, const rx_camera& cam, const rx_pm_options& 
   unsigned buckets = 1u << 16;
   while (buckets < cap && buckets < (1u << 26)) buckets <<= 1;
   const unsigned nscan = buckets + 1, nblk = (nscan + 1023) / 1024;
-  Workspace::Frame frame(c->ws);
+  WorkspaceHold::Frame frame(c->ws);
   std::vector<WsBuf> bufs(12);
   cudaError_t e;
   auto al = [&](int k, size_t bytes) { return bufs[k].alloc(c->ws, bytes); };
