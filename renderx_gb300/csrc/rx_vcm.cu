@@ -1944,6 +1944,15 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
   const bool full_mis = (opt.flags & RX_VCM_FULL_PATH_MIS) != 0;
   const uint32_t pair_cap = 1u << 27;  // pairs per evaluation window
   uint32_t pair_alloc = 1u << 20;      // grows with demand up to pair_cap
+  unsigned long long sq_alloc = 0;     // shadow rays that the queue holds, at most pair_alloc
+  // New size of a list that held `have` and has to hold `need`. What it outgrows stays taken
+  // until the render ends, and the number of connections varies by a few per cent from one
+  // iteration to the next: a quarter of slack, and at least twice as large each time (with the
+  // exact size each new highest number took another queue: 60 BPT iterations at 512^2 2.4 GB
+  // where one takes 0.9).
+  auto grown = [](unsigned long long need, unsigned long long have, unsigned long long most) {
+    return std::min(most, std::max(need + need / 4, 2 * have));
+  };
   if ((e = al(17, (size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return e;
   if ((e = al(18, (size_t)pair_alloc * sizeof(int))) != cudaSuccess) return e;
   unsigned long long* ctr = bufs[11].as<unsigned long long>();
@@ -2045,7 +2054,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       cudaError_t err = cudaStreamSynchronize(s);
       total = tail[0] + tail[1];
       if (err == cudaSuccess && total > pair_alloc && pair_alloc < pair_cap) {
-        pair_alloc = (uint32_t)std::min<unsigned long long>(pair_cap, std::max<unsigned long long>(total, 2ull * pair_alloc));
+        pair_alloc = (uint32_t)grown(total, pair_alloc, pair_cap);
         if ((err = al(17, (size_t)pair_alloc * sizeof(uint32_t))) != cudaSuccess) return err;
         err = al(18, (size_t)pair_alloc * sizeof(int));
       }
@@ -2062,8 +2071,11 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
                                                   bufs[10].as<float>());
       if ((e = scan_total(P.n_pixels, total)) != cudaSuccess) return e;
       // the shadow-ray queue: at most one ray per connection of a window
-      const size_t sq_bytes = (size_t)std::min<unsigned long long>(pair_alloc, std::max(total, 1ull)) * sizeof(ShadowQ);
-      if (bufs[32].bytes < sq_bytes && (e = al(32, sq_bytes)) != cudaSuccess) return e;
+      const unsigned long long sq_need = std::min<unsigned long long>(pair_alloc, std::max(total, 1ull));
+      if (sq_alloc < sq_need) {
+        sq_alloc = grown(sq_need, sq_alloc, pair_alloc);
+        if ((e = al(32, (size_t)sq_alloc * sizeof(ShadowQ))) != cudaSuccess) return e;
+      }
       unsigned* sq_n = reinterpret_cast<unsigned*>(ctr + 13);
       unsigned long long* sq_cursor = ctr + 12;
       for (unsigned long long w0 = 0; w0 < total; w0 += pair_alloc) {
