@@ -1315,12 +1315,20 @@ struct alignas(16) EyeSide {
   uint32_t flags;  // kEyeRandom: pe sampled at random; kEyeBehind
   uint32_t pixel;
 };
+// The queries are merged in windows of kMergeWindow: the eye sides of every vertex an image
+// could have would take as much memory as all else that is kept per eye vertex (96 bytes
+// beside 124), for about a tenth of which are queries; a window beyond their number costs
+// three empty launches. j0: the window's first query.
+constexpr uint32_t kMergeWindow = 1u << 23;
+__device__ __forceinline__ uint32_t window_queries(uint32_t count, uint32_t j0) {
+  return count > j0 ? min(count - j0, kMergeWindow) : 0u;
+}
 __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, const float4* ev, const MisE* emis,
                                                    const uint32_t* qlist, const uint32_t* order, unsigned* count,
-                                                   EyeSide* out) {
-  const uint32_t n = count[0];  // count[1]: queries with kEyeBehind
+                                                   uint32_t j0, EyeSide* out) {
+  const uint32_t n = window_queries(count[0], j0);  // count[1]: queries with kEyeBehind so far
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const uint32_t q = __ldg(&qlist[__ldg(&order[j])]);  // vertex q % maxv >= 1 of pixel q / maxv
+    const uint32_t q = __ldg(&qlist[__ldg(&order[j0 + j])]);  // vertex q % maxv >= 1 of pixel q / maxv
     const PV E = load_pv(ev + 4 * (size_t)q), pe = load_pv(ev + 4 * ((size_t)q - 1));
     const MisE me = emis[q];
     EyeSide e;
@@ -1426,13 +1434,14 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
 constexpr int kMergeList = 32 + 128;
 template <bool BEHIND>
 __global__ void __launch_bounds__(128, 6) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
-                                               const unsigned* count, float* img, unsigned long long* merges) {
+                                               const unsigned* count, uint32_t j0, float* img,
+                                               unsigned long long* merges) {
   __shared__ uint2 s_list[4][kMergeList];
   if (BEHIND && count[1] == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint2* list = s_list[warp];
   const unsigned lt = (1u << lane) - 1u;
-  const uint32_t nq = *count, nw = gridDim.x * 4;
+  const uint32_t nq = window_queries(*count, j0), nw = gridDim.x * 4;
   const float r = P.radius;
   uint32_t fill = 0, cur = 0xffffffffu;
   unsigned long long total = 0;
@@ -1939,7 +1948,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
     if ((e = al(29, (size_t)nq * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = al(30, ((size_t)kRayBins + 1024) * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = al(31, 16)) != cudaSuccess) return e;
-    if ((e = al(24, (size_t)nq * sizeof(EyeSide))) != cudaSuccess) return e;  // their eye sides
+    if ((e = al(24, (size_t)std::min(nq, kMergeWindow) * sizeof(EyeSide))) != cudaSuccess) return e;  // eye sides of a window
   }
   const bool full_mis = (opt.flags & RX_VCM_FULL_PATH_MIS) != 0;
   const uint32_t pair_cap = 1u << 27;  // pairs per evaluation window
@@ -2109,7 +2118,7 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
                                                    bufs[17].as<uint32_t>(), bufs[18].as<int>(), np,
                                                    bufs[10].as<float>());
       }
-    } else {  // the queries in spatial order, one walk appending pairs, then one pair per lane
+    } else {  // the queries in spatial order, their eye sides, then the walk that evaluates the pairs
       if (m0) cudaEventRecord(m0, s);
       uint32_t* qlist = bufs[27].as<uint32_t>();
       uint32_t* qkey = bufs[28].as<uint32_t>();
@@ -2121,10 +2130,13 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
       k_merge_queries<<<grid, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[13].as<int>(), qlist, qkey, qhist, qcount);
       scan_bins(qhist, qhist + kRayBins, s);
       k_ray_scatter<<<grid * 2, 256, 0, s>>>(qkey, 0, qcount, qhist, qorder);
-      k_merge_eye<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), qlist, qorder, qcount,
-                                           bufs[24].as<EyeSide>());
-      k_merge<false><<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
-      k_merge<true><<<merge_grid, 128, 0, s>>>(S, P, G, bufs[24].as<EyeSide>(), qcount, bufs[10].as<float>(), ctr + 4);
+      for (uint64_t j0 = 0; j0 < nq; j0 += kMergeWindow) {
+        EyeSide* eye = bufs[24].as<EyeSide>();
+        k_merge_eye<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), qlist, qorder, qcount,
+                                             (uint32_t)j0, eye);
+        k_merge<false><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, (uint32_t)j0, bufs[10].as<float>(), ctr + 4);
+        k_merge<true><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, (uint32_t)j0, bufs[10].as<float>(), ctr + 4);
+      }
       k_count_photons<<<1, 1, 0, s>>>(qcount, nq, ctr + 5);
       if (m1) {  // device time of this iteration's merge gather (walk + pair evaluation)
         cudaEventRecord(m1, s);
