@@ -32,6 +32,7 @@
 #include "rx_walk.cuh"
 #include "rx_internal.h"
 #include "rx_material.cuh"
+#include "rx_rcp.cuh"
 
 namespace rx {
 
@@ -473,15 +474,6 @@ __device__ __forceinline__ void img_add(float* img, int pixel, F3 c) {
 }
 
 // ---- subpath records --------------------------------------------------------------------
-// 1 / x in double precision: for x well within single precision's range the
-// single-precision reciprocal and two Newton steps (a double division is three times the
-// FP64 operations, and the FP64 pipe is what bounds the records), else the division.
-__device__ __forceinline__ double rcp64(double x) {
-  if (!(x > 1e-30 && x < 1e30)) return 1.0 / x;
-  double y = (double)(1.0f / (float)x);
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
 // Ray::getCosineTerm of a vertex with contact normal `n` along `d`.
 __device__ __forceinline__ float cos_at(const DevScene& S, int contact, F3 n, F3 d) {
   const bool has_cos = contact == kCameraObj || (contact >= 0 && !is_vpm(S, contact));
