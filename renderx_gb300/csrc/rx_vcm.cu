@@ -1311,14 +1311,13 @@ struct alignas(16) EyeSide {
 // could have would take as much memory as all else that is kept per eye vertex (96 bytes
 // beside 124), for about a tenth of which are queries; a window beyond their number costs
 // three empty launches. j0: the window's first query.
+// count: {queries, those with kEyeBehind so far, the window's queries}.
 constexpr uint32_t kMergeWindow = 1u << 23;
-__device__ __forceinline__ uint32_t window_queries(uint32_t count, uint32_t j0) {
-  return count > j0 ? min(count - j0, kMergeWindow) : 0u;
-}
 __global__ void __launch_bounds__(128) k_merge_eye(DevScene S, VcmParams P, const float4* ev, const MisE* emis,
                                                    const uint32_t* qlist, const uint32_t* order, unsigned* count,
                                                    uint32_t j0, EyeSide* out) {
-  const uint32_t n = window_queries(count[0], j0);  // count[1]: queries with kEyeBehind so far
+  const uint32_t all = count[0], n = all > j0 ? min(all - j0, kMergeWindow) : 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) count[2] = n;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const uint32_t q = __ldg(&qlist[__ldg(&order[j0 + j])]);  // vertex q % maxv >= 1 of pixel q / maxv
     const PV E = load_pv(ev + 4 * (size_t)q), pe = load_pv(ev + 4 * ((size_t)q - 1));
@@ -1426,14 +1425,13 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
 constexpr int kMergeList = 32 + 128;
 template <bool BEHIND>
 __global__ void __launch_bounds__(128, 6) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
-                                               const unsigned* count, uint32_t j0, float* img,
-                                               unsigned long long* merges) {
+                                               const unsigned* count, float* img, unsigned long long* merges) {
   __shared__ uint2 s_list[4][kMergeList];
   if (BEHIND && count[1] == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint2* list = s_list[warp];
   const unsigned lt = (1u << lane) - 1u;
-  const uint32_t nq = window_queries(*count, j0), nw = gridDim.x * 4;
+  const uint32_t nq = count[2], nw = gridDim.x * 4;
   const float r = P.radius;
   uint32_t fill = 0, cur = 0xffffffffu;
   unsigned long long total = 0;
@@ -2126,8 +2124,8 @@ cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options
         EyeSide* eye = bufs[24].as<EyeSide>();
         k_merge_eye<<<grid * 2, 128, 0, s>>>(S, P, bufs[12].as<float4>(), bufs[20].as<MisE>(), qlist, qorder, qcount,
                                              (uint32_t)j0, eye);
-        k_merge<false><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, (uint32_t)j0, bufs[10].as<float>(), ctr + 4);
-        k_merge<true><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, (uint32_t)j0, bufs[10].as<float>(), ctr + 4);
+        k_merge<false><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, bufs[10].as<float>(), ctr + 4);
+        k_merge<true><<<merge_grid, 128, 0, s>>>(S, P, G, eye, qcount, bufs[10].as<float>(), ctr + 4);
       }
       k_count_photons<<<1, 1, 0, s>>>(qcount, nq, ctr + 5);
       if (m1) {  // device time of this iteration's merge gather (walk + pair evaluation)
