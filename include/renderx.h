@@ -420,8 +420,10 @@ rx_status rx_trace_set_timing(rx_context* ctx, int32_t max_calls);
 /* ms3[3*i + j]: device milliseconds of kernel j in recorded call i (waits for the
  * events); *calls = number of recorded calls. ms3 may be NULL to query the count. */
 rx_status rx_trace_read_timing(rx_context* ctx, float* ms3, int32_t* calls);
-/* Rays whose lazy winner failed the reference-visibility check and were re-traced
- * exactly, counted since the last reset (diagnostic). */
+/* Diagnostics: out[2] = rays whose lazy winner failed the reference-visibility check and were
+ * re-traced exactly, out[1] = box tests decided by the exact test, out[3] = errors, all since
+ * the last reset; out[0] = length of the re-trace queue of the last device batch that had
+ * one (a batch of the one-launch walk has none). */
 rx_status rx_trace_counters(rx_context* ctx, uint64_t out[4], int reset);
 
 /* ---- learned guiding ------------------------------------------------------------- */

@@ -8,8 +8,9 @@
 // scene box, the shading normal, the outgoing direction, a constant 1) -> 4 hidden
 // layers of 64 ReLU units -> 64 outputs of which 40 are used: 8 lobes x (weight logit,
 // log-concentration, 3 mean coordinates). Weights and activations BF16, accumulation
-// FP32 in tensor memory. One CTA of 128 threads owns a tile of 128 samples; thread s owns
-// sample s (tensor-memory lane s of the M = 128 accumulators).
+// FP32 in tensor memory. A tile is 128 samples, sample s in lane s of an M = 128 accumulator: one
+// warpgroup per tile and eight tiles per CTA in the inference kernel, two warpgroups per tile
+// (half of the columns each) and two tiles per CTA in the training kernel.
 //
 // Training minimises the cross entropy of the mixture against the renderer's integrand
 // samples, -sum_s w_s log q(wi_s) / sum_s w_s, with w_s = (BSDF x cosine x incident

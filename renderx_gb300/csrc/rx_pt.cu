@@ -720,9 +720,7 @@ __global__ void __launch_bounds__(kShadeThreads<MEDIA>, 1024 / kShadeThreads<MED
   }
 }
 
-// The next queue's length, the extension walk's refill cursor for the next bounce
-// (kWalk4P: every k_extend_p launch of a pass is followed by this one, so the cursor is
-// zero when the next starts) and the number of visibility rays.
+// The next pass begins where this one ended (one thread, last in a pass).
 __global__ void k_advance(PassState* ps) {
   ps->base += ps->per_pass;
   ps->pass += 1;
@@ -1438,7 +1436,8 @@ cudaError_t render_pt_jobs(rx_context* c, const PtJob* jobs, int nj, const PtRun
 // whose pass size the caller left open runs in even passes of up to 2^24 paths: a pass's late
 // bounces hold few paths and cost latency, 1.4 of 10.3 ms with 2^22 paths over 1 M triangles
 // (1024^2 x 16: 41.3 ms in passes of 2^22 paths, 37.2 of 2^23, 35.1 of 2^24). 184 bytes a
-// path, 3 GB; where that much is not to be had, passes of 2^22 after all.
+// path, 3.1 GB, and with light sampling's visibility rays 256 bytes, 4.3 GB; where that much is
+// not to be had, passes of 2^22 after all.
 constexpr uint64_t kFramePass = 1u << 24;
 cudaError_t render_pt(rx_context* c, const rx_camera& cam, const rx_pt_options& opt, double* film_sum,
                       double* film_sq, rx_render_stats* stats, cudaStream_t s) {

@@ -49,8 +49,9 @@ constexpr uint32_t kNoRay = 0xffffffffu;
 // 8, 12, 16 lanes left behind and refills at once; 6.66, 6.62, 6.49, 6.39, 6.33 with 8 and
 // refills from 2, 4, 8, 12, 16 on), a 1024^2 x 16 frame over 1 M triangles 47.7 -> 43.3 ms,
 // the Cornell frame 0.868 -> 0.85 ms. A warp that walks one ray per lane has nothing to
-// refill and gains nothing by leaving early (100,003 rays over 25 K triangles 59.1 us, 62.5
-// with 4).
+// refill and leaving early (kLeave 0: never) costs it more than it gains: the one-launch walk
+// of 100,003 rays over 36, 25 K, 256 K and 4.1 M triangles 18.5, 51.3, 84.0 and 182.6 us, with 4
+// lanes left behind 20.5, 55.3, 84.7 and 179.0.
 constexpr int kWalkLeave = 6, kWalkRefill = 12;
 // Lanes of each warp that a launch of resident 128-thread blocks uses for n rays: as few as
 // let every ray start at once, since the lanes of a warp wait for one another. (A frame's
