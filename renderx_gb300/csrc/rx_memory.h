@@ -55,7 +55,7 @@ class Workspace {
     return cudaSuccess;
   }
   void pop() {
-    cudaFree(blocks_.back().p);
+    if (blocks_.back().p) cudaFree(blocks_.back().p);
     blocks_.pop_back();
   }
   std::vector<Block> blocks_;
@@ -135,11 +135,15 @@ inline cudaError_t device_malloc(void** p, size_t bytes) {
 inline cudaError_t Workspace::alloc(size_t bytes, void** out) {
   bytes = (bytes + 255) & ~(size_t)255;
   for (Block& b : blocks_)
-    if (b.size - b.used >= bytes) return take(b, bytes, out);
+    if (b.p && b.size - b.used >= bytes) return take(b, bytes, out);
   Block b{nullptr, std::max({bytes, std::min(size() / 2, (size_t)512 << 20), (size_t)32 << 20}), 0};
   cudaError_t e = device_malloc(&b.p, b.size);
-  if (e == cudaErrorMemoryAllocation) {  // give back the unused blocks at the top, take no more than asked
-    while (!blocks_.empty() && blocks_.back().used == 0) pop();
+  if (e == cudaErrorMemoryAllocation) {  // give back the unused blocks, take no more than asked
+    for (Block& u : blocks_)  // (an empty block keeps its place: the frames' marks go by it)
+      if (u.p && u.used == 0) {
+        cudaFree(u.p);
+        u = Block{nullptr, 0, 0};
+      }
     b.size = bytes;
     e = device_malloc(&b.p, b.size);
   }

@@ -111,6 +111,25 @@ int main() {
     CHECK(a.ws.alloc(GB, (void**)&r) == cudaSuccess && r == q);
   }
   CHECK(g_used == 0);
+  {  // kept blocks that a larger render takes nothing from are given back wherever they lie
+    Context a;
+    {
+      WorkspaceHold::Frame f(a.ws);
+      void* p;
+      for (size_t n : {GB, 2 * GB, 4 * GB}) CHECK(a.ws.alloc(n, &p) == cudaSuccess);
+      CHECK(g_used == 7 * GB);
+    }
+    WorkspaceHold::Frame outer(a.ws);
+    char *p, *q, *r;
+    CHECK(a.ws.alloc(GB, (void**)&p) == cudaSuccess && a.ws.alloc(3 * GB, (void**)&q) == cudaSuccess);
+    CHECK(g_used == 7 * GB);  // the blocks of 1 and 4 GB, with the one of 2 GB between them
+    {
+      WorkspaceHold::Frame inner(a.ws);
+      CHECK(a.ws.alloc(g_size - 5 * GB, (void**)&r) == cudaSuccess && g_used == g_size);
+    }
+    CHECK(a.ws.alloc(g_size - 5 * GB, (void**)&p) == cudaSuccess && p == r && g_used == g_size);
+  }
+  CHECK(g_used == 0);
   // renders in several threads, too large to be kept and at times for the device: no two hold the same bytes
   g_size = 24 * GB;
   std::mutex held_m;
