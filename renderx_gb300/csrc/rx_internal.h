@@ -288,6 +288,17 @@ cudaError_t render_pt(rx_context* c, const rx_camera& cam, const rx_pt_options& 
 constexpr uint32_t kVcmBidirectional = 1u << 31;
 cudaError_t render_vcm(rx_context* c, const rx_camera& cam, const rx_vcm_options& opt, double* film,
                        rx_render_stats* stats, cudaStream_t s);
+// Blocks of four warps for PhotonMap's gathers, one pixel per warp up to 256 blocks per SM, so
+// that the last ones to run are a small part of the work. With eight blocks per SM, of which five
+// or six fit, the blocks that come second ran on a part of the SMs: ms per iteration with 8,
+// 64 and 256, and with 8 in the 80 registers that let six blocks fit:
+//   medium 512^2, 2^18 photon paths, r 0.0963   19.6   15.1   15.2   19.7
+//   medium 512^2, 2^18, r 0.03                   8.69   8.08   6.72   8.81
+//   Cornell 512^2, 2^20, r 0.3                  41.4   32.5   29.5   40.3
+//   Cornell 100^2, 10,000, r 0.0963              0.385  0.363  0.366  0.384
+inline unsigned pm_eye_blocks(uint32_t pixels, int sms) {
+  return (unsigned)std::min<uint64_t>(((uint64_t)pixels + 3) / 4, 256ull * (unsigned)sms);
+}
 // PhotonMap (rx_vcm.cu): adds iteration images to `film` (sum).
 cudaError_t render_pm(rx_context* c, const rx_camera& cam, const rx_pm_options& opt, double* film,
                       rx_render_stats* stats, cudaStream_t s);

@@ -1743,8 +1743,9 @@ __device__ F3 pm_gather_lane(const DevScene& S, const CamDev& cam, const Grid& G
 
 // One warp per pixel: lane 0 samples the eye merge path into shared memory, then the
 // lanes share the ray-marching steps of each medium segment (one gather per lane) and
-// split the photons of the gather at the first random surface vertex.
-// (At least four blocks per SM: 20.1 ms per iteration at 512^2, 20.5 unbounded, 21.1 with six.)
+// split the photons of the gather at the first random surface vertex. Four blocks or more
+// per SM (five fit: 94 registers; in the 80 of six it spills), a pixel or two per warp
+// (pm_eye_blocks).
 __global__ void __launch_bounds__(128, 4) k_pm_eye(DevScene S, VcmParams P, Grid G, const float4* pdata, const int* box,
                                                 float* img, unsigned long long* rays) {
   __shared__ float4 paths[4][kPmMaxV * 4];
@@ -2233,7 +2234,7 @@ cudaError_t render_pm(rx_context* c, const rx_camera& cam, const rx_pm_options& 
     k_pm_box<<<grid, 256, 0, s>>>(bufs[0].as<float4>(), nph, cap, bufs[11].as<int>());
     Grid G{cell, buckets - 1, bufs[6].as<unsigned>(), bufs[3].as<float4>(), nullptr, nullptr};
     cudaMemsetAsync(bufs[9].p, 0, bufs[9].bytes, s);
-    k_pm_eye<<<grid * 2, 128, 0, s>>>(S, P, G, bufs[4].as<float4>(), bufs[11].as<int>(), bufs[9].as<float>(), ctr + 1);
+    k_pm_eye<<<pm_eye_blocks(P.n_pixels, c->trace_cfg.sms), 128, 0, s>>>(S, P, G, bufs[4].as<float4>(), bufs[11].as<int>(), bufs[9].as<float>(), ctr + 1);
     k_vcm_accumulate<<<grid, 256, 0, s>>>(P, bufs[9].as<float>(), film);
     unsigned np = 0;
     cudaMemcpyAsync(&np, nph, sizeof np, cudaMemcpyDeviceToHost, s);
