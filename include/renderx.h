@@ -26,7 +26,7 @@ typedef enum rx_status {
   RX_ERR_CUDA = 2,        /* CUDA runtime error */
   RX_ERR_OOM = 3,         /* device or host allocation failed */
   RX_ERR_STATE = 4,       /* call out of order (e.g. trace before build) */
-  RX_ERR_TIMEOUT = 5,     /* a bounded device loop ran out of iterations */
+  RX_ERR_TIMEOUT = 5,     /* a bounded wait on the device ran out of time */
   RX_ERR_UNSUPPORTED = 6
 } rx_status;
 

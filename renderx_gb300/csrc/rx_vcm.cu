@@ -1419,9 +1419,12 @@ __device__ __forceinline__ F3 merge_pair(const DevScene& S, const float4* jd, co
 // back, one counter that every walking warp waited on, the list's size read by the host
 // and the walk repeated when it had grown), and the evaluation formed both vertices'
 // normals and reversed directions per pair: 14.1 + 3.75 ms (7.5 when the walk repeated)
-// against 5.06 ms here. BEHIND: the queries whose pairs may look up an inside object, hardly
-// any; apart from them the kernel fits in 80 registers and six blocks per SM (7, 5 and 4
-// blocks: 5.64, 5.54 and 6.34 ms; with the look-up in the one kernel 6.76 at 128 registers).
+// against 5.06 ms here. BEHIND: the queries whose pairs may look up an inside object, vertices
+// that a ray reached from behind a glossy or Phong surface; apart from them the kernel fits in
+// 80 registers and six blocks per SM (7, 5 and 4 blocks: 5.64, 5.54 and 6.34 ms; with the
+// look-up in the one kernel 6.76 at 128 registers). Where all queries are such (a room of
+// glossy walls seen from behind, 7.3 M pairs an iteration) merging takes 0.69 ms against 1.10
+// with the list of pairs, with the medium sphere in it (13.8 M pairs) 1.63 against 8.16.
 constexpr int kMergeList = 32 + 128;
 template <bool BEHIND>
 __global__ void __launch_bounds__(128, 6) k_merge(DevScene S, VcmParams P, Grid G, const EyeSide* __restrict__ eye,
